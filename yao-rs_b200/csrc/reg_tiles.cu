@@ -1,0 +1,1448 @@
+// reg_tiles.cu — register passes (see reg_tiles.h): the planner that cuts a
+// program of 1- and 2-qubit gates into passes and segments, and the kernel.
+//
+// A pass reads each 2^tbits-amplitude tile once, applies its ops and writes
+// it back.  Each thread owns 2^RB amplitudes that differ in the segment's RB
+// tile positions and applies all ops of the segment in registers; between
+// segments the tile changes hands through shared memory (one barrier).
+//
+// What bounds it: an op's own latency (its description from shared memory,
+// the jump to its code, its coefficients: about 290 cycles) beside its FP64
+// or packed FP32 work (192 cycles a warp for a rotation of 16 amplitudes),
+// with three warps a scheduler to overlap them: the FP64 pipe is busy half of
+// the time.  So ops are few and large: a rotation carries the phase before
+// it and the CZ signs around it (561 ops for the 1950 gates of the layered
+// circuit, n = 28, 20 layers), and 16 amplitudes a thread share each op's
+// fixed cost.  Against the block passes of sv_tiles.cu on that circuit, kernel
+// time: complex128 FUSED 185 -> 109 ms, complex64 FUSED 222 -> 111 ms; TILED
+// at n = 25, 8 layers (no multiplication of gates, no FMA) 62.7 -> 23 ms.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "device_common.cuh"
+#include "reg_tiles.h"
+#include "tc_sm100.cuh"
+#include "tma_sm100.cuh"
+
+namespace yao {
+
+// ================================================================== device
+
+struct RHdr {
+    int32_t tbits, nsegs, blob16, nbuf;  // blob16: 16-byte words of the description
+    int32_t ops16, coef16;               // first 16-byte word of the ops and of the coefficients
+    int32_t use_tma, pad;
+    uint32_t ntiles, pad2;
+    int8_t tb[16];
+    TmaPlan tma;
+};
+
+constexpr uint64_t kRegWaitNs = 1000000000ull;  // 1 s
+
+__device__ __forceinline__ uint64_t reg_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// 128-byte TMA swizzle on byte offsets within a 1024-byte aligned tile.
+__device__ __forceinline__ uint32_t rswz(uint32_t b) { return b ^ ((b >> 3) & 0x70u); }
+
+// Arithmetic on one amplitude type.  complex128: EXACT is num_complex's
+// operations without FMA, else FMA.  complex64: coefficients split into
+// high and low FP32 parts, each stored twice so that one packed FP32x2 FMA
+// handles both components; the small low products are summed first.
+template <bool EXACT>
+struct A128 {
+    typedef double2 Amp;
+    static constexpr int kCoef16 = 1;  // 16-byte words a complex coefficient
+    struct Coef {
+        double2 c;
+    };
+    static __device__ __forceinline__ Coef load(const uint4* p) { return Coef{*(const double2*)p}; }
+    static __device__ __forceinline__ bool is_one(const Coef& k) { return k.c.x == 1.0 && k.c.y == 0.0; }
+    static __device__ __forceinline__ Amp mul(const Coef& k, Amp x) {
+        if (EXACT) return cmulassign_x(x, k.c);
+        return make_double2(fma(k.c.x, x.x, -k.c.y * x.y), fma(k.c.x, x.y, k.c.y * x.x));
+    }
+    static __device__ __forceinline__ Amp mad(Amp acc, const Coef& k, Amp x) {
+        if (EXACT) return cadd_x(acc, cmul_x(k.c, x));
+        return make_double2(fma(k.c.x, x.x, fma(-k.c.y, x.y, acc.x)), fma(k.c.x, x.y, fma(k.c.y, x.x, acc.y)));
+    }
+    // a w + b x
+    static __device__ __forceinline__ Amp two(const Coef& a, Amp w, const Coef& b, Amp x) {
+        if (EXACT) return cadd_x(cmul_x(a.c, w), cmul_x(b.c, x));
+        return mad(make_double2(fma(a.c.x, w.x, -a.c.y * w.y), fma(a.c.x, w.y, a.c.y * w.x)), b, x);
+    }
+    // real matrix [[a, b], [c, d]]: p = (a, b), q = (c, d)
+    struct Real {
+        double2 p, q;
+    };
+    static __device__ __forceinline__ Real load_real(const uint4* m) { return Real{*(const double2*)m, *(const double2*)(m + 1)}; }
+    static __device__ __forceinline__ void real(const Real& k, Amp& w, Amp& x) {
+        const Amp y = make_double2(k.q.y * x.x, k.q.y * x.y), z = make_double2(k.p.y * x.x, k.p.y * x.y);
+        x = make_double2(fma(k.q.x, w.x, y.x), fma(k.q.x, w.y, y.y));
+        w = make_double2(fma(k.p.x, w.x, z.x), fma(k.p.x, w.y, z.y));
+    }
+    // first column real: p = (a, c), then b, d
+    static __device__ __forceinline__ void rcol(const double2& p, const Coef& b, const Coef& d, Amp& w, Amp& x) {
+        const Amp u = mul(b, x), v = mul(d, x);
+        x = make_double2(fma(p.y, w.x, v.x), fma(p.y, w.y, v.y));
+        w = make_double2(fma(p.x, w.x, u.x), fma(p.x, w.y, u.y));
+    }
+    // first row real: p = (a, b), then c, d
+    static __device__ __forceinline__ void rrow(const double2& p, const Coef& c, const Coef& d, Amp& w, Amp& x) {
+        const Amp v = two(c, w, d, x);
+        w = make_double2(fma(p.x, w.x, p.y * x.x), fma(p.x, w.y, p.y * x.y));
+        x = v;
+    }
+    typedef double2 Two;  // two real coefficients
+    static __device__ __forceinline__ Two load_two(const uint4* m) { return *(const double2*)m; }
+    // the second column of a matrix (the second of two reals) times -1 when
+    // the top bit of s is set
+    static __device__ __forceinline__ double flip(double x, uint32_t s) {
+        return __hiloint2double(__double2hiint(x) ^ (int)s, __double2loint(x));
+    }
+    static __device__ __forceinline__ Real sign_real(const Real& k, uint32_t s) {
+        return Real{make_double2(k.p.x, flip(k.p.y, s)), make_double2(k.q.x, flip(k.q.y, s))};
+    }
+    static __device__ __forceinline__ Two sign_two(const Two& k, uint32_t s) { return make_double2(k.x, flip(k.y, s)); }
+    static __device__ __forceinline__ Coef sign_coef(const Coef& k, uint32_t s) {
+        return Coef{make_double2(flip(k.c.x, s), flip(k.c.y, s))};
+    }
+    // x times -1 when the top bit of s is set
+    static __device__ __forceinline__ Amp sign(Amp x, uint32_t s) {
+        return make_double2(__hiloint2double(__double2hiint(x.x) ^ (int)s, __double2loint(x.x)),
+                            __hiloint2double(__double2hiint(x.y) ^ (int)s, __double2loint(x.y)));
+    }
+    static __device__ __forceinline__ Amp neg(Amp x) { return make_double2(-x.x, -x.y); }
+};
+
+__device__ __forceinline__ uint64_t pk(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// i x = (-im, re)
+__device__ __forceinline__ uint64_t iturn(uint64_t x) {
+    float re, im;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(re), "=f"(im) : "l"(x));
+    return pk(-im, re);
+}
+
+struct A64 {
+    typedef uint64_t Amp;
+    static constexpr int kCoef16 = 2;
+    struct Coef {
+        uint64_t hr, hi, lr, li;
+    };
+    static __device__ __forceinline__ Coef load(const uint4* p) {
+        const ulonglong2 a = *(const ulonglong2*)p, b = *(const ulonglong2*)(p + 1);
+        return Coef{a.x, a.y, b.x, b.y};
+    }
+    static __device__ __forceinline__ bool is_one(const Coef& k) {
+        return k.hr == 0x3f8000003f800000ull && k.hi == 0 && k.lr == 0 && k.li == 0;
+    }
+    static __device__ __forceinline__ Amp mul(const Coef& k, Amp x) {
+        const uint64_t t = iturn(x);
+        return fma2(k.hr, x, fma2(k.hi, t, fma2(k.lr, x, mul2(k.li, t))));
+    }
+    static __device__ __forceinline__ Amp mad(Amp acc, const Coef& k, Amp x) {
+        const uint64_t t = iturn(x);
+        return fma2(k.hr, x, fma2(k.hi, t, fma2(k.lr, x, fma2(k.li, t, acc))));
+    }
+    static __device__ __forceinline__ Amp two(const Coef& a, Amp w, const Coef& b, Amp x) {
+        const uint64_t u = iturn(w), t = iturn(x);
+        const uint64_t lo = fma2(b.lr, x, fma2(b.li, t, fma2(a.lr, w, mul2(a.li, u))));
+        return fma2(b.hr, x, fma2(b.hi, t, fma2(a.hr, w, fma2(a.hi, u, lo))));
+    }
+    struct Real {
+        Coef p, q;  // hr, lr: first of the two reals; hi, li: the second
+    };
+    typedef Coef Two;
+    static __device__ __forceinline__ Two load_two(const uint4* m) { return load(m); }
+    static __device__ __forceinline__ Real load_real(const uint4* m) { return Real{load(m), load(m + 2)}; }
+    static __device__ __forceinline__ void real(const Real& k, Amp& w, Amp& x) {
+        const Amp y = fma2(k.q.lr, w, mul2(k.q.li, x)), z = fma2(k.p.lr, w, mul2(k.p.li, x));
+        const Amp v = fma2(k.q.hr, w, fma2(k.q.hi, x, y));
+        w = fma2(k.p.hr, w, fma2(k.p.hi, x, z));
+        x = v;
+    }
+    static __device__ __forceinline__ void rcol(const Coef& p, const Coef& b, const Coef& d, Amp& w, Amp& x) {
+        const uint64_t t = iturn(x);
+        const Amp lu = fma2(p.lr, w, fma2(b.lr, x, mul2(b.li, t))), lv = fma2(p.li, w, fma2(d.lr, x, mul2(d.li, t)));
+        const Amp v = fma2(p.hi, w, fma2(d.hr, x, fma2(d.hi, t, lv)));
+        w = fma2(p.hr, w, fma2(b.hr, x, fma2(b.hi, t, lu)));
+        x = v;
+    }
+    static __device__ __forceinline__ void rrow(const Coef& p, const Coef& c, const Coef& d, Amp& w, Amp& x) {
+        const Amp v = two(c, w, d, x);
+        w = fma2(p.hr, w, fma2(p.hi, x, fma2(p.lr, w, mul2(p.li, x))));
+        x = v;
+    }
+    static __device__ __forceinline__ Amp sign(Amp x, uint32_t s) { return x ^ ((uint64_t)s << 32 | s); }
+    static __device__ __forceinline__ Coef sign_coef(const Coef& k, uint32_t s) {
+        return Coef{sign(k.hr, s), sign(k.hi, s), sign(k.lr, s), sign(k.li, s)};
+    }
+    static __device__ __forceinline__ Two sign_two(const Two& k, uint32_t s) { return Coef{k.hr, sign(k.hi, s), k.lr, sign(k.li, s)}; }
+    static __device__ __forceinline__ Real sign_real(const Real& k, uint32_t s) { return Real{sign_two(k.p, s), sign_two(k.q, s)}; }
+    static __device__ __forceinline__ Amp neg(Amp x) { return x ^ 0x8000000080000000ull; }
+};
+
+// Negates the second member of the pairs in sg (bit j: pair of amplitude j).
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_sign(typename A::Amp (&v)[1 << RB], uint32_t sg) {
+    if (sg) {
+#pragma unroll
+        for (int j = 0; j < (1 << RB); j++)
+            if (!(j & (1 << P))) v[j | (1 << P)] = A::sign(v[j | (1 << P)], (sg << (31 - j)) & 0x80000000u);
+    }
+}
+
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_real1(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t sg, uint32_t cs) {
+    const typename A::Real k = A::sign_real(A::load_real(m), cs);
+    r_sign<A, RB, P>(v, sg);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++)
+        if (!(j & (1 << P))) A::real(k, v[j], v[j | (1 << P)]);
+}
+
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_rcol1(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t sg, uint32_t cs) {
+    const typename A::Two p = A::load_two(m);
+    const typename A::Coef b = A::sign_coef(A::load(m + A::kCoef16), cs), d = A::sign_coef(A::load(m + 2 * A::kCoef16), cs);
+    r_sign<A, RB, P>(v, sg);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++)
+        if (!(j & (1 << P))) A::rcol(p, b, d, v[j], v[j | (1 << P)]);
+}
+
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_rrow1(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t sg, uint32_t cs) {
+    const typename A::Two p = A::sign_two(A::load_two(m), cs);
+    const typename A::Coef c = A::load(m + A::kCoef16), d = A::sign_coef(A::load(m + 2 * A::kCoef16), cs);
+    r_sign<A, RB, P>(v, sg);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++)
+        if (!(j & (1 << P))) A::rrow(p, c, d, v[j], v[j | (1 << P)]);
+}
+
+template <typename A, int RB, int P, bool ALL>
+__device__ __forceinline__ void r_dense1(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t jm, uint32_t sg, uint32_t cs) {
+    const typename A::Coef a = A::load(m), b = A::sign_coef(A::load(m + A::kCoef16), cs), c = A::load(m + 2 * A::kCoef16),
+                           d = A::sign_coef(A::load(m + 3 * A::kCoef16), cs);
+    r_sign<A, RB, P>(v, sg);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++) {
+        if (j & (1 << P)) continue;
+        if (!ALL && !((jm >> j) & 1)) continue;
+        const typename A::Amp w = v[j], x = v[j | (1 << P)];
+        v[j] = A::two(a, w, b, x);
+        v[j | (1 << P)] = A::two(c, w, d, x);
+    }
+}
+
+// (A permutation without the tests costs registers: the compiler then has
+// every other op's results moved to match it.)
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_x(typename A::Amp (&v)[1 << RB], uint32_t jm) {
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++) {
+        if (j & (1 << P)) continue;
+        if (!((jm >> j) & 1)) continue;
+        const typename A::Amp w = v[j];
+        v[j] = v[j | (1 << P)];
+        v[j | (1 << P)] = w;
+    }
+}
+
+template <typename A, bool EXACT, int RB, int P>
+__device__ __forceinline__ void r_phase1(typename A::Amp (&v)[1 << RB], const typename A::Coef& c) {
+    if (EXACT && A::is_one(c)) return;
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++)
+        if (j & (1 << P)) v[j] = A::mul(c, v[j]);
+}
+
+// Which entry of its table a thread's diagonal op takes.
+__device__ __forceinline__ uint32_t r_entry(const uint4& w1, uint32_t t, uint32_t lb) {
+    const int ns = (int)(w1.z >> 8);
+    uint32_t e = 0;
+    for (int q = 0; q < ns; q++) {
+        const uint32_t p = (q < 5 ? w1.y >> (6 * q) : w1.z) & 63u;
+        e |= (p < 16 ? (lb >> p) & 1u : (t >> (p - 16)) & 1u) << q;
+    }
+    return e;
+}
+
+template <typename A, int RB, int PAIR>
+__device__ __forceinline__ void r_dense2(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t jm) {
+    constexpr int B0 = 1 << (2 * PAIR), B1 = 2 << (2 * PAIR);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++) {
+        if (j & (B0 | B1)) continue;
+        if (!((jm >> j) & 1)) continue;
+        const typename A::Amp x0 = v[j], x1 = v[j | B0], x2 = v[j | B1], x3 = v[j | B0 | B1];
+        typename A::Amp y[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const uint4* mr = m + 4 * r * A::kCoef16;
+            y[r] = A::mad(A::mad(A::two(A::load(mr), x0, A::load(mr + A::kCoef16), x1), A::load(mr + 2 * A::kCoef16), x2),
+                          A::load(mr + 3 * A::kCoef16), x3);
+        }
+        v[j] = y[0];
+        v[j | B0] = y[1];
+        v[j | B1] = y[2];
+        v[j | B0 | B1] = y[3];
+    }
+}
+
+template <typename A, int RB, int PAIR>
+__device__ __forceinline__ void r_swap(typename A::Amp (&v)[1 << RB], uint32_t jm) {
+    constexpr int B0 = 1 << (2 * PAIR), B1 = 2 << (2 * PAIR);
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++) {
+        if (j & (B0 | B1)) continue;
+        if (!((jm >> j) & 1)) continue;
+        const typename A::Amp w = v[j | B0];
+        v[j | B0] = v[j | B1];
+        v[j | B1] = w;
+    }
+}
+
+// The ops of one segment on one thread's amplitudes.  t: the tile's number;
+// lb: the thread's tile position (register positions at 0).
+template <typename A, bool EXACT, int RB>
+__device__ __forceinline__ void r_ops(typename A::Amp (&v)[1 << RB], const uint4* ops, const uint4* coef, int begin,
+                                      int end, uint32_t t, uint32_t lb) {
+    for (int oi = begin; oi < end; oi++) {
+        const uint4 w0 = ops[2 * oi], w1 = ops[2 * oi + 1];
+        const bool on = (t & w0.w) == w1.x && (lb & (w0.z & 0xffffu)) == (w0.z >> 16);
+        const uint32_t jm = on ? w0.x >> 16 : 0u;
+        const uint32_t sg = EXACT ? 0u : w1.w & 0xffffu;                       // pairs negated
+        const uint32_t cs = !EXACT && on && (w1.w >> 16) ? 0x80000000u : 0u;   // the second column negated
+        const uint4* m = coef + (size_t)w0.y * A::kCoef16;
+        switch (w0.x & 0xffu) {
+        case RC_DENSE1 + 0: r_dense1<A, RB, 0, !EXACT>(v, m, jm, sg, cs); break;
+        case RC_DENSE1 + 1: r_dense1<A, RB, 1, !EXACT>(v, m, jm, sg, cs); break;
+        case RC_DENSE1 + 2:
+            if constexpr (RB > 2) r_dense1<A, RB, 2, !EXACT>(v, m, jm, sg, cs);
+            break;
+        case RC_DENSE1 + 3:
+            if constexpr (RB > 3) r_dense1<A, RB, 3, !EXACT>(v, m, jm, sg, cs);
+            break;
+        case RC_REAL1 + 0:
+            if constexpr (!EXACT) r_real1<A, RB, 0>(v, m, sg, cs);
+            break;
+        case RC_REAL1 + 1:
+            if constexpr (!EXACT) r_real1<A, RB, 1>(v, m, sg, cs);
+            break;
+        case RC_REAL1 + 2:
+            if constexpr (!EXACT && RB > 2) r_real1<A, RB, 2>(v, m, sg, cs);
+            break;
+        case RC_REAL1 + 3:
+            if constexpr (!EXACT && RB > 3) r_real1<A, RB, 3>(v, m, sg, cs);
+            break;
+        case RC_RCOL1 + 0:
+            if constexpr (!EXACT) r_rcol1<A, RB, 0>(v, m, sg, cs);
+            break;
+        case RC_RCOL1 + 1:
+            if constexpr (!EXACT) r_rcol1<A, RB, 1>(v, m, sg, cs);
+            break;
+        case RC_RCOL1 + 2:
+            if constexpr (!EXACT && RB > 2) r_rcol1<A, RB, 2>(v, m, sg, cs);
+            break;
+        case RC_RCOL1 + 3:
+            if constexpr (!EXACT && RB > 3) r_rcol1<A, RB, 3>(v, m, sg, cs);
+            break;
+        case RC_RROW1 + 0:
+            if constexpr (!EXACT) r_rrow1<A, RB, 0>(v, m, sg, cs);
+            break;
+        case RC_RROW1 + 1:
+            if constexpr (!EXACT) r_rrow1<A, RB, 1>(v, m, sg, cs);
+            break;
+        case RC_RROW1 + 2:
+            if constexpr (!EXACT && RB > 2) r_rrow1<A, RB, 2>(v, m, sg, cs);
+            break;
+        case RC_RROW1 + 3:
+            if constexpr (!EXACT && RB > 3) r_rrow1<A, RB, 3>(v, m, sg, cs);
+            break;
+        case RC_MASKED1 + 0: r_dense1<A, RB, 0, false>(v, m, jm, 0u, 0u); break;
+        case RC_MASKED1 + 1: r_dense1<A, RB, 1, false>(v, m, jm, 0u, 0u); break;
+        case RC_MASKED1 + 2:
+            if constexpr (RB > 2) r_dense1<A, RB, 2, false>(v, m, jm, 0u, 0u);
+            break;
+        case RC_MASKED1 + 3:
+            if constexpr (RB > 3) r_dense1<A, RB, 3, false>(v, m, jm, 0u, 0u);
+            break;
+        case RC_X + 0: r_x<A, RB, 0>(v, jm); break;
+        case RC_X + 1: r_x<A, RB, 1>(v, jm); break;
+        case RC_X + 2:
+            if constexpr (RB > 2) r_x<A, RB, 2>(v, jm);
+            break;
+        case RC_X + 3:
+            if constexpr (RB > 3) r_x<A, RB, 3>(v, jm);
+            break;
+        case RC_PHASE1 + 0: r_phase1<A, EXACT, RB, 0>(v, A::load(m + r_entry(w1, t, lb) * A::kCoef16)); break;
+        case RC_PHASE1 + 1: r_phase1<A, EXACT, RB, 1>(v, A::load(m + r_entry(w1, t, lb) * A::kCoef16)); break;
+        case RC_PHASE1 + 2:
+            if constexpr (RB > 2) r_phase1<A, EXACT, RB, 2>(v, A::load(m + r_entry(w1, t, lb) * A::kCoef16));
+            break;
+        case RC_PHASE1 + 3:
+            if constexpr (RB > 3) r_phase1<A, EXACT, RB, 3>(v, A::load(m + r_entry(w1, t, lb) * A::kCoef16));
+            break;
+        case RC_DENSE2 + 0: r_dense2<A, RB, 0>(v, m, jm); break;
+        case RC_DENSE2 + 1:
+            if constexpr (RB > 3) r_dense2<A, RB, 1>(v, m, jm);
+            break;
+        case RC_SWAP + 0: r_swap<A, RB, 0>(v, jm); break;
+        case RC_SWAP + 1:
+            if constexpr (RB > 3) r_swap<A, RB, 1>(v, jm);
+            break;
+        case RC_NEG:
+#pragma unroll
+            for (int j = 0; j < (1 << RB); j++)
+                if ((jm >> j) & 1) v[j] = A::neg(v[j]);
+            break;
+        case RC_DIAG: {
+            if (EXACT) break;  // not planned
+            const uint4* md = m + ((size_t)r_entry(w1, t, lb) << RB) * A::kCoef16;
+            // the tests also keep the loads apart: all coefficients at once would not fit the registers
+#pragma unroll
+            for (int j = 0; j < (1 << RB); j++)
+                if ((jm >> j) & 1) v[j] = A::mul(A::load(md + j * A::kCoef16), v[j]);
+            break;
+        }
+        default: {  // RC_PHASE
+            const typename A::Coef c = A::load(m + r_entry(w1, t, lb) * A::kCoef16);
+            if (EXACT && A::is_one(c)) break;  // as a gate alone: an entry of exactly 1 leaves its amplitudes alone
+#pragma unroll
+            for (int j = 0; j < (1 << RB); j++)
+                if ((jm >> j) & 1) v[j] = A::mul(c, v[j]);
+            break;
+        }
+        }
+    }
+}
+
+__device__ __forceinline__ uint64_t r_base(const RHdr& h, uint32_t t) { return insert_zeros(t, h.tb, h.tbits); }
+__device__ __forceinline__ uint64_t r_deposit(const RHdr& h, uint32_t l) {
+    uint64_t o = 0;
+    for (int j = 0; j < h.tbits; j++) o |= (uint64_t)((l >> j) & 1u) << h.tb[j];
+    return o;
+}
+
+// A thread's place in a segment: its tile position (register positions at
+// 0) and the swizzled byte offsets of that and of each register position.
+template <int RB>
+struct RPlace {
+    uint32_t lb, sb, so[RB];
+    __device__ __forceinline__ RPlace(const uint4& sg, uint32_t amp) {
+        lb = threadIdx.x;
+#pragma unroll
+        for (int i = 0; i < RB; i++) {
+            const uint32_t p = (sg.z >> (8 * i)) & 0xffu;
+            lb = ((lb >> p) << (p + 1)) | (lb & ((1u << p) - 1));
+            so[i] = rswz(amp << ((sg.w >> (8 * i)) & 0xffu));
+        }
+        sb = rswz(lb * amp);
+    }
+    __device__ __forceinline__ uint32_t at(int j) const {
+        uint32_t o = sb;
+#pragma unroll
+        for (int i = 0; i < RB; i++)
+            if (j & (1 << i)) o ^= so[i];
+        return o;
+    }
+};
+
+// Threads of a CTA and CTAs an SM that the registers are divided for.  At 16
+// amplitudes a thread, complex128 takes 168 registers (at 128 the compiler
+// spills, and the register passes of the layered circuit, n = 28, 20 layers,
+// took 118 ms against 109 ms) and 2^11 tiles; complex64 takes 128 and 2^12
+// tiles (one more moving bit a pass: 111 ms against 116 ms).
+template <typename A, int RB>
+constexpr int reg_threads() {
+    return RB < 4 ? 512 : sizeof(typename A::Amp) == 16 ? 128 : 256;
+}
+template <typename A, int RB>
+constexpr int reg_ctas() {
+    return RB < 4 ? 1 : sizeof(typename A::Amp) == 16 ? 3 : 2;
+}
+
+// Persistent: CTA b takes tiles b, b + grid, ...  A tile arrives in a shared
+// buffer (TMA; small tiles and shapes without a tensor map by plain loads),
+// changes hands there between segments, and leaves from the last segment's
+// registers by plain stores (that segment's register positions are not the
+// lowest, so a warp writes whole 128-byte runs).  The buffer is free once
+// the last segment has read it: thread 0 then issues the load of the tile
+// nbuf tiles on, which arrives while this one computes.  Every wait is
+// bounded: one that gives up sets *err and the pass's result is void.
+template <typename A, bool EXACT, int RB>
+__global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
+    k_reg_tiles(typename A::Amp* __restrict__ st, const RHdr phdr, const uint4* __restrict__ gblob,
+                int* __restrict__ err, const __grid_constant__ CUtensorMap tmap) {
+    typedef typename A::Amp Amp;
+    constexpr uint32_t AB = sizeof(Amp);
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ RHdr hdr;
+    __shared__ uint64_t full_bar[4];
+    __shared__ uint64_t tbase[4];  // base index of the tile in each buffer
+    if (threadIdx.x == 0) hdr = phdr;
+    __syncthreads();
+    unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
+    const uint32_t tile_bytes = AB << hdr.tbits;
+    const uint32_t nbuf = (uint32_t)hdr.nbuf, grid = gridDim.x;
+    uint4* blob = (uint4*)(smem + (size_t)nbuf * tile_bytes);
+    for (int i = threadIdx.x; i < hdr.blob16; i += blockDim.x) blob[i] = gblob[i];
+    const bool use_tma = hdr.use_tma != 0;
+    uint32_t t = blockIdx.x;
+    uint32_t pending = 0;  // thread 0: buffers with a load in flight
+    auto load = [&](uint32_t tt, uint32_t b) {
+        const uint64_t base = r_base(hdr, tt);
+        tbase[b] = base;
+        if (!use_tma) return;
+        tc::mbar_arrive_expect_tx(&full_bar[b], tile_bytes);
+        tma::load_boxes(&tmap, hdr.tma, base, tc::smem_u32(smem) + b * tile_bytes, tc::smem_u32(&full_bar[b]));
+        pending |= 1u << b;
+    };
+    if (threadIdx.x == 0) {
+        if (use_tma) {
+            tma::prefetch_map(&tmap);
+            for (uint32_t q = 0; q < nbuf; q++) tc::mbar_init(&full_bar[q], 1);
+        }
+        for (uint32_t q = 0; q < nbuf; q++)
+            if ((uint64_t)t + (uint64_t)q * grid < hdr.ntiles) load(t + q * grid, q);
+    }
+    __syncthreads();
+    const uint4* ops = blob + hdr.ops16;
+    const uint4* coef = blob + hdr.coef16;
+    const bool mine = threadIdx.x < (1u << (hdr.tbits - RB));
+    const int last = hdr.nsegs - 1;
+    bool dead = false;
+    uint32_t b = 0, par = 0;
+    for (; t < hdr.ntiles; t += grid) {
+        unsigned char* s = smem + (size_t)b * tile_bytes;
+        if (use_tma) {
+            if (!dead) {
+                const uint64_t t0 = reg_ns();
+                while (!tc::mbar_try_wait(&full_bar[b], par)) {
+                    if (reg_ns() - t0 > kRegWaitNs) {
+                        dead = true;
+                        atomicExch(err, 1);
+                        break;
+                    }
+                }
+                if (!dead && threadIdx.x == 0) pending &= ~(1u << b);
+            }
+        } else {
+            for (uint32_t l = threadIdx.x; l < (1u << hdr.tbits); l += blockDim.x)
+                *(Amp*)(s + rswz(l * AB)) = st[tbase[b] | r_deposit(hdr, l)];
+            __syncthreads();
+        }
+        const uint64_t base = tbase[b];
+        for (int si = 0; si <= last; si++) {
+            const uint4 sg = blob[si];
+            if (si) __syncthreads();
+            uint32_t lb;
+            Amp v[1 << RB];
+            {
+                const RPlace<RB> pl(sg, AB);
+                lb = pl.lb;
+                if (mine) {
+#pragma unroll
+                    for (int j = 0; j < (1 << RB); j++) v[j] = *(const Amp*)(s + pl.at(j));
+                }
+            }
+            if (si == last) {
+                tc::fence_proxy_async();  // this thread's writes to the buffer come before the next tile's copy
+                __syncthreads();
+                if (threadIdx.x == 0 && (uint64_t)t + (uint64_t)nbuf * grid < hdr.ntiles) load(t + nbuf * grid, b);
+            }
+            if (!mine) continue;
+            r_ops<A, EXACT, RB>(v, ops, coef, (int)sg.x, (int)sg.y, t, lb);
+            // the place again from the segment's words: kept through the ops
+            // it would take registers from the amplitudes
+            asm volatile("" ::: "memory");
+            const uint4 sg2 = blob[si];
+            const RPlace<RB> pl(sg2, AB);
+            if (si < last) {
+#pragma unroll
+                for (int j = 0; j < (1 << RB); j++) *(Amp*)(s + pl.at(j)) = v[j];
+            } else {
+                Amp* dst = st + (base | r_deposit(hdr, pl.lb));
+                uint64_t goff[RB];
+#pragma unroll
+                for (int i = 0; i < RB; i++) goff[i] = 1ull << hdr.tb[(sg2.w >> (8 * i)) & 0xffu];
+#pragma unroll
+                for (int j = 0; j < (1 << RB); j++) {
+                    uint64_t o = 0;
+#pragma unroll
+                    for (int i = 0; i < RB; i++)
+                        if (j & (1 << i)) o |= goff[i];
+                    dst[o] = v[j];
+                }
+            }
+        }
+        if (!use_tma) __syncthreads();  // the next tile's base is in place
+        b = b + 1 == nbuf ? 0u : b + 1;
+        if (b == 0) par ^= 1u;
+    }
+    if (threadIdx.x == 0) {
+        const uint64_t t0 = reg_ns();
+        for (uint32_t q = 0; q < nbuf; q++)
+            if (pending & (1u << q))
+                for (uint32_t ph = 0; ph < 2; ph++)
+                    while (!tc::mbar_try_wait(&full_bar[q], ph) && reg_ns() - t0 < kRegWaitNs) {
+                    }
+    }
+}
+
+// ================================================================= planner
+
+static uint64_t target_mask(const LGate& g) {
+    uint64_t m = 0;
+    for (int i = 0; i < g.k; i++) m |= (uint64_t)1 << g.tb[i];
+    return m;
+}
+static uint64_t qubit_mask(const LGate& g) {
+    uint64_t m = target_mask(g);
+    for (int i = 0; i < g.nc; i++) m |= (uint64_t)1 << g.cb[i];
+    return m;
+}
+// Bits that must be in the tile, and in registers: the ones a gate moves
+// amplitudes along and, where order is free, a 1-qubit diagonal's (it then
+// costs half the amplitudes and joins its neighbours).
+static uint64_t need_mask(const LGate& g, bool exact) {
+    return g.cls == GC_DIAG && !(g.k == 1 && g.nc == 0 && !exact) ? 0 : target_mask(g);
+}
+static bool is_perm(const LGate& g) { return g.cls == GC_X || g.cls == GC_SWAP; }
+
+bool reg_supported(const std::vector<LGate>& prog, uint32_t nbits) {
+    if (nbits < 4 || nbits > 33) return false;
+    for (const LGate& g : prog)
+        if ((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1)) return false;
+    return true;
+}
+
+// Which gates of a list may be taken next, scanning it in order: a gate
+// passes skipped ones only when it shares no qubit with them (and, for an
+// exact result, it or all of them are permutations).
+struct Scan {
+    bool exact;
+    uint64_t blocked = 0;
+    bool arith = false;  // some skipped gate computes
+    explicit Scan(bool e) : exact(e) {}
+    bool free(const LGate& g) const { return !(qubit_mask(g) & blocked) && (!exact || !arith || is_perm(g)); }
+    void skip(const LGate& g) {
+        blocked |= qubit_mask(g);
+        arith |= !is_perm(g);
+    }
+    bool closed(uint64_t all) const { return (blocked & all) == all; }
+};
+
+static Cx cmul(Cx a, Cx b) { return Cx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
+static Cx conj(Cx a) { return Cx{a.re, -a.im}; }
+static bool is(Cx c, double re) { return c.re == re && c.im == 0.0; }
+// a / |a|
+static Cx unit(Cx a) {
+    const double r = std::hypot(a.re, a.im);
+    return Cx{a.re / r, a.im / r};
+}
+
+namespace {
+
+// What waits to be applied on one qubit: nothing, a diagonal or a matrix.
+struct Pend {
+    bool on = false;
+    Cx m[4];
+    bool diag() const { return is(m[1], 0.0) && is(m[2], 0.0); }
+    void mul(const Cx* u) {  // m <- u m
+        if (!on) {
+            std::copy(u, u + 4, m);
+            on = true;
+            return;
+        }
+        Cx r[4];
+        for (int i = 0; i < 2; i++)
+            for (int j = 0; j < 2; j++) {
+                const Cx x = cmul(u[2 * i], m[j]), y = cmul(u[2 * i + 1], m[2 + j]);
+                r[2 * i + j] = Cx{x.re + y.re, x.im + y.im};
+            }
+        std::copy(r, r + 4, m);
+    }
+    bool unitary() const {
+        const double eps = 1e-13;
+        const double a = m[0].re * m[0].re + m[0].im * m[0].im, b = m[1].re * m[1].re + m[1].im * m[1].im,
+                     c = m[2].re * m[2].re + m[2].im * m[2].im, d = m[3].re * m[3].re + m[3].im * m[3].im;
+        const Cx x = cmul(conj(m[0]), m[1]), y = cmul(conj(m[2]), m[3]);
+        return std::fabs(a + c - 1.0) < eps && std::fabs(b + d - 1.0) < eps && std::fabs(x.re + y.re) < eps &&
+               std::fabs(x.im + y.im) < eps;
+    }
+};
+
+struct Splitter {
+    std::vector<Pend> pend;
+    std::vector<LGate>& out;
+    Cx phase{1.0, 0.0};  // of the whole state
+    Splitter(uint32_t n, std::vector<LGate>& o) : pend(n), out(o) {}
+
+    void emit1(int b, int cls, std::vector<Cx> m) {
+        LGate g;
+        g.cls = cls;
+        g.k = 1;
+        g.tb[0] = b;
+        g.m = std::move(m);
+        out.push_back(std::move(g));
+    }
+    // Applies what waits on bit b, except a diagonal when `keep_diag`
+    // (what comes next commutes with it).
+    void flush(int b, bool keep_diag) {
+        Pend& p = pend[b];
+        if (!p.on) return;
+        const Cx *m = p.m, one{1.0, 0.0}, zero{0.0, 0.0};
+        if (!p.diag()) {
+            if (is(m[0], 0.0) && is(m[3], 0.0) && is(m[1], 1.0) && is(m[2], 1.0)) {
+                emit1(b, GC_X, {});
+                p.on = false;
+                return;
+            }
+            if (!p.unitary()) {
+                emit1(b, GC_DENSE, std::vector<Cx>(m, m + 4));
+                p.on = false;
+                return;
+            }
+            // e^{i alpha} diag(1, f) [[c, -s], [s, c]] diag(1, l): the larger
+            // of a column's entries fixes its phase
+            const double c = std::hypot(m[0].re, m[0].im), s = std::hypot(m[2].re, m[2].im);
+            Cx al, f, l;
+            if (c >= s) {
+                al = unit(m[0]);
+                const Cx fl = cmul(unit(m[3]), conj(al));  // f l
+                f = s > 0.0 ? cmul(unit(m[2]), conj(al)) : fl;
+                l = cmul(fl, conj(f));
+            } else {
+                const Cx g = unit(m[2]);                               // alpha f
+                const Cx h = unit(Cx{-m[1].re, -m[1].im});             // alpha l
+                al = c > 0.0 ? unit(m[0]) : g;
+                f = cmul(g, conj(al));
+                l = cmul(h, conj(al));
+            }
+            phase = cmul(phase, al);
+            // what is left of the diagonal after it waits for the next
+            // rotation of this bit, else it joins the matrix
+            const Cx g = keep_diag ? one : f;
+            emit1(b, GC_DENSE, {Cx{c, 0.0}, Cx{-s * l.re, -s * l.im}, Cx{s * g.re, s * g.im}, cmul(cmul(g, l), Cx{c, 0.0})});
+            p.m[0] = one;
+            p.m[1] = p.m[2] = zero;
+            p.m[3] = f;
+            p.on = keep_diag && !is(f, 1.0);
+            return;
+        }
+        if (keep_diag || !p.on) return;
+        if (p.unitary()) {
+            phase = cmul(phase, p.m[0]);
+            p.m[3] = cmul(p.m[3], conj(p.m[0]));
+            p.m[0] = one;
+        }
+        if (!(is(p.m[0], 1.0) && is(p.m[3], 1.0))) emit1(b, GC_DIAG, {p.m[0], p.m[3]});
+        p.on = false;
+    }
+};
+
+}  // namespace
+
+void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vector<LGate>& out) {
+    out.clear();
+    Splitter sp(nbits, out);
+    auto single = [](const LGate& g) { return g.k == 1 && g.nc == 0; };
+    // per gate: whether the next gate on its target that is no 1-qubit
+    // diagonal is a 1-qubit rotation
+    std::vector<char> rot_next(prog.size(), 0), next(nbits, 0);
+    for (size_t i = prog.size(); i-- > 0;) {
+        const LGate& g = prog[i];
+        rot_next[i] = next[g.tb[0]];
+        if (single(g)) {
+            if (g.cls == GC_DENSE) next[g.tb[0]] = 1;
+            continue;
+        }
+        for (int q = 0; q < g.k; q++) next[g.tb[q]] = 0;
+        for (int q = 0; q < g.nc; q++) next[g.cb[q]] = 0;
+    }
+    const double h = std::sqrt(0.5);
+    const Cx had[4] = {{h, 0.0}, {h, 0.0}, {h, 0.0}, {-h, 0.0}};
+    for (size_t i = 0; i < prog.size(); i++) {
+        const LGate& g = prog[i];
+        if (single(g)) {
+            Cx u[4] = {{0, 0}, {1, 0}, {1, 0}, {0, 0}};  // GC_X
+            if (g.cls == GC_DENSE) {
+                std::copy(g.m.begin(), g.m.begin() + 4, u);
+            } else if (g.cls == GC_DIAG) {
+                u[0] = g.m[0];
+                u[1] = u[2] = Cx{0, 0};
+                u[3] = g.m[1];
+            }
+            sp.pend[g.tb[0]].mul(u);
+            continue;
+        }
+        const int t = g.tb[0];
+        if (g.cls == GC_X && g.nc == 1 && rot_next[i] && sp.pend[t].on && !sp.pend[t].diag() && sp.pend[t].unitary()) {
+            sp.pend[t].mul(had);
+            sp.flush(t, true);
+            sp.flush(g.cb[0], true);
+            LGate z;
+            z.cls = GC_DIAG;
+            z.k = 2;
+            z.tb[0] = std::min(t, (int)g.cb[0]);
+            z.tb[1] = std::max(t, (int)g.cb[0]);
+            z.m.assign(4, Cx{1.0, 0.0});
+            z.m[g.cv[0] ? 3 : (t == z.tb[0] ? 1 : 2)] = Cx{-1.0, 0.0};
+            out.push_back(std::move(z));
+            sp.pend[t].mul(had);
+            continue;
+        }
+        for (int q = 0; q < g.k; q++) sp.flush(g.tb[q], g.cls == GC_DIAG);
+        for (int q = 0; q < g.nc; q++) sp.flush(g.cb[q], true);
+        out.push_back(g);
+    }
+    for (uint32_t b = 0; b < nbits; b++) sp.flush((int)b, false);
+    // the state's phase joins the last phase gate, else the last matrix
+    if (is(sp.phase, 1.0)) return;
+    for (int cls : {(int)GC_DIAG, (int)GC_DENSE})
+        for (size_t i = out.size(); i-- > 0;)
+            if (out[i].cls == cls && out[i].nc == 0) {
+                for (Cx& x : out[i].m) x = cmul(x, sp.phase);
+                return;
+            }
+    sp.emit1(0, GC_DIAG, {sp.phase, sp.phase});
+}
+
+// Description of a pass kept below this, so that three CTAs of 2^11
+// complex128 amplitudes (two buffers each) share an SM; a longer run of
+// gates becomes further passes.
+constexpr size_t kRegBlobCap = 8 * 1024;
+
+namespace {
+
+// Gates of one segment and the register positions they need.
+struct SegPlan {
+    std::vector<const LGate*> gates;
+    std::vector<int> bits;                    // tile positions in registers
+    std::vector<std::pair<int, int>> pairs;   // (even, odd) register positions of 2-qubit dense gates and swaps
+};
+
+// -1 where two bits have their values; a bit is a tile position, or 16 + a
+// bit of the tile's number.
+struct Sign {
+    int bit[2], val[2];
+};
+
+struct PassBuilder {
+    int rb;
+    bool exact;
+    int8_t local[64];     // global bit -> tile position, -1 outside
+    int8_t outside[64];   // global bit -> bit of the tile's number
+    RegPass* p;
+
+    bool fits(const SegPlan& s, const LGate& g) const {
+        if (!need_mask(g, exact)) return true;
+        int fresh = 0;
+        for (int i = 0; i < g.k; i++)
+            if (std::find(s.bits.begin(), s.bits.end(), (int)local[g.tb[i]]) == s.bits.end()) fresh++;
+        if ((int)s.bits.size() + fresh > rb) return false;
+        if (g.k == 1) return true;
+        const int a = local[g.tb[0]], b = local[g.tb[1]];
+        for (const auto& q : s.pairs) {
+            if (q.first == a && q.second == b) return true;
+            if (g.cls == GC_SWAP && q.first == b && q.second == a) return true;
+            if (q.first == a || q.second == a || q.first == b || q.second == b) return false;
+        }
+        return (int)s.pairs.size() < rb / 2;
+    }
+    void add(SegPlan& s, const LGate& g) const {
+        s.gates.push_back(&g);
+        if (!need_mask(g, exact)) return;
+        for (int i = 0; i < g.k; i++)
+            if (std::find(s.bits.begin(), s.bits.end(), (int)local[g.tb[i]]) == s.bits.end())
+                s.bits.push_back(local[g.tb[i]]);
+        if (g.k == 2) {
+            const int a = local[g.tb[0]], b = local[g.tb[1]];
+            for (const auto& q : s.pairs)
+                if (q.first == a || q.first == b) return;
+            s.pairs.push_back({a, b});
+        }
+    }
+    void emit(const SegPlan& s) {
+        RSeg sg;
+        memset(&sg, 0, sizeof(sg));
+        std::vector<int> order;
+        for (const auto& q : s.pairs) {
+            order.push_back(q.first);
+            order.push_back(q.second);
+        }
+        for (int b : s.bits)
+            if (std::find(order.begin(), order.end(), b) == order.end()) order.push_back(b);
+        // unused register positions: the highest free tile bits, so that the
+        // lanes of a warp step through the low ones
+        for (int b = p->tbits - 1; (int)order.size() < rb && b >= 0; b--)
+            if (std::find(order.begin(), order.end(), b) == order.end()) order.push_back(b);
+        std::vector<int> sorted(order);
+        std::sort(sorted.begin(), sorted.end());
+        for (int i = 0; i < rb; i++) {
+            sg.sorted[i] = (int8_t)sorted[i];
+            sg.order[i] = (int8_t)order[i];
+        }
+        auto pos = [&](int l) -> int {
+            const auto it = std::find(order.begin(), order.end(), l);
+            return it == order.end() ? -1 : (int)(it - order.begin());
+        };
+        sg.op_begin = (int32_t)p->ops.size();
+        const uint32_t na = 1u << rb;
+        // A diagonal under way (not in exact passes): a table over the
+        // register index and at most one bit outside the registers, dep the
+        // register positions it depends on.  Diagonals commute with each
+        // other, so it is applied when a gate moves one of those positions.
+        struct {
+            bool on = false;
+            uint32_t dep = 0;
+            int sel = -1;
+            std::vector<Cx> tab;
+        } acc;
+        auto push = [&](uint32_t code, uint32_t jm, const ROp& base) {
+            ROp op = base;
+            if (code == RC_PHASE && !op.ctl && !op.gmask)
+                for (int q = 0; q < rb; q++) {
+                    uint32_t bit = 0;
+                    for (uint32_t j = 0; j < na; j++) bit |= ((j >> q) & 1u) << j;
+                    if (jm == bit) code = RC_PHASE1 + (uint32_t)q;
+                }
+            op.head = code | (jm << 16);
+            p->ops.push_back(op);
+        };
+        auto flush = [&]() {
+            if (!acc.on) return;
+            acc.on = false;
+            const uint32_t ne = acc.sel >= 0 ? 2 : 1;
+            uint32_t jm = 0;
+            for (uint32_t j = 0; j < na; j++)
+                for (uint32_t e = 0; e < ne; e++)
+                    if (!is(acc.tab[e * na + j], 1.0)) jm |= 1u << j;
+            if (!jm) return;
+            bool same = true;  // one coefficient for every amplitude it changes
+            const uint32_t j0 = (uint32_t)__builtin_ctz(jm);
+            for (uint32_t j = 0; j < na; j++)
+                for (uint32_t e = 0; e < ne; e++)
+                    if ((jm >> j) & 1)
+                        same &= acc.tab[e * na + j].re == acc.tab[e * na + j0].re && acc.tab[e * na + j].im == acc.tab[e * na + j0].im;
+            ROp op;
+            memset(&op, 0, sizeof(op));
+            op.coef = (uint32_t)p->coef.size();
+            if (acc.sel >= 0) {
+                op.sel0 = (uint32_t)acc.sel;
+                op.sel1 = 1u << 8;
+            }
+            if (same)
+                for (uint32_t e = 0; e < ne; e++) p->coef.push_back(acc.tab[e * na + j0]);
+            else
+                p->coef.insert(p->coef.end(), acc.tab.begin(), acc.tab.begin() + ne * na);
+            push(same ? RC_PHASE : RC_DIAG, jm, op);
+        };
+        // Signs under way (not in exact passes): -1 where both tile positions
+        // / outside bits have their values.  The next rotation of a register
+        // position takes it along; otherwise it becomes an RC_NEG op.
+        std::vector<Sign> signs;
+        auto flush_sign = [&](const Sign& z) {
+            ROp op;
+            memset(&op, 0, sizeof(op));
+            uint32_t jm = (1u << na) - 1;
+            for (int q = 0; q < 2; q++) {
+                if (z.bit[q] >= 16) {
+                    op.gmask |= 1u << (z.bit[q] - 16);
+                    op.gval |= (uint32_t)z.val[q] << (z.bit[q] - 16);
+                } else if (pos(z.bit[q]) >= 0) {
+                    for (uint32_t j = 0; j < na; j++)
+                        if (((j >> pos(z.bit[q])) & 1u) != (uint32_t)z.val[q]) jm &= ~(1u << j);
+                } else {
+                    op.ctl |= (1u << z.bit[q]) | ((uint32_t)z.val[q] << (16 + z.bit[q]));
+                }
+            }
+            push(RC_NEG, jm, op);
+        };
+        for (const LGate* g : s.gates) {
+            ROp op;
+            memset(&op, 0, sizeof(op));
+            uint32_t rmask = 0, rval = 0, tmask = 0, tval = 0;
+            for (int c = 0; c < g->nc; c++) {
+                const int l = local[g->cb[c]];
+                if (l < 0) {
+                    op.gmask |= 1u << outside[g->cb[c]];
+                    op.gval |= (uint32_t)(g->cv[c] ? 1 : 0) << outside[g->cb[c]];
+                } else if (pos(l) >= 0) {
+                    rmask |= 1u << pos(l);
+                    rval |= (uint32_t)(g->cv[c] ? 1 : 0) << pos(l);
+                } else {
+                    tmask |= 1u << l;
+                    tval |= (uint32_t)(g->cv[c] ? 1 : 0) << l;
+                }
+            }
+            op.ctl = tmask | (tval << 16);
+            op.coef = (uint32_t)p->coef.size();
+            if (g->cls == GC_DIAG) {
+                Sign z;
+                if (!exact && two_bit_sign(*g, z))
+                    signs.push_back(z);
+                else
+                    diagonal(*g, op, rmask, rval, na, pos, acc, flush, push);
+                continue;
+            }
+            uint32_t bm = 0, jm = 0, pairs = 0;
+            for (int i = 0; i < g->k; i++) bm |= 1u << pos(local[g->tb[i]]);
+            for (uint32_t j = 0; j < na; j++)
+                if (!(j & bm)) {
+                    pairs |= 1u << j;
+                    if ((j & rmask) == rval) jm |= 1u << j;
+                }
+            if (acc.on && (acc.dep & bm)) flush();
+            const uint32_t p0 = (uint32_t)pos(local[g->tb[0]]);
+            const bool matrix = g->cls == GC_DENSE && g->k == 1 && g->nc == 0 && !exact;
+            bool cond = false;  // the op's controls are taken by a sign
+            for (size_t q = 0; q < signs.size();) {
+                const Sign z = signs[q];
+                int hit = -1;  // the sign's half that this gate moves
+                for (int i = 0; i < g->k; i++)
+                    for (int w = 0; w < 2; w++)
+                        if (z.bit[w] == (int)local[g->tb[i]]) hit = w;
+                if (hit < 0) {
+                    q++;
+                    continue;
+                }
+                signs.erase(signs.begin() + q);
+                const int o = z.bit[1 - hit], ov = z.val[1 - hit];
+                if (!matrix || z.val[hit] != 1) {
+                    flush_sign(z);
+                } else if (o < 16 && pos(o) >= 0) {
+                    for (uint32_t j = 0; j < na; j++)
+                        if (((pairs >> j) & 1u) && ((j >> pos(o)) & 1u) == (uint32_t)ov) op.sign ^= 1u << j;
+                } else if (!cond) {
+                    cond = true;
+                    if (o < 16) {
+                        op.ctl = (1u << o) | ((uint32_t)ov << (16 + o));
+                    } else {
+                        op.gmask = 1u << (o - 16);
+                        op.gval = (uint32_t)ov << (o - 16);
+                    }
+                    op.sign |= pairs << 16;
+                } else {
+                    flush_sign(z);
+                }
+            }
+            op.coef = (uint32_t)p->coef.size();
+            uint32_t code;
+            auto is_real = [&](int i) { return g->m[i].im == 0.0; };
+            auto two = [&](int i, int j) { p->coef.push_back(Cx{g->m[i].re, g->m[j].re}); };
+            if (matrix && is_real(0) && is_real(1) && is_real(2) && is_real(3)) {
+                code = RC_REAL1 + p0;
+                two(0, 1);
+                two(2, 3);
+            } else if (matrix && is_real(0) && is_real(2)) {
+                code = RC_RCOL1 + p0;
+                two(0, 2);
+                p->coef.push_back(g->m[1]);
+                p->coef.push_back(g->m[3]);
+            } else if (matrix && is_real(0) && is_real(1)) {
+                code = RC_RROW1 + p0;
+                two(0, 1);
+                p->coef.push_back(g->m[2]);
+                p->coef.push_back(g->m[3]);
+            } else {
+                if (g->k == 1)
+                    code = (g->cls == GC_X ? RC_X : g->nc == 0 ? RC_DENSE1 : RC_MASKED1) + p0;
+                else
+                    code = (g->cls == GC_SWAP ? RC_SWAP : RC_DENSE2) + p0 / 2;
+                for (const Cx& c : g->m) p->coef.push_back(c);
+            }
+            push(code, jm, op);
+        }
+        for (const Sign& z : signs) flush_sign(z);
+        flush();
+        sg.op_end = (int32_t)p->ops.size();
+        if (sg.op_end > sg.op_begin) p->segs.push_back(sg);
+    }
+
+    // A CZ (one control or two targets, one entry -1, the others 1).
+    bool two_bit_sign(const LGate& g, Sign& z) const {
+        if (g.k + g.nc != 2) return false;
+        int minus = -1;
+        for (size_t i = 0; i < g.m.size(); i++) {
+            if (is(g.m[i], 1.0)) continue;
+            if (!is(g.m[i], -1.0) || minus >= 0) return false;
+            minus = (int)i;
+        }
+        if (minus < 0) return false;
+        auto where = [&](int b) { return local[b] >= 0 ? (int)local[b] : 16 + (int)outside[b]; };
+        for (int q = 0; q < g.k; q++) {
+            z.bit[q] = where(g.tb[q]);
+            z.val[q] = (minus >> q) & 1;
+        }
+        if (g.nc) {
+            z.bit[1] = where(g.cb[0]);
+            z.val[1] = g.cv[0] ? 1 : 0;
+        }
+        return true;
+    }
+
+    // A diagonal gate: signs become RC_NEG ops; otherwise it joins the
+    // diagonal under way or, in exact passes and when it depends on more
+    // than one bit outside the registers, becomes one RC_PHASE op per
+    // combination of its register targets.
+    template <typename Pos, typename Acc, typename Flush, typename Push>
+    void diagonal(const LGate& g, const ROp& base, uint32_t rmask, uint32_t rval, uint32_t na, const Pos& pos, Acc& acc,
+                  const Flush& flush, const Push& push) {
+        uint32_t dmask = 0;  // entry bits held in registers
+        std::vector<int> sel, selbit;
+        for (int i = 0; i < g.k; i++) {
+            const int l = local[g.tb[i]];
+            if (l >= 0 && pos(l) >= 0) {
+                dmask |= 1u << i;
+            } else {
+                sel.push_back(l >= 0 ? l : 16 + outside[g.tb[i]]);
+                selbit.push_back(i);
+            }
+        }
+        auto entry = [&](uint32_t reg, uint32_t e) {  // register part of the entry index, entry of the selected bits
+            uint32_t x = reg;
+            for (size_t q = 0; q < sel.size(); q++) x |= ((e >> q) & 1u) << selbit[q];
+            return g.m[x];
+        };
+        auto reg_part = [&](uint32_t j) {
+            uint32_t x = 0;
+            for (int i = 0; i < g.k; i++)
+                if (dmask & (1u << i)) x |= ((j >> pos(local[g.tb[i]])) & 1u) << i;
+            return x;
+        };
+        bool signs = true;
+        for (const Cx& c : g.m) signs &= c.im == 0.0 && (c.re == 1.0 || c.re == -1.0);
+        const bool ctl_outside = base.ctl || base.gmask;
+        uint32_t dep = rmask;
+        for (int i = 0; i < g.k; i++)
+            if (dmask & (1u << i)) dep |= 1u << pos(local[g.tb[i]]);
+        // a control outside the registers is one more selected bit
+        const int nsel = (int)sel.size() + __builtin_popcount(base.ctl & 0xffffu) + __builtin_popcount(base.gmask);
+        int one = -1;
+        if (nsel == 1) one = !sel.empty() ? sel[0] : (base.ctl & 0xffffu) ? __builtin_ctz(base.ctl & 0xffffu) : 16 + __builtin_ctz(base.gmask);
+        if (!exact && !(signs && nsel > 0) && nsel <= 1) {
+            if (acc.on && one >= 0 && acc.sel >= 0 && acc.sel != one) flush();
+            if (!acc.on) {
+                acc.on = true;
+                acc.dep = 0;
+                acc.sel = -1;
+                acc.tab.assign(2 * na, Cx{1.0, 0.0});
+            }
+            if (one >= 0) acc.sel = one;
+            acc.dep |= dep;
+            const uint32_t cval = ctl_outside ? ((base.ctl >> 16) || base.gval ? 1u : 0u) : 0u;
+            for (uint32_t e = 0; e < 2; e++)
+                for (uint32_t j = 0; j < na; j++) {
+                    if ((j & rmask) != rval || (ctl_outside && e != cval)) continue;
+                    Cx& x = acc.tab[e * na + j];
+                    x = cmul(x, entry(reg_part(j), sel.empty() ? 0u : e));
+                }
+            return;
+        }
+        for (uint32_t s2 = 0; s2 < (1u << g.k); s2++) {
+            if (s2 & ~dmask) continue;
+            uint32_t jm = 0;
+            for (uint32_t j = 0; j < na; j++)
+                if ((j & rmask) == rval && reg_part(j) == s2) jm |= 1u << j;
+            if (!jm) continue;
+            const uint32_t ne = 1u << sel.size();
+            if (signs) {
+                for (uint32_t e = 0; e < ne; e++) {
+                    if (entry(s2, e).re == 1.0) continue;
+                    ROp op = base;
+                    for (size_t q = 0; q < sel.size(); q++) {
+                        const uint32_t bit = (e >> q) & 1u;
+                        if (sel[q] < 16)
+                            op.ctl |= (1u << sel[q]) | (bit << (16 + sel[q]));
+                        else {
+                            op.gmask |= 1u << (sel[q] - 16);
+                            op.gval |= bit << (sel[q] - 16);
+                        }
+                    }
+                    push(RC_NEG, jm, op);
+                }
+                continue;
+            }
+            ROp op = base;
+            op.coef = (uint32_t)p->coef.size();
+            bool any = false;
+            for (uint32_t e = 0; e < ne; e++) {
+                any |= !is(entry(s2, e), 1.0);
+                p->coef.push_back(entry(s2, e));
+            }
+            if (!any) {
+                p->coef.resize(op.coef);
+                continue;
+            }
+            for (size_t q = 0; q < sel.size(); q++) {
+                if (q < 5)
+                    op.sel0 |= (uint32_t)sel[q] << (6 * q);
+                else
+                    op.sel1 |= (uint32_t)sel[q];
+            }
+            op.sel1 |= (uint32_t)sel.size() << 8;
+            push(RC_PHASE, jm, op);
+        }
+    }
+};
+
+size_t pass_bytes(const RegPass& p, size_t coef_bytes) {
+    return p.segs.size() * sizeof(RSeg) + p.ops.size() * sizeof(ROp) + p.coef.size() * coef_bytes;
+}
+
+}  // namespace
+
+void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits_max, bool exact,
+              RegPlan& out) {
+    out.passes.clear();
+    out.blob.clear();
+    const size_t amp = precision == YAO_C128 ? 16 : 8, coef_bytes = precision == YAO_C128 ? 16 : 32;
+    const int low = precision == YAO_C128 ? 3 : 4;  // 128-byte runs: the tile's lowest bits
+    const int tbits = std::min((int)nbits, tbits_max);
+    const bool whole = (int)nbits <= tbits;
+    const uint64_t lowmask = whole ? 0 : ((1ull << low) - 1), all = (1ull << nbits) - 1;
+    const int cap = whole ? (int)nbits : tbits - low;
+    // Amplitudes a thread: 16 once the tiles fill the GPU twice over, else 4
+    // (8 in a 2^12 tile: at most 512 threads), which shortens an op's chain
+    // where the time of one CTA is the time of the pass.
+    const uint64_t ntiles = 1ull << (nbits - tbits);
+    const int rb = ntiles >= 296 ? 4 : (tbits > 11 ? 3 : 2);
+    std::vector<char> used(prog.size(), 0);
+    size_t i0 = 0, left = prog.size();
+    while (left) {
+        // the gates of this pass
+        std::vector<const LGate*> run;
+        std::vector<size_t> at;
+        uint64_t hi = 0;
+        {
+            Scan sc(exact);
+            for (size_t j = i0; j < prog.size() && !sc.closed(all); j++) {
+                if (used[j]) continue;
+                const LGate& g = prog[j];
+                const uint64_t nh = hi | (need_mask(g, exact) & ~lowmask);
+                if (!sc.free(g) || __builtin_popcountll(nh) > cap) {
+                    sc.skip(g);
+                    continue;
+                }
+                hi = nh;
+                run.push_back(&g);
+                at.push_back(j);
+            }
+        }
+        uint64_t tile = hi | lowmask;
+        for (uint32_t b = 0; __builtin_popcountll(tile) < tbits; b++) tile |= 1ull << b;
+        RegPass p;
+        p.tbits = tbits;
+        p.rb = rb;
+        p.ntiles = ntiles;
+        PassBuilder pb;
+        pb.rb = rb;
+        pb.exact = exact;
+        int nt = 0, no = 0;
+        for (uint32_t b = 0; b < 64; b++) {
+            pb.local[b] = pb.outside[b] = -1;
+            if (b >= nbits) continue;
+            if ((tile >> b) & 1) {
+                p.tb[nt] = (int8_t)b;
+                pb.local[b] = (int8_t)nt++;
+            } else {
+                pb.outside[b] = (int8_t)no++;
+            }
+        }
+        pb.p = &p;
+        // its segments, until the description is full
+        std::vector<char> done(run.size(), 0);
+        size_t ndone = 0, first = 0;
+        while (ndone < run.size()) {
+            SegPlan s;
+            Scan sc(exact);
+            std::vector<size_t> took;
+            size_t bytes = pass_bytes(p, coef_bytes) + sizeof(RSeg);
+            bool full = false;
+            for (size_t j = first; j < run.size() && !full && !sc.closed(all); j++) {
+                if (done[j]) continue;
+                const LGate& g = *run[j];
+                if (!sc.free(g) || !pb.fits(s, g)) {
+                    sc.skip(g);
+                    continue;
+                }
+                // a diagonal may become one op per combination of its register targets
+                const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) +
+                                  g.m.size() * coef_bytes;
+                if (bytes + nb > kRegBlobCap && !(p.ops.empty() && s.gates.empty())) {
+                    full = true;
+                    break;
+                }
+                bytes += nb;
+                pb.add(s, g);
+                took.push_back(j);
+            }
+            if (took.empty()) break;  // the description is full
+            pb.emit(s);
+            for (size_t j : took) done[j] = 1;
+            ndone += took.size();
+            while (first < run.size() && done[first]) first++;
+            if (full) break;
+        }
+        for (size_t j = 0; j < run.size(); j++)
+            if (done[j]) {
+                used[at[j]] = 1;
+                left--;
+            }
+        while (i0 < prog.size() && used[i0]) i0++;
+        if (p.ops.empty()) continue;
+        // the tile leaves from the last segment's registers: whole 128-byte
+        // runs a warp need the low positions on the lanes
+        if (tbits - rb >= low) {
+            bool lowest = false;
+            for (int q = 0; q < rb; q++) lowest |= p.segs.back().sorted[q] < low;
+            if (lowest) {
+                RSeg sg;
+                memset(&sg, 0, sizeof(sg));
+                sg.op_begin = sg.op_end = (int32_t)p.ops.size();
+                for (int q = 0; q < rb; q++) sg.sorted[q] = sg.order[q] = (int8_t)(tbits - rb + q);
+                p.segs.push_back(sg);
+            }
+        }
+        out.passes.push_back(std::move(p));
+    }
+    // one packed description for the whole plan
+    size_t total = 0;
+    for (RegPass& p : out.passes) {
+        p.blob_off = total;
+        p.blob_bytes = pass_bytes(p, coef_bytes);
+        total += (p.blob_bytes + 255) / 256 * 256;
+    }
+    out.blob.assign(total, 0);
+    for (RegPass& p : out.passes) {
+        unsigned char* d = out.blob.data() + p.blob_off;
+        memcpy(d, p.segs.data(), p.segs.size() * sizeof(RSeg));
+        d += p.segs.size() * sizeof(RSeg);
+        memcpy(d, p.ops.data(), p.ops.size() * sizeof(ROp));
+        d += p.ops.size() * sizeof(ROp);
+        for (const Cx& c : p.coef) {
+            if (amp == 16) {
+                memcpy(d, &c, 16);
+            } else {
+                const float hr = (float)c.re, hi = (float)c.im;
+                const float f[8] = {hr, hr, hi, hi, (float)(c.re - (double)hr), (float)(c.re - (double)hr),
+                                    (float)(c.im - (double)hi), (float)(c.im - (double)hi)};
+                memcpy(d, f, 32);
+            }
+            d += coef_bytes;
+        }
+    }
+}
+
+// ================================================================== launch
+
+template <typename A, bool EXACT, int RB>
+static int launch_k(Ctx* ctx, void* st, RHdr& hdr, const uint4* blob, size_t blob_bytes, const CUtensorMap& tmap) {
+    auto kern = k_reg_tiles<A, EXACT, RB>;
+    static int optin = 0, sm_total = 0, fixed = 0;
+    if (!optin) {
+        int dev = 0, v = 0;
+        YAO_CUDA(cudaGetDevice(&dev));
+        YAO_CUDA(cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        cudaFuncAttributes fa;
+        YAO_CUDA(cudaFuncGetAttributes(&fa, kern));
+        fixed = (int)fa.sharedSizeBytes;
+        YAO_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, v - fixed));
+        YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        optin = v;
+    }
+    const size_t tile = sizeof(typename A::Amp) << hdr.tbits;
+    const unsigned threads = std::max(32u, 1u << (hdr.tbits - RB));
+    // as many CTAs as the registers allow, then as many tile buffers as fit
+    auto ctas = [&](int nbuf) {
+        const size_t per = (size_t)nbuf * tile + blob_bytes + 1024 + fixed + 1024;
+        const size_t limit = (size_t)reg_ctas<A, RB>() * reg_threads<A, RB>() / threads;
+        return std::min<size_t>((size_t)sm_total / per, std::max<size_t>(1, limit));
+    };
+    hdr.nbuf = 1;
+    while (hdr.use_tma && hdr.nbuf < 4 && ctas(hdr.nbuf + 1) == ctas(hdr.nbuf)) hdr.nbuf++;
+    const size_t smem = (size_t)hdr.nbuf * tile + blob_bytes + 1024;
+    if (smem + fixed > (size_t)optin) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
+    int per_sm = 0;
+    YAO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
+    if (per_sm < 1) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
+    const unsigned grid = (unsigned)std::min<uint64_t>(hdr.ntiles, (uint64_t)per_sm * (uint64_t)ctx->num_sms);
+    kern<<<grid, threads, smem, ctx->stream>>>((typename A::Amp*)st, hdr, blob, ctx->d_err, tmap);
+    return YAO_OK;
+}
+
+template <typename A, bool EXACT>
+static int launch_rb(Ctx* ctx, void* st, int rb, RHdr& hdr, const uint4* blob, size_t bytes, const CUtensorMap& tmap) {
+    if (rb == 4) return launch_k<A, EXACT, 4>(ctx, st, hdr, blob, bytes, tmap);
+    if (rb == 3) return launch_k<A, EXACT, 3>(ctx, st, hdr, blob, bytes, tmap);
+    return launch_k<A, EXACT, 2>(ctx, st, hdr, blob, bytes, tmap);
+}
+
+int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
+               size_t step) {
+    if (plan.passes.empty()) return YAO_OK;
+    if (!ctx->d_err) {
+        YAO_CUDA(cudaMalloc((void**)&ctx->d_err, sizeof(int)));
+        YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+    }
+    unsigned char* dblob = nullptr;
+    YAO_CUDA(cudaMallocAsync((void**)&dblob, plan.blob.size(), ctx->stream));
+    YAO_CUDA(cudaMemcpyAsync(dblob, plan.blob.data(), plan.blob.size(), cudaMemcpyHostToDevice, ctx->stream));
+    const size_t amp = precision == YAO_C128 ? 16 : 8;
+    int s = YAO_OK;
+    for (size_t i = first; i < plan.passes.size() && !s; i += step) {
+        const RegPass& p = plan.passes[i];
+        RHdr h;
+        memset(&h, 0, sizeof(h));
+        h.tbits = p.tbits;
+        h.nsegs = (int32_t)p.segs.size();
+        h.blob16 = (int32_t)(p.blob_bytes / 16);
+        h.ops16 = (int32_t)(p.segs.size() * sizeof(RSeg) / 16);
+        h.coef16 = h.ops16 + (int32_t)(p.ops.size() * sizeof(ROp) / 16);
+        h.ntiles = (uint32_t)p.ntiles;
+        memcpy(h.tb, p.tb, sizeof(h.tb));
+        CUtensorMap tmap;
+        memset(&tmap, 0, sizeof(tmap));
+        h.use_tma = tma_enabled() && tma_make_plan(p.tb, p.tbits, nbits, amp, st, h.tma, &tmap) ? 1 : 0;
+        const uint4* blob = (const uint4*)(dblob + p.blob_off);
+        {
+            ProfScope prof(ctx, exact ? "reg_pass_exact" : "reg_pass_fused",
+                           (double)p.ntiles * (double)((uint64_t)1 << p.tbits) * 2.0 * (double)amp);
+            if (precision == YAO_C128)
+                s = exact ? launch_rb<A128<true>, true>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap)
+                          : launch_rb<A128<false>, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap);
+            else
+                s = launch_rb<A64, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap);
+        }
+        ctx->launches++;
+        if (!s && cudaPeekAtLastError() != cudaSuccess) s = cuda_fail(cudaGetLastError(), "register pass launch");
+    }
+    cudaFreeAsync(dblob, ctx->stream);
+    return s;
+}
+
+}  // namespace yao

@@ -35,6 +35,7 @@
 #include <cudaTypedefs.h>
 
 #include "device_common.cuh"
+#include "reg_tiles.h"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -2131,6 +2132,7 @@ struct TileConfig {
     int tbits = 0;
     int rb = 0;
     int tc = 1;  // complex64 FUSED: dense 3..5-qubit blocks may go to the tensor cores
+    int reg = 0; // register passes (reg_tiles.h): k = 1 keeps 2-qubit gates apart, k = 2 fuses into 2-qubit blocks
 };
 
 // FP32 -> TF32, round to nearest even (low 13 mantissa bits cleared)
@@ -2235,6 +2237,20 @@ static void plan_run(uint32_t nbits, const std::vector<LGate>& prog, int32_t mod
     }
 }
 
+// The register-pass plan of a run (cfg.reg); false when a gate does not fit.
+static bool plan_reg_run(uint32_t nbits, int32_t precision, const std::vector<LGate>& prog, int32_t mode,
+                         const TileConfig& cfg, RegPlan& out) {
+    std::vector<LGate> work;
+    if (mode == YAO_MODE_FUSED && cfg.k > 1)
+        fuse_blocks(prog, nbits, 2, work);
+    else if (mode == YAO_MODE_FUSED)
+        split_single_qubit(prog, nbits, work);
+    const std::vector<LGate>& w = mode == YAO_MODE_FUSED ? work : prog;
+    if (!reg_supported(w, nbits)) return false;
+    reg_plan(w, nbits, precision, cfg.tbits, mode == YAO_MODE_TILED, out);
+    return true;
+}
+
 // Launches passes[first], passes[first + step], ... of a plan.
 template <typename V>
 static int launch_passes(Ctx* ctx, V* st, uint32_t nbits, int32_t precision, int32_t mode,
@@ -2257,10 +2273,16 @@ static int launch_passes(Ctx* ctx, V* st, uint32_t nbits, int32_t precision, int
 template <typename V>
 static int run_program_cfg(Ctx* ctx, V* st, uint32_t nbits, int32_t precision, const std::vector<LGate>& prog,
                            int32_t mode, const TileConfig& cfg, bool check_err = true) {
-    std::vector<PassPlan> passes;
     bool any_tc = false;
-    plan_run<V>(nbits, prog, mode, cfg, passes, &any_tc);
-    int s = launch_passes<V>(ctx, st, nbits, precision, mode, passes);
+    int s;
+    RegPlan rplan;
+    if (cfg.reg && plan_reg_run(nbits, precision, prog, mode, cfg, rplan)) {
+        s = reg_launch(ctx, st, nbits, precision, mode == YAO_MODE_TILED && sizeof(V) == 16, rplan, 0, 1);
+    } else {
+        std::vector<PassPlan> passes;
+        plan_run<V>(nbits, prog, mode, cfg, passes, &any_tc);
+        s = launch_passes<V>(ctx, st, nbits, precision, mode, passes);
+    }
     if (s) return s;
     ctx->tc_used = any_tc;
     // a bounded wait of some pass (a tile's TMA copies, a tensor-core
@@ -2290,7 +2312,7 @@ static int run_program_cfg(Ctx* ctx, V* st, uint32_t nbits, int32_t precision, c
 // time scaled by passes / sampled passes estimates the run.  The fastest is
 // kept per (device, qubits, precision, mode, requested k).  Choices live in
 // memory and, when YAO_TUNE_CACHE names a file, in that file (one
-// "key k tbits rb tc" line per entry).  YAO_TILE_BITS / YAO_REG_BITS pin the
+// "key k tbits rb tc" line per entry; tc + 2 for register passes).  YAO_TILE_BITS / YAO_REG_BITS pin the
 // shape and YAO_AUTOTUNE=0 turns tuning off (defaults below).
 
 static std::mutex g_tune_mu;
@@ -2334,7 +2356,11 @@ static void tune_load_locked() {
     char line[256], key[128];
     while (fgets(line, sizeof(line), f)) {
         TileConfig c;
-        if (sscanf(line, "%127s %d %d %d %d", key, &c.k, &c.tbits, &c.rb, &c.tc) == 5) g_tune[key] = c;
+        if (sscanf(line, "%127s %d %d %d %d", key, &c.k, &c.tbits, &c.rb, &c.tc) == 5) {
+            c.reg = (c.tc >> 1) & 1;
+            c.tc &= 1;
+            g_tune[key] = c;
+        }
     }
     fclose(f);
 }
@@ -2345,7 +2371,8 @@ static void tune_store_locked() {
     FILE* f = fopen(path, "w");
     if (!f) return;
     for (const auto& kv : g_tune)
-        fprintf(f, "%s %d %d %d %d\n", kv.first.c_str(), kv.second.k, kv.second.tbits, kv.second.rb, kv.second.tc);
+        fprintf(f, "%s %d %d %d %d\n", kv.first.c_str(), kv.second.k, kv.second.tbits, kv.second.rb,
+                kv.second.tc | kv.second.reg << 1);
     fclose(f);
 }
 
@@ -2399,6 +2426,44 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
     *best_ms = -1.0;
     const uint32_t n = r->nbits;
     if (prog.empty()) return YAO_OK;
+    // A program of 1- and 2-qubit gates (after fusion into 2-qubit blocks):
+    // register passes, gates apart (k = 1) or fused (k = 2), and the block
+    // form that was fastest where those do not apply.  Other programs, and
+    // widths asked for above 2: every block shape.  Tiles of 2^11 complex128
+    // and 2^12 complex64 amplitudes (see reg_tiles.cu).
+    bool reg = false;
+    if (mode == YAO_MODE_TILED) {
+        reg = reg_supported(prog, n);
+    } else if (kreq <= 2) {
+        std::vector<LGate> w2;
+        fuse_blocks(prog, n, 2, w2);
+        reg = reg_supported(w2, n);
+    }
+    std::vector<TileConfig> forms;
+    if (reg) {
+        TileConfig c = *best;
+        c.tc = 0;
+        c.reg = 1;
+        c.rb = max_reg_bits<V>();
+        c.tbits = sizeof(V) == 16 ? 11 : 12;
+        for (int k = 1; k <= 2; k++) {
+            if (mode == YAO_MODE_FUSED ? kreq > 0 && k != kreq : k > 1) continue;
+            c.k = mode == YAO_MODE_FUSED ? k : 0;
+            forms.push_back(c);
+        }
+        if (mode == YAO_MODE_FUSED && kreq <= 0) {
+            c = *best;
+            c.k = sizeof(V) == 16 ? 4 : 5;
+            c.tbits = 12;
+            c.rb = max_reg_bits<V>();
+            forms.push_back(c);
+        }
+        *best = forms[0];
+        if (forms.size() == 1) {  // nothing to time
+            *best_ms = 0.0;
+            return YAO_OK;
+        }
+    }
     const size_t bytes = ((size_t)1 << n) * sizeof(V);
     V* scratch = nullptr;
     if (cudaMallocAsync((void**)&scratch, bytes, ctx->stream) != cudaSuccess) {
@@ -2416,15 +2481,22 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
     struct Cand {
         TileConfig c;
         std::vector<PassPlan> passes;
-        size_t first = 0, step = 1, nsample = 0;
+        RegPlan reg;
+        size_t npasses = 0, first = 0, step = 1, nsample = 0;
         float best = 0.f;  // estimated ms of the whole run
     };
     auto make = [&](const TileConfig& c) {
         Cand x;
         x.c = c;
         bool any_tc = false;
-        plan_run<V>(n, prog, mode, c, x.passes, &any_tc);
-        const size_t P = x.passes.size();
+        if (c.reg) {
+            plan_reg_run(n, r->precision, prog, mode, c, x.reg);
+            x.npasses = x.reg.passes.size();
+        } else {
+            plan_run<V>(n, prog, mode, c, x.passes, &any_tc);
+            x.npasses = x.passes.size();
+        }
+        const size_t P = x.npasses;
         x.step = P > kTuneSample ? P / kTuneSample : 1;
         x.first = P > kTuneSample ? (P - x.step * (kTuneSample - 1)) / 2 : 0;
         x.nsample = 0;
@@ -2433,12 +2505,14 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
     };
     auto timed = [&](Cand& x, float* ms) -> int {
         YAO_CUDA(cudaEventRecord(a, ctx->stream));
-        int s = launch_passes<V>(ctx, scratch, n, r->precision, mode, x.passes, x.first, x.step);
+        int s = x.c.reg ? reg_launch(ctx, scratch, n, r->precision, mode == YAO_MODE_TILED && sizeof(V) == 16, x.reg, x.first,
+                                     x.step)
+                        : launch_passes<V>(ctx, scratch, n, r->precision, mode, x.passes, x.first, x.step);
         if (s) return s;
         YAO_CUDA(cudaEventRecord(b, ctx->stream));
         YAO_CUDA(cudaEventSynchronize(b));
         YAO_CUDA(cudaEventElapsedTime(ms, a, b));
-        *ms *= (float)x.passes.size() / (float)std::max<size_t>(1, x.nsample);
+        *ms *= (float)x.npasses / (float)std::max<size_t>(1, x.nsample);
         return YAO_OK;
     };
     // Candidates are timed in interleaved rounds (every candidate once per
@@ -2465,62 +2539,68 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
         if (log)
             for (size_t i = 0; i < cand.size(); i++)
                 fprintf(stderr,
-                        "[yao tune] n=%u %s mode=%d k=%d tbits=%d rb=%d tc=%d: %.3f ms (%zu of %zu passes timed)%s\n",
+                        "[yao tune] n=%u %s mode=%d k=%d tbits=%d rb=%d tc=%d reg=%d: %.3f ms (%zu of %zu passes timed)%s\n",
                         n, sizeof(V) == 8 ? "c64" : "c128", mode, cand[i].c.k, cand[i].c.tbits, cand[i].c.rb,
-                        cand[i].c.tc, cand[i].best, cand[i].nsample, cand[i].passes.size(),
+                        cand[i].c.tc, cand[i].c.reg, cand[i].best, cand[i].nsample, cand[i].npasses,
                         i == *pick ? "  <- chosen" : "");
         return YAO_OK;
     };
-    std::vector<TileConfig> shapes;
-    tile_candidates<V>(n, shapes);
     std::vector<Cand> cand;
-    for (const TileConfig& sc : shapes) {
-        TileConfig c = *best;
-        c.tbits = sc.tbits;
-        c.rb = sc.rb;
-        cand.push_back(make(c));
-    }
     size_t pick = 0;
     float bms = 0.f;
-    st = best_of(cand, &pick, &bms);
-    if (!st) *best = cand[pick].c;
-    if (!st && mode == YAO_MODE_FUSED && kreq <= 0) {
-        // widths 2..6 with the chosen shape; complex64 widths 3..5 also
-        // with the tensor cores' 2^12 tile, on and off the tensor cores
-        const TileConfig shape = *best;
-        std::vector<TileConfig> cs;
-        for (int k = 2; k <= kMaxTargets; k++) {
-            TileConfig c = shape;
-            c.k = k;
-            c.tc = 0;
-            cs.push_back(c);
-            if (sizeof(V) == 8 && k >= 3 && k <= kTcK)
-                for (int rb = 3; rb <= 4; rb++) {  // 512 or 256 threads a tile
-                    c.tbits = kTcTileBits;
-                    c.rb = rb;
-                    c.tc = 1;
-                    cs.push_back(c);
-                }
+    if (reg) {
+        for (const TileConfig& c : forms) cand.push_back(make(c));
+        st = best_of(cand, &pick, &bms);
+        if (!st) *best = cand[pick].c;
+    } else {
+        std::vector<TileConfig> shapes;
+        tile_candidates<V>(n, shapes);
+        for (const TileConfig& sc : shapes) {
+            TileConfig c = *best;
+            c.tbits = sc.tbits;
+            c.rb = sc.rb;
+            cand.push_back(make(c));
         }
-        cand.clear();
-        for (const TileConfig& c : cs) cand.push_back(make(c));
         st = best_of(cand, &pick, &bms);
         if (!st) *best = cand[pick].c;
-    } else if (!st && mode == YAO_MODE_FUSED && sizeof(V) == 8 && kreq >= 3 && kreq <= kTcK) {
-        // a requested complex64 width: the tensor cores' 2^12 tile against the
-        // chosen shape on the CUDA cores
-        TileConfig on = *best, on4 = *best, off = *best;
-        on.tbits = on4.tbits = kTcTileBits;
-        on.rb = 3;
-        on4.rb = 4;
-        on.tc = on4.tc = 1;
-        off.tc = 0;
-        cand.clear();
-        cand.push_back(make(on));
-        cand.push_back(make(on4));
-        cand.push_back(make(off));
-        st = best_of(cand, &pick, &bms);
-        if (!st) *best = cand[pick].c;
+        if (!st && mode == YAO_MODE_FUSED && kreq <= 0) {
+            // widths 2..6 with the chosen shape; complex64 widths 3..5 also
+            // with the tensor cores' 2^12 tile, on and off the tensor cores
+            const TileConfig shape = *best;
+            std::vector<TileConfig> cs;
+            for (int k = 2; k <= kMaxTargets; k++) {
+                TileConfig c = shape;
+                c.k = k;
+                c.tc = 0;
+                cs.push_back(c);
+                if (sizeof(V) == 8 && k >= 3 && k <= kTcK)
+                    for (int rb = 3; rb <= 4; rb++) {  // 512 or 256 threads a tile
+                        c.tbits = kTcTileBits;
+                        c.rb = rb;
+                        c.tc = 1;
+                        cs.push_back(c);
+                    }
+            }
+            cand.clear();
+            for (const TileConfig& c : cs) cand.push_back(make(c));
+            st = best_of(cand, &pick, &bms);
+            if (!st) *best = cand[pick].c;
+        } else if (!st && mode == YAO_MODE_FUSED && sizeof(V) == 8 && kreq >= 3 && kreq <= kTcK) {
+            // a requested complex64 width: the tensor cores' 2^12 tile against the
+            // chosen shape on the CUDA cores
+            TileConfig on = *best, on4 = *best, off = *best;
+            on.tbits = on4.tbits = kTcTileBits;
+            on.rb = 3;
+            on4.rb = 4;
+            on.tc = on4.tc = 1;
+            off.tc = 0;
+            cand.clear();
+            cand.push_back(make(on));
+            cand.push_back(make(on4));
+            cand.push_back(make(off));
+            st = best_of(cand, &pick, &bms);
+            if (!st) *best = cand[pick].c;
+        }
     }
     ctx->prof = prof;
     cudaEventDestroy(a);
@@ -2635,7 +2715,8 @@ int autotune_program(Ctx* ctx, Reg* r, const std::vector<LGate>& prog, int32_t m
     int s = r->precision == YAO_C128 ? choose_config<double2>(ctx, r, prog, mode, k, true, &c)
                                      : choose_config<float2>(ctx, r, prog, mode, k, true, &c);
     if (s) return s;
-    out[0] = c.k;
+    // register passes keep 1- and 2-qubit ops: at least width 2 when it was free
+    out[0] = c.reg && mode == YAO_MODE_FUSED && k <= 0 ? std::max(c.k, 2) : c.k;
     out[1] = c.tbits;
     out[2] = c.rb;
     out[3] = c.tc;
