@@ -59,6 +59,18 @@ def layer_elements(Y, n, layer, seed=2026):
     return els
 
 
+def gate_circuits(Y, n, layer):
+    """The layer as circuits of one gate: applied one after another, every
+    gate is one launch over the state (a circuit of several gates shares
+    passes)."""
+    return [Y.Circuit.qubits(n, [el]) for el in layer_elements(Y, n, layer)]
+
+
+def apply_gates(Y, circuits, reg):
+    for c in circuits:
+        Y.apply_inplace(c, reg)
+
+
 def layer_bytes(n, layer, amp_bytes=16):
     """Algorithmic bytes of one layer: 3n full-state gates + CNOTs on half."""
     full = 2 * amp_bytes * (1 << n)
@@ -339,6 +351,7 @@ def main():
     n = args.qubits
     dev = local
     circuits = [Y.Circuit.qubits(n, layer_elements(Y, n, l)) for l in range(LAYERS)]
+    gates = [gate_circuits(Y, n, l) for l in range(LAYERS)]
     stream = torch.cuda.ExternalStream(A.stream_ptr(dev), device=torch.device("cuda", dev))
 
     def barrier():
@@ -349,7 +362,7 @@ def main():
 
     reg = Y.ArrayReg.zero_state(n, device=dev)
     for i in range(args.warmup):
-        Y.apply_inplace(circuits[i % LAYERS], reg)
+        apply_gates(Y, gates[i % LAYERS], reg)
     # timed region starts from |0...0>: K = 40 steps is one full circuit
     A.check(A.lib().yao_ctx_synchronize(A.context(dev)))
     del reg
@@ -364,7 +377,7 @@ def main():
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record(stream)
     for i in range(args.steps):
-        Y.apply_inplace(circuits[i % LAYERS], reg)
+        apply_gates(Y, gates[i % LAYERS], reg)
     e1.record(stream)
     e1.synchronize()
     launches = Y.launch_count(dev) - launches0
@@ -413,7 +426,8 @@ def main():
     state_bytes = 16 * (1 << n)
     e2e = {"value": job_gbps(nbytes, world, e2e_ms), "unit": "GB/s",
            "h2d_bytes_per_step": state_bytes / args.steps, "d2h_bytes_per_step": state_bytes / args.steps,
-           "note": "one state upload + one download per K steps"}
+           "note": "one state upload + one download per K steps; a layer is one apply call, which runs several gates "
+                   "a pass (bit-identical; bytes counted per gate as in value)"}
     del host
 
     extras = {}
@@ -547,7 +561,10 @@ def profile_case(args):
                          "fused64": (Y.MODE_FUSED, Y.C128, 5), "fused32": (Y.MODE_FUSED, Y.C64, 5)}[args.profile_case]
         c = Y.Circuit.qubits(n, layer_elements(Y, n, 0))
         r = Y.ArrayReg.zero_state(n, prec)
-        Y.apply_inplace(c, r, mode, k)
+        if mode == Y.MODE_PLAIN:
+            apply_gates(Y, gate_circuits(Y, n, 0), r)
+        else:
+            Y.apply_inplace(c, r, mode, k)
     A.synchronize()
     print(f"profile case {args.profile_case} done: {Y.launch_count()} launches")
 

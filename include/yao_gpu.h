@@ -96,8 +96,10 @@ enum yao_postprocess { YAO_POST_NONE = 0, YAO_POST_RESET_TO = 1, YAO_POST_REMOVE
 enum yao_precision { YAO_C128 = 0, YAO_C64 = 1 };
 
 /* Execution form of yao_apply_inplace_mode.
- *   PLAIN     one kernel per gate, arithmetic identical to yao-rs (bit-exact);
- *   TILED     runs of gates applied per shared-memory tile, same arithmetic
+ *   PLAIN     every gate with yao-rs's own arithmetic, in order (bit-exact);
+ *             on complex128 registers runs of gates share passes over the
+ *             state where that is faster, else one kernel per gate;
+ *   TILED     runs of gates applied per tile of the state, same arithmetic
  *             and order as PLAIN (bit-exact), fewer HBM passes;
  *   FUSED     gates multiplied into dense k-qubit blocks on the host (FP64),
  *             each block one tiled pass; not bit-exact, report 1 - fidelity.

@@ -68,6 +68,30 @@ def test_register_passes(n):
             assert np.linalg.norm(r.state_vec() - ref) < 6e-8 * len(c.elements) * norm, k
 
 
+@pytest.mark.parametrize("n", [3, 4, 8, 11, 12, 14, 17, 20])
+def test_plain_runs_are_the_same_bits(n):
+    """PLAIN shares passes among gates: every bit, signed zeros among them, is
+    the oracle's, and every bit and NaN that of one launch a gate (circuits
+    of one gate) on states with infinities and NaN, where the launches leave
+    amplitudes alone that a diagonal entry of exactly 1 meets.  Gates on
+    three qubits are launches of their own in between."""
+    rng = np.random.default_rng(50 + n)
+    for c in (random_circuit(rng, n, 80, max_ctrl=min(3, n - 1)), layered_circuit(n, 2, seed=n)):
+        psi = random_state(rng, n)
+        r = Y.ArrayReg.from_vec(n, psi)
+        Y.apply_inplace(c, r)
+        assert np.array_equal(r.state_vec().view(np.uint64), O.apply_circuit(c, psi).view(np.uint64))
+        psi[1], psi[2], psi[5] = np.inf, complex(0.5, np.nan), complex(0.0, -np.inf)
+        r, one = Y.ArrayReg.from_vec(n, psi), Y.ArrayReg.from_vec(n, psi)
+        Y.apply_inplace(c, r)
+        for el in c.elements:
+            Y.apply_inplace(Y.Circuit.qubits(n, [el]), one)
+        got, ref = r.state_vec().view(np.float64), one.state_vec().view(np.float64)
+        finite = ~np.isnan(ref)
+        assert np.array_equal(np.isnan(got), ~finite)
+        assert np.array_equal(got.view(np.uint64)[finite], ref.view(np.uint64)[finite])
+
+
 def test_long_program_splits_its_description():
     """More gates on one tile than one pass describes."""
     rng = np.random.default_rng(0)

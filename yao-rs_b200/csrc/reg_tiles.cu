@@ -118,6 +118,7 @@ struct A128 {
                             __hiloint2double(__double2hiint(x.y) ^ (int)s, __double2loint(x.y)));
     }
     static __device__ __forceinline__ Amp neg(Amp x) { return make_double2(-x.x, -x.y); }
+    static __device__ __forceinline__ Amp zero() { return make_double2(0.0, 0.0); }
 };
 
 __device__ __forceinline__ uint64_t pk(float lo, float hi) {
@@ -199,6 +200,7 @@ struct A64 {
     static __device__ __forceinline__ Two sign_two(const Two& k, uint32_t s) { return Coef{k.hr, sign(k.hi, s), k.lr, sign(k.li, s)}; }
     static __device__ __forceinline__ Real sign_real(const Real& k, uint32_t s) { return Real{sign_two(k.p, s), sign_two(k.q, s)}; }
     static __device__ __forceinline__ Amp neg(Amp x) { return x ^ 0x8000000080000000ull; }
+    static __device__ __forceinline__ Amp zero() { return 0; }
 };
 
 // Negates the second member of the pairs in sg (bit j: pair of amplitude j).
@@ -288,7 +290,7 @@ __device__ __forceinline__ uint32_t r_entry(const uint4& w1, uint32_t t, uint32_
     return e;
 }
 
-template <typename A, int RB, int PAIR>
+template <typename A, bool EXACT, int RB, int PAIR>
 __device__ __forceinline__ void r_dense2(typename A::Amp (&v)[1 << RB], const uint4* m, uint32_t jm) {
     constexpr int B0 = 1 << (2 * PAIR), B1 = 2 << (2 * PAIR);
 #pragma unroll
@@ -300,8 +302,10 @@ __device__ __forceinline__ void r_dense2(typename A::Amp (&v)[1 << RB], const ui
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const uint4* mr = m + 4 * r * A::kCoef16;
-            y[r] = A::mad(A::mad(A::two(A::load(mr), x0, A::load(mr + A::kCoef16), x1), A::load(mr + 2 * A::kCoef16), x2),
-                          A::load(mr + 3 * A::kCoef16), x3);
+            // exact: from zero, as a gate alone does (the sign of a zero)
+            const typename A::Amp s = EXACT ? A::mad(A::mad(A::zero(), A::load(mr), x0), A::load(mr + A::kCoef16), x1)
+                                            : A::two(A::load(mr), x0, A::load(mr + A::kCoef16), x1);
+            y[r] = A::mad(A::mad(s, A::load(mr + 2 * A::kCoef16), x2), A::load(mr + 3 * A::kCoef16), x3);
         }
         v[j] = y[0];
         v[j | B0] = y[1];
@@ -404,9 +408,9 @@ __device__ __forceinline__ void r_ops(typename A::Amp (&v)[1 << RB], const uint4
         case RC_PHASE1 + 3:
             if constexpr (RB > 3) r_phase1<A, EXACT, RB, 3>(v, A::load(m + r_entry(w1, t, lb) * A::kCoef16));
             break;
-        case RC_DENSE2 + 0: r_dense2<A, RB, 0>(v, m, jm); break;
+        case RC_DENSE2 + 0: r_dense2<A, EXACT, RB, 0>(v, m, jm); break;
         case RC_DENSE2 + 1:
-            if constexpr (RB > 3) r_dense2<A, RB, 1>(v, m, jm);
+            if constexpr (RB > 3) r_dense2<A, EXACT, RB, 1>(v, m, jm);
             break;
         case RC_SWAP + 0: r_swap<A, RB, 0>(v, jm); break;
         case RC_SWAP + 1:
@@ -631,10 +635,13 @@ static uint64_t need_mask(const LGate& g, bool exact) {
 }
 static bool is_perm(const LGate& g) { return g.cls == GC_X || g.cls == GC_SWAP; }
 
+static bool reg_width(uint32_t nbits) { return nbits >= 4 && nbits <= 33; }
+static bool reg_gate(const LGate& g) { return !((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1)); }
+
 bool reg_supported(const std::vector<LGate>& prog, uint32_t nbits) {
-    if (nbits < 4 || nbits > 33) return false;
+    if (!reg_width(nbits)) return false;
     for (const LGate& g : prog)
-        if ((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1)) return false;
+        if (!reg_gate(g)) return false;
     return true;
 }
 
@@ -1169,7 +1176,7 @@ struct PassBuilder {
                 if ((j & rmask) == rval && reg_part(j) == s2) jm |= 1u << j;
             if (!jm) continue;
             const uint32_t ne = 1u << sel.size();
-            if (signs) {
+            if (signs && !exact) {  // (exact: multiplied, as a gate alone does)
                 for (uint32_t e = 0; e < ne; e++) {
                     if (entry(s2, e).re == 1.0) continue;
                     ROp op = base;
@@ -1215,8 +1222,9 @@ size_t pass_bytes(const RegPass& p, size_t coef_bytes) {
 
 }  // namespace
 
-void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits_max, bool exact,
-              RegPlan& out) {
+// The plan of prog[0 .. ngates).
+static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int32_t precision, int tbits_max,
+                           bool exact, RegPlan& out) {
     out.passes.clear();
     out.blob.clear();
     const size_t amp = precision == YAO_C128 ? 16 : 8, coef_bytes = precision == YAO_C128 ? 16 : 32;
@@ -1230,8 +1238,8 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
     // where the time of one CTA is the time of the pass.
     const uint64_t ntiles = 1ull << (nbits - tbits);
     const int rb = ntiles >= 296 ? 4 : (tbits > 11 ? 3 : 2);
-    std::vector<char> used(prog.size(), 0);
-    size_t i0 = 0, left = prog.size();
+    std::vector<char> used(ngates, 0);
+    size_t i0 = 0, left = ngates;
     while (left) {
         // the gates of this pass
         std::vector<const LGate*> run;
@@ -1239,7 +1247,7 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
         uint64_t hi = 0;
         {
             Scan sc(exact);
-            for (size_t j = i0; j < prog.size() && !sc.closed(all); j++) {
+            for (size_t j = i0; j < ngates && !sc.closed(all); j++) {
                 if (used[j]) continue;
                 const LGate& g = prog[j];
                 const uint64_t nh = hi | (need_mask(g, exact) & ~lowmask);
@@ -1312,7 +1320,7 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
                 used[at[j]] = 1;
                 left--;
             }
-        while (i0 < prog.size() && used[i0]) i0++;
+        while (i0 < ngates && used[i0]) i0++;
         if (p.ops.empty()) continue;
         // the tile leaves from the last segment's registers: whole 128-byte
         // runs a warp need the low positions on the lanes
@@ -1355,6 +1363,10 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
             d += coef_bytes;
         }
     }
+}
+
+void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out) {
+    reg_plan_range(prog.data(), prog.size(), nbits, precision, tbits, exact, out);
 }
 
 // ================================================================== launch
@@ -1427,7 +1439,8 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
         memcpy(h.tb, p.tb, sizeof(h.tb));
         CUtensorMap tmap;
         memset(&tmap, 0, sizeof(tmap));
-        h.use_tma = tma_enabled() && tma_make_plan(p.tb, p.tbits, nbits, amp, st, h.tma, &tmap) ? 1 : 0;
+        // (one tile: nothing to overlap, and no wait that could give up)
+        h.use_tma = p.ntiles > 1 && tma_enabled() && tma_make_plan(p.tb, p.tbits, nbits, amp, st, h.tma, &tmap) ? 1 : 0;
         const uint4* blob = (const uint4*)(dblob + p.blob_off);
         {
             ProfScope prof(ctx, exact ? "reg_pass_exact" : "reg_pass_fused",
@@ -1443,6 +1456,64 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
     }
     cudaFreeAsync(dblob, ctx->stream);
     return s;
+}
+
+// ==================================================== gate-by-gate programs
+
+// Seconds (estimate) of a gate's own launch: 3 us and its amplitudes, read
+// and written, at 6.2 TB/s.
+static double gate_seconds(const LGate& g, double state_bytes) {
+    double part = 1.0;
+    if (g.cls == GC_SWAP) part = 0.5;
+    if (g.cls == GC_DIAG) {
+        size_t n = 0;
+        for (const Cx& c : g.m) n += !is(c, 1.0);
+        part = (double)n / (double)g.m.size();
+    }
+    return 3e-6 + 2.0 * state_bytes * part / (double)(1ull << g.nc) / 6.2e12;
+}
+// FP64 operations of an exact op on every amplitude
+static double gate_flops(const LGate& g) {
+    return (g.cls == GC_DIAG ? 3.0 : g.cls == GC_DENSE ? (g.k == 1 ? 14.0 : 30.0) : 0.0) / (double)(1ull << g.nc);
+}
+
+int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
+    const uint32_t n = r->nbits;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    YAO_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    const bool passes = r->precision == YAO_C128 && reg_width(n) && cs == cudaStreamCaptureStatusNone;
+    const double bytes = (double)r->bytes(), amps = (double)(1ull << n);
+    bool waits = false;
+    for (size_t i = 0; i < prog.size();) {
+        size_t end = i;  // the gates from i on that a register pass can run
+        while (passes && end < prog.size() && reg_gate(prog[end])) end++;
+        if (end - i >= 2) {
+            // Passes where they are estimated to be faster: 8 us and the state
+            // read and written at 5.2 TB/s each, and the gates' arithmetic at
+            // 1e13 operations a second (measured: 22 passes of 696 gates,
+            // n = 25, 23 ms).  A few gates that touch a fraction of a large
+            // state, and gates that share no pass, stay launches of their own.
+            RegPlan plan;
+            reg_plan_range(&prog[i], end - i, n, YAO_C128, 11, true, plan);
+            double alone = 0.0, joint = (double)plan.passes.size() * (8e-6 + 2.0 * bytes / 5.2e12);
+            for (size_t q = i; q < end; q++) {
+                alone += gate_seconds(prog[q], bytes);
+                joint += gate_flops(prog[q]) * amps / 1e13;
+            }
+            if (joint < alone) {
+                int s = reg_launch(ctx, r->d, n, YAO_C128, true, plan, 0, 1);
+                if (s) return s;
+                waits |= n > 11;
+                i = end;
+                continue;
+            }
+        }
+        for (end = std::max(i + 1, end); i < end; i++) {
+            int s = launch_gate(ctx, r->d, r->precision, n, prog[i]);
+            if (s) return s;
+        }
+    }
+    return waits ? read_device_err(ctx, "apply") : YAO_OK;
 }
 
 }  // namespace yao

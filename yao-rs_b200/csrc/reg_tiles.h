@@ -86,4 +86,10 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
                size_t step);
 
+// A program with each gate's own arithmetic in program order (the PLAIN
+// form): runs of gates as exact register passes where that is faster, else
+// one launch a gate; the results are the same bits either way.  Wide gates,
+// complex64 and runs under stream capture: one launch a gate.
+int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog);
+
 }  // namespace yao

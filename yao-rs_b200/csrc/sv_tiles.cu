@@ -2649,13 +2649,7 @@ static int choose_config(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog,
 template <typename V>
 static int run_program_t(Ctx* ctx, Reg* r, const std::vector<LGate>& prog, int32_t mode, int32_t k, bool check_err) {
     V* st = (V*)r->d;
-    if (mode == YAO_MODE_PLAIN) {
-        for (const LGate& g : prog) {
-            int s = launch_gate(ctx, st, r->precision, r->nbits, g);
-            if (s) return s;
-        }
-        return YAO_OK;
-    }
+    if (mode == YAO_MODE_PLAIN) return plain_run(ctx, r, prog);
     TileConfig cfg;
     int s = choose_config<V>(ctx, r, prog, mode, k, false, &cfg);
     if (s) return s;

@@ -14,8 +14,8 @@ from .register import ArrayReg, DensityMatrix
 def apply_inplace(circuit, reg: ArrayReg, mode: int = A.MODE_PLAIN, k: int = 0):
     """apply_inplace (src/apply.rs:123-147).
 
-    mode: MODE_PLAIN (one kernel per gate, bit-exact), MODE_TILED (gates run
-    in shared-memory tiles, bit-exact) or MODE_FUSED (k-qubit fused blocks)."""
+    mode: MODE_PLAIN (each gate's own arithmetic, bit-exact), MODE_TILED (gates
+    run per tile of the state, bit-exact) or MODE_FUSED (gates multiplied)."""
     A.check(A.lib().yao_apply_inplace_mode(circuit.handle, reg.handle, mode, k))
     return reg
 
