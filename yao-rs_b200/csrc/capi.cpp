@@ -45,6 +45,42 @@ static cudaError_t alloc_device(Ctx* ctx, void** p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+// Registers of up to 256 MiB come from the device's memory pool
+// (stream-ordered on the context's stream; it keeps at most 4 GiB): a
+// cudaMalloc and a cudaFree of a 16 MB register took 400 and 350 us where its
+// whole circuit takes 280.  Larger ones would soon take the pool beyond what
+// it keeps, and it then unmaps and maps again (1 GiB registers: passes of 13
+// ms took 95); they are milliseconds of work each and are given back to the
+// driver when freed.  An allocation made while the stream is captured must
+// outlive the graph.
+constexpr size_t kPooledBytes = (size_t)256 << 20;
+
+static cudaError_t alloc_state(Ctx* ctx, void** p, size_t bytes, bool* pooled) {
+    *pooled = false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (bytes <= kPooledBytes && cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess &&
+        cs == cudaStreamCaptureStatusNone) {
+        if (cudaMallocAsync(p, bytes, ctx->stream) == cudaSuccess) {
+            *pooled = true;
+            return cudaSuccess;
+        }
+        cudaGetLastError();
+    }
+    return alloc_device(ctx, p, bytes);
+}
+
+// exported: the address was handed out, so work on any stream may still use
+// it (cudaFree waits for the device by itself)
+static void free_state(Ctx* ctx, void* p, bool pooled, bool exported) {
+    if (!pooled) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(p);
+        return;
+    }
+    if (exported) cudaDeviceSynchronize();
+    cudaFreeAsync(p, ctx->stream);
+}
+
 int Ctx::ensure_scratch(size_t bytes) {
     if (bytes <= scratch_bytes) return 0;
     size_t nb = std::max<size_t>(bytes, 1 << 20);
@@ -279,7 +315,7 @@ static int alloc_reg(Ctx* ctx, uint32_t nbits, int32_t prec, Reg** out) {
     r->ctx = ctx;
     r->nbits = nbits;
     r->precision = prec;
-    cudaError_t e = alloc_device(ctx, &r->d, r->bytes());
+    cudaError_t e = alloc_state(ctx, &r->d, r->bytes(), &r->pooled);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate a " + std::to_string(nbits) + "-qubit register (" +
@@ -296,7 +332,7 @@ static int alloc_dm(Ctx* ctx, uint32_t nbits, DM** out) {
     std::unique_ptr<yao_dm> d(new yao_dm());
     d->ctx = ctx;
     d->nbits = nbits;
-    if (alloc_device(ctx, &d->d, d->bytes()) != cudaSuccess) {
+    if (alloc_state(ctx, &d->d, d->bytes(), &d->pooled) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the density matrix");
     }
@@ -597,7 +633,7 @@ int yao_reg_zero_state(yao_ctx* ctx, uint32_t nbits, int32_t precision, yao_reg*
     if (s) return s;
     s = launch_fill_zero_state(ctx, r, 0);
     if (s) {
-        cudaFree(r->d);
+        free_state(ctx, r->d, r->pooled, false);
         delete r;
         return s;
     }
@@ -627,7 +663,7 @@ int yao_reg_from_host(yao_ctx* ctx, uint32_t nbits, const double* amps, yao_reg*
     cudaError_t e = cudaMemcpyAsync(r->d, amps, r->bytes(), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        cudaFree(r->d);
+        free_state(ctx, r->d, r->pooled, false);
         delete r;
         return cuda_fail(e, "upload");
     }
@@ -679,8 +715,7 @@ int yao_reg_deterministic_state(yao_ctx* ctx, uint32_t nbits, yao_reg** out) {
 void yao_reg_free(yao_reg* r) {
     if (!r) return;
     cudaSetDevice(r->ctx->device);
-    cudaStreamSynchronize(r->ctx->stream);
-    cudaFree(r->d);
+    free_state(r->ctx, r->d, r->pooled, r->exported);
     delete r;
 }
 
@@ -741,6 +776,10 @@ int yao_reg_upload(yao_reg* r, const void* amps) {
 int yao_reg_device_ptr(const yao_reg* r, void** out) {
     CHECK_NULL(r);
     CHECK_NULL(out);
+    // stream-ordered memory may be used on other streams once its allocation
+    // has taken place
+    if (r->pooled && !r->exported) YAO_CUDA(cudaStreamSynchronize(r->ctx->stream));
+    r->exported = true;
     *out = r->d;
     return YAO_OK;
 }
@@ -985,8 +1024,7 @@ int yao_dm_mixed(yao_ctx* ctx, const double* weights, const yao_reg* const* regs
 void yao_dm_free(yao_dm* d) {
     if (!d) return;
     cudaSetDevice(d->ctx->device);
-    cudaStreamSynchronize(d->ctx->stream);
-    cudaFree(d->d);
+    free_state(d->ctx, d->d, d->pooled, false);
     delete d;
 }
 

@@ -86,8 +86,8 @@ __global__ void k_fill(V* st, uint64_t n, double re, double im) {
     GRID_STRIDE(i, n) st[i] = v;
 }
 template <typename V>
-__global__ void k_set_one(V* st, uint64_t idx, double re, double im) {
-    st[idx] = from_d2<V>(make_double2(re, im));
+__global__ void k_basis(V* st, uint64_t n, uint64_t idx) {
+    GRID_STRIDE(i, n) st[i] = from_d2<V>(make_double2(i == idx ? 1.0 : 0.0, 0.0));
 }
 
 static int fill(Ctx* ctx, Reg* r, double re, double im) {
@@ -102,21 +102,17 @@ static int fill(Ctx* ctx, Reg* r, double re, double im) {
     return YAO_OK;
 }
 
-static int set_one(Ctx* ctx, Reg* r, uint64_t idx, double re, double im) {
+// ArrayReg::zero_state / product_state (src/register.rs:21-33)
+int launch_fill_zero_state(Ctx* ctx, Reg* r, uint64_t basis) {
+    uint64_t n = (uint64_t)1 << r->nbits;
+    unsigned g = grid_for(n, 256, ctx->num_sms);
     if (r->precision == YAO_C128)
-        k_set_one<double2><<<1, 1, 0, ctx->stream>>>((double2*)r->d, idx, re, im);
+        k_basis<double2><<<g, 256, 0, ctx->stream>>>((double2*)r->d, n, basis);
     else
-        k_set_one<float2><<<1, 1, 0, ctx->stream>>>((float2*)r->d, idx, re, im);
+        k_basis<float2><<<g, 256, 0, ctx->stream>>>((float2*)r->d, n, basis);
     ctx->launches++;
     YAO_CUDA(cudaGetLastError());
     return YAO_OK;
-}
-
-// ArrayReg::zero_state / product_state (src/register.rs:21-33)
-int launch_fill_zero_state(Ctx* ctx, Reg* r, uint64_t basis) {
-    int s = fill(ctx, r, 0.0, 0.0);
-    if (s) return s;
-    return set_one(ctx, r, basis, 1.0, 0.0);
 }
 
 // ArrayReg::uniform_state (src/register.rs:47-54): 1/sqrt(dim) everywhere

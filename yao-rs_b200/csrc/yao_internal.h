@@ -177,6 +177,8 @@ struct Reg {
     uint32_t nbits = 0;
     int32_t precision = YAO_C128;
     void* d = nullptr;  // double2* (C128) or float2* (C64)
+    bool pooled = false;            // d is stream-ordered memory of ctx->stream
+    mutable bool exported = false;  // the address was handed out (yao_reg_device_ptr)
     size_t bytes() const { return ((size_t)1 << nbits) * (precision == YAO_C128 ? 16 : 8); }
 };
 
@@ -184,6 +186,7 @@ struct DM {
     Ctx* ctx = nullptr;
     uint32_t nbits = 0;
     void* d = nullptr;  // double2*, 4^n
+    bool pooled = false;
     size_t bytes() const { return ((size_t)1 << (2 * nbits)) * 16; }
 };
 
