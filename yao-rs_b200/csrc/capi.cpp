@@ -1212,15 +1212,9 @@ int yao_expect_arrayreg(const yao_reg* r, const yao_term* terms, size_t nterms, 
     int s = build_mono_terms(terms, nterms, r->nbits, true, mt);
     if (s) return s;
     YAO_CUDA(cudaSetDevice(r->ctx->device));
-    std::vector<Cx> vals;
-    s = expect_terms(r->ctx, r, mt, vals);
-    if (s) return s;
     Cx acc{0, 0};
-    for (size_t t = 0; t < mt.size(); t++) {
-        Cx p = cxmul(mt[t].coeff, vals[t]);
-        acc.re += p.re;
-        acc.im += p.im;
-    }
+    s = expect_sum(r->ctx, r, mt, &acc);
+    if (s) return s;
     out[0] = acc.re;
     out[1] = acc.im;
     return YAO_OK;

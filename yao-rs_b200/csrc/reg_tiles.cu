@@ -39,17 +39,6 @@ struct RHdr {
     TmaPlan tma;
 };
 
-constexpr uint64_t kRegWaitNs = 1000000000ull;  // 1 s
-
-__device__ __forceinline__ uint64_t reg_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// 128-byte TMA swizzle on byte offsets within a 1024-byte aligned tile.
-__device__ __forceinline__ uint32_t rswz(uint32_t b) { return b ^ ((b >> 3) & 0x70u); }
-
 // Arithmetic on one amplitude type.  complex128: EXACT is num_complex's
 // operations without FMA, else FMA.  complex64: coefficients split into
 // high and low FP32 parts, each stored twice so that one packed FP32x2 FMA
@@ -460,9 +449,9 @@ struct RPlace {
         for (int i = 0; i < RB; i++) {
             const uint32_t p = (sg.z >> (8 * i)) & 0xffu;
             lb = ((lb >> p) << (p + 1)) | (lb & ((1u << p) - 1));
-            so[i] = rswz(amp << ((sg.w >> (8 * i)) & 0xffu));
+            so[i] = tma::swizzle128(amp << ((sg.w >> (8 * i)) & 0xffu));
         }
-        sb = rswz(lb * amp);
+        sb = tma::swizzle128(lb * amp);
     }
     __device__ __forceinline__ uint32_t at(int j) const {
         uint32_t o = sb;
@@ -542,9 +531,9 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
         unsigned char* s = smem + (size_t)b * tile_bytes;
         if (use_tma) {
             if (!dead) {
-                const uint64_t t0 = reg_ns();
+                const uint64_t t0 = tma::now_ns();
                 while (!tc::mbar_try_wait(&full_bar[b], par)) {
-                    if (reg_ns() - t0 > kRegWaitNs) {
+                    if (tma::now_ns() - t0 > tma::kWaitNs) {
                         dead = true;
                         atomicExch(err, 1);
                         break;
@@ -554,7 +543,7 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
             }
         } else {
             for (uint32_t l = threadIdx.x; l < (1u << hdr.tbits); l += blockDim.x)
-                *(Amp*)(s + rswz(l * AB)) = st[tbase[b] | r_deposit(hdr, l)];
+                *(Amp*)(s + tma::swizzle128(l * AB)) = st[tbase[b] | r_deposit(hdr, l)];
             __syncthreads();
         }
         const uint64_t base = tbase[b];
@@ -606,11 +595,11 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
         if (b == 0) par ^= 1u;
     }
     if (threadIdx.x == 0) {
-        const uint64_t t0 = reg_ns();
+        const uint64_t t0 = tma::now_ns();
         for (uint32_t q = 0; q < nbuf; q++)
             if (pending & (1u << q))
                 for (uint32_t ph = 0; ph < 2; ph++)
-                    while (!tc::mbar_try_wait(&full_bar[q], ph) && reg_ns() - t0 < kRegWaitNs) {
+                    while (!tc::mbar_try_wait(&full_bar[q], ph) && tma::now_ns() - t0 < tma::kWaitNs) {
                     }
     }
 }

@@ -75,6 +75,13 @@ static int finish_sum(Ctx* ctx, double* partial, int nblocks, int nv, double* ho
     return YAO_OK;
 }
 
+int launch_final_sum(Ctx* ctx, const double* partial, int nblocks, int nv, double* out) {
+    k_final_sum<<<1, kRT, 0, ctx->stream>>>(partial, nblocks, nv, out);
+    ctx->launches++;
+    YAO_CUDA(cudaGetLastError());
+    return YAO_OK;
+}
+
 #define GRID_STRIDE(i, n) \
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (uint64_t)gridDim.x * blockDim.x)
 

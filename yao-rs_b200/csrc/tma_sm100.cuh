@@ -34,6 +34,18 @@ bool tma_enabled();
 
 namespace tma {
 
+constexpr uint64_t kWaitNs = 1000000000ull;  // limit of a wait for a tile: 1 s
+
+__device__ __forceinline__ uint64_t now_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Where the 128-byte swizzle puts byte b of a tile that starts on a
+// 1024-byte boundary (exclusive-or linear in b).
+__device__ __forceinline__ uint32_t swizzle128(uint32_t b) { return b ^ ((b >> 3) & 0x70u); }
+
 // Load of one box at coordinates c0..c4 (elements; c0 * element size is a
 // multiple of 16 bytes) into shared memory at `dst` (shared-window address,
 // 1024-byte aligned for the 128-byte swizzle); the barrier at `bar` counts

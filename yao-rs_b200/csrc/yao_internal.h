@@ -251,6 +251,11 @@ struct ExpectPending {
 };
 int expect_terms_launch(Ctx* ctx, const Reg* r, const std::vector<MonoTerm>& terms, ExpectPending& pend);
 void expect_terms_collect(Ctx* ctx, const ExpectPending& pend, std::vector<Cx>& values);
+// sum_t coeff_t <psi|O_t|psi> (sv_expect.cu): Pauli strings over tiles of the
+// state in a few passes, other terms by expect_terms.
+int expect_sum(Ctx* ctx, const Reg* r, const std::vector<MonoTerm>& terms, Cx* out);
+// out[v] = sum over b of partial[b * nv + v], one launch (sv_reduce.cu).
+int launch_final_sum(Ctx* ctx, const double* partial, int nblocks, int nv, double* out);
 // The allocation-free expectation value (static device scratch), sv_reduce.cu.
 int expect_noalloc(Ctx* ctx, const Reg* r, const yao_term* terms, size_t nterms, double* out);
 int build_lambda(Ctx* ctx, const Reg* psi, const std::vector<MonoTerm>& terms, Reg* lambda);
