@@ -1,0 +1,97 @@
+"""Gradients by the register sweep (csrc/sweep.cu), of one and of several
+parameter vectors, against the oracle at register counts around its tile
+and thread edges."""
+import numpy as np
+import pytest
+
+import oracle as O
+import yao_rs as Y
+from helpers import random_state
+from yao_rs import Gate
+
+
+def ansatz(rng, n, layers, kind):
+    """0: Ry, Rz and a CNOT ring; 1: Hadamards, constants and every 1-parameter
+    gate in a run; 2: sparse runs.  1 and 2 are entangled by CNOTs with
+    controls of either value (one or two), CZ, SWAP and controlled SWAP."""
+    def t():
+        return float(rng.uniform(-3, 3))
+    els = []
+    for _ in range(layers):
+        for q in range(n):
+            run = ([Gate.Ry(t()), Gate.Rz(t())] if kind == 0 else
+                   [Gate.H, Gate.Rx(t()), Gate.Phase(t()), Gate.Ry(t()), Gate.T] if kind == 1 else
+                   [Gate.Rz(t())] if rng.random() < 0.5 else [Gate.X, Gate.Rx(t()), Gate.Y])
+            els += [Y.put([q], g) for g in run]
+        for q in range(n):
+            p, r = [int(x) for x in rng.permutation(n)], rng.random()
+            if kind == 0:
+                els.append(Y.control([q], [(q + 1) % n], Gate.X))
+            elif r < 0.4:
+                els.append(Y.PositionedGate(Gate.X, [p[0]], [p[1]], [bool(rng.integers(2))]))
+            elif r < 0.6:
+                els.append(Y.control([p[0]], [p[1]], Gate.Z))
+            elif r < 0.75:
+                els.append(Y.put(p[:2], Gate.SWAP))
+            elif r < 0.9:
+                els.append(Y.PositionedGate(Gate.X, [p[0]], p[1:3], [True, False]))
+            else:
+                els.append(Y.PositionedGate(Gate.SWAP, p[:2], [p[2]], [False]))
+    return Y.Circuit.qubits(n, els)
+
+
+def hamiltonian(n):
+    cs, ss = [0.3], [Y.OperatorString([(0, Y.Op.Y), (n - 1, Y.Op.X)])]
+    for i in range(n):
+        cs += [-1.0, 0.7]
+        ss += [Y.OperatorString([(i, Y.Op.Z), ((i + 1) % n, Y.Op.Z)]), Y.OperatorString([(i, Y.Op.X)])]
+    return Y.OperatorPolynomial(cs, ss)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 4, 7, 8, 10, 11, 12, 13, 14])
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_gradients(n, kind):
+    rng = np.random.default_rng([n, kind])
+    c, h, psi = ansatz(rng, n, 3, kind), hamiltonian(n), random_state(rng, n)
+    reg = Y.ArrayReg.from_vec(n, psi)
+    # a few hundred gates of 1.1e-16 each on terms of magnitude 1.7 n
+    tol = 1e-12
+    value, grad = O.expect_grad(h, c, psi)
+    v, g = Y.expect_grad(h, c, reg)
+    assert abs(v - value) < tol and np.max(np.abs(np.array(g) - np.array(grad))) < tol
+    sets = rng.uniform(-3, 3, size=(7, c.num_params()))
+    sets[2] = c.parameters()
+    vs, gs = Y.expect_grad_batch(h, c, sets, reg)
+    assert abs(vs[2] - value) < tol and np.max(np.abs(gs[2] - np.array(grad))) < tol
+    c.dispatch(list(sets[6]))
+    value, grad = O.expect_grad(h, c, psi)
+    assert abs(vs[6] - value) < tol and np.max(np.abs(gs[6] - np.array(grad))) < tol
+    assert np.max(np.abs(reg.state_vec() - psi)) == 0.0
+
+
+@pytest.mark.gpu
+def test_more_sets_than_a_group():
+    """Groups of states that fit the cache, the last one smaller: every set as
+    by itself."""
+    n, nsets = 14, 131  # 128 sets of 2 x 256 KiB are one group
+    rng = np.random.default_rng(0)
+    c, h = ansatz(rng, n, 1, 0), hamiltonian(n)
+    sets = rng.uniform(-3, 3, size=(nsets, c.num_params()))
+    reg = Y.ArrayReg.zero_state(n)
+    vs, gs = Y.expect_grad_batch(h, c, sets, reg)
+    for s in (0, 127, 128, 130):
+        c.dispatch(list(sets[s]))
+        v, g = Y.expect_grad(h, c, reg)
+        assert abs(v - vs[s]) < 1e-12 and np.max(np.abs(np.array(g) - gs[s])) < 1e-12
+
+
+@pytest.mark.gpu
+def test_long_runs_of_ops_split_passes():
+    """More runs on one tile than a pass holds."""
+    n = 6
+    rng = np.random.default_rng(1)
+    c, h, psi = ansatz(rng, n, 30, 0), hamiltonian(n), random_state(rng, n)
+    value, grad = O.expect_grad(h, c, psi)
+    v, g = Y.expect_grad(h, c, Y.ArrayReg.from_vec(n, psi))
+    assert abs(v - value) < 1e-12 and np.max(np.abs(np.array(g) - np.array(grad))) < 1e-12

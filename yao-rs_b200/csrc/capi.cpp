@@ -12,6 +12,7 @@
 #include <set>
 #include <sstream>
 
+#include "sweep.h"
 #include "yao_internal.h"
 
 namespace yao {
@@ -1303,12 +1304,20 @@ int yao_expect_grad(const yao_term* terms, size_t nterms, const yao_circuit* cc,
     // (YAO_ADJ_TILES=0, or a wider gate: the per-gate form below)
     struct PlanHold {
         AdjPlan* p = nullptr;
+        SweepPlan* s = nullptr;
         ~PlanHold() {
             if (p) adjoint_plan_free(p);
+            if (s) sweep_plan_free(s);
         }
     } plan;
     const char* at = getenv("YAO_ADJ_TILES");
-    if (np && !(at && at[0] == '0')) {
+    // parameters in uncontrolled 1-qubit gates only: the register sweep (the
+    // YAO_ADJ_* switches choose among the forms of the other one)
+    const char* forms[] = {"YAO_ADJ_TILES", "YAO_ADJ_REORDER", "YAO_ADJ_SEGMENTS", "YAO_ADJ_UPAIR", "YAO_ADJ_XFOLD", "YAO_ADJ_FUSE"};
+    bool form_set = false;
+    for (const char* f : forms) form_set |= getenv(f) != nullptr;
+    if (np && !form_set) plan.s = sweep_plan_new(c, psi0->nbits);
+    if (np && !plan.s && !(at && at[0] == '0')) {
         int pst = YAO_OK;
         plan.p = adjoint_plan_new(c, psi0->nbits, YAO_C128, np, &pst);
         if (!plan.p && pst != YAO_ERR_UNSUPPORTED) return pst;
@@ -1340,6 +1349,14 @@ int yao_expect_grad(const yao_term* terms, size_t nterms, const yao_circuit* cc,
     // same pass (read back with the gradient)
     s = build_lambda_energy(ctx, psi, mt, lam);
     if (s) return s;
+    if (plan.s) {
+        std::vector<double> params(np);
+        s = yao_circuit_parameters(cc, params.data(), np);
+        if (!s) s = sweep_reverse(ctx, plan.s, psi->d, lam->d, params.data(), grad);
+        if (s) return s;
+        *value = lambda_energy_collect(ctx);  // sweep_reverse synchronised
+        return YAO_OK;
+    }
     // reverse sweep over shared-memory tiles of psi and lambda
     if (plan.p) {
         s = adjoint_run(ctx, psi, lam, plan.p, grad);
@@ -1409,6 +1426,11 @@ int yao_expect_grad_batch(const yao_term* terms, size_t nterms, const yao_circui
     s = build_mono_terms(terms, nterms, psi0->nbits, true, mt);
     if (s) return s;
     YAO_CUDA(cudaSetDevice(psi0->ctx->device));
+    if (SweepPlan* p = sweep_plan_new(c, psi0->nbits)) {
+        s = sweep_batch(psi0->ctx, p, mt, params, nsets, psi0, values, grads);
+        sweep_plan_free(p);
+        return s;
+    }
     return expect_grad_batch(psi0->ctx, mt, c, params, nsets, psi0, values, grads);
 }
 
