@@ -262,9 +262,10 @@ int yao_dm_apply(yao_dm* d, const yao_circuit* c);
 /* The same with an execution form: YAO_MODE_PLAIN (= yao_dm_apply, the exact
  * Kraus sum of yao-rs) or YAO_MODE_FUSED: rho as a 2n-qubit vector, each
  * gate as U on the row bits and conj(U) on the column bits, each channel as
- * its superoperator sum_i K_i (x) conj(K_i) (a dense op on 2k bits), all run
- * through the FUSED tile-pass engine in FP64 (not bit-identical; agrees to
- * ~1e-14). */
+ * its superoperator sum_i K_i (x) conj(K_i), all run through register passes
+ * in FP64 (through the FUSED block passes where a step has no form there:
+ * three or more targets, a 2-qubit channel that is not a sum of Pauli
+ * products).  Not bit-identical; agrees to ~1e-14. */
 int yao_dm_apply_mode(yao_dm* d, const yao_circuit* c, int32_t mode);
 /* trace / purity / partial_tr (src/density_matrix.rs:63-112). */
 int yao_dm_trace(const yao_dm* d, double out[2]);

@@ -1137,34 +1137,58 @@ int yao_dm_apply_mode(yao_dm* d, const yao_circuit* cc, int32_t mode) {
     if (sw) return sw;
     YAO_CUDA(cudaSetDevice(d->ctx->device));
     const uint32_t n = d->nbits, nb = 2 * n;
-    if (mode == YAO_MODE_FUSED) return dm_apply_fused(d, c);
+    std::vector<DMStep> steps;
+    // named channels seen so far: kind, parameters and the order of the
+    // locations (2-qubit operators are sorted by it)
+    struct Seen {
+        const ChannelElem* ch;
+        int at;
+    };
+    std::vector<Seen> seen;
+    auto same = [](const ChannelElem& a, const ChannelElem& b) {
+        return a.type == b.type && a.mats.empty() && b.mats.empty() && a.depol_n == b.depol_n &&
+               memcmp(a.params, b.params, sizeof(a.params)) == 0 && a.locs.size() == b.locs.size() &&
+               (a.locs.size() < 2 || (a.locs.size() == 2 && (a.locs[0] < a.locs[1]) == (b.locs[0] < b.locs[1])));
+    };
     for (const Element& el : c->elems) {
+        DMStep s;
         if (el.kind == YAO_ELEM_GATE) {
-            std::vector<LGate> rows, cols;
-            lower_gate(el.g, nb, 0, false, rows);
-            lower_gate(el.g, nb, n, true, cols);
-            for (size_t i = 0; i < rows.size(); i++) {
-                int s = launch_dm_gate(d->ctx, d, rows[i], cols[i]);
-                if (s) return s;
-            }
+            lower_gate(el.g, nb, 0, false, s.rows);
+            lower_gate(el.g, nb, n, true, s.cols);
+            if (s.rows.empty()) continue;
         } else if (el.kind == YAO_ELEM_CHANNEL) {
+            s.channel = true;
             std::vector<Cx> kraus;
             uint32_t nk, dim;
-            int s = channel_kraus(el.ch, kraus, nk, dim);
-            if (s) return s;
-            std::vector<LGate> rows, cols;
-            for (uint32_t q = 0; q < nk; q++) {
+            int st = channel_kraus(el.ch, kraus, nk, dim);
+            if (st) return st;
+            for (const Seen& e : seen)
+                if (same(*e.ch, el.ch)) s.like = e.at;
+            if (s.like < 0) seen.push_back(Seen{&el.ch, (int)steps.size()});
+            for (uint32_t q = 0; q < (s.like < 0 ? nk : 1u); q++) {
                 std::vector<Cx> K(kraus.begin() + (size_t)q * dim * dim, kraus.begin() + (size_t)(q + 1) * dim * dim);
                 bool diag = matrix_is_diagonal(K.data(), dim);
                 std::vector<Cx> Kc(K);
                 for (auto& v : Kc) v.im = -v.im;
-                rows.push_back(lower_matrix(K, dim, diag, el.ch.locs, {}, {}, nb, 0));
-                cols.push_back(lower_matrix(Kc, dim, diag, el.ch.locs, {}, {}, nb, n));
+                s.rows.push_back(lower_matrix(K, dim, diag, el.ch.locs, {}, {}, nb, 0));
+                s.cols.push_back(lower_matrix(Kc, dim, diag, el.ch.locs, {}, {}, nb, n));
             }
-            s = launch_dm_channel(d->ctx, d, rows, cols, {}, {});
+        } else {
+            continue;
+        }
+        steps.push_back(std::move(s));
+    }
+    if (mode == YAO_MODE_FUSED) {
+        // pinned tile shapes choose the block passes
+        bool done = false;
+        if (!getenv("YAO_TILE_BITS") && !getenv("YAO_REG_BITS")) {
+            int s = dm_fused_run(d->ctx, d, steps, &done);
             if (s) return s;
         }
+        return done ? YAO_OK : dm_apply_fused(d, c);
     }
+    int sp = dm_plain_run(d->ctx, d, steps);
+    if (sp) return sp;
     YAO_CUDA(cudaGetLastError());
     return YAO_OK;
 }

@@ -316,9 +316,176 @@ __device__ __forceinline__ void r_swap(typename A::Amp (&v)[1 << RB], uint32_t j
     }
 }
 
+// Density matrices: the register index of entry (row a, column b) of the
+// pairs' qubits is b0 + 2 a0 + 4 b1 + 8 a1.  The Kraus sum of a channel is
+// formed operator by operator like in the passes of one channel (dm.cu):
+// acc = 0; acc += c_b (r_a entry), each product and sum rounded, with real
+// weights (a pair of imaginary ones is a real pair).
+__device__ __forceinline__ double2 d_kraus(double2 acc, double r, double c, double2 x) {
+    return make_double2(__dadd_rn(acc.x, __dmul_rn(c, __dmul_rn(r, x.x))), __dadd_rn(acc.y, __dmul_rn(c, __dmul_rn(r, x.y))));
+}
+
+// Operator types of RC_CHAN1: 0 diagonal, 1 exchange of 0 and 1, 2 |0><1|,
+// 3 |1><0| (times weights).  G groups of entries go
+// through the operators together: an operator's words are read once for them,
+// and their sums are independent (one group at a time waited for each sum).
+// Measured on 11 qubits (64 MiB), 66 rotations and 15 CZ with a channel after
+// each and 33 dampings: a pass for every gate and channel 5.1 ms, register
+// passes with one group at a time 3.8, with two 2.8; bound by the rounded
+// products and sums (no fused multiply-adds, like the lone passes).
+template <int RB, int PAIR, int G>
+__device__ __forceinline__ void r_chan1(double2 (&v)[1 << RB], const uint4* m, int nk) {
+    constexpr int B = 1 << (2 * PAIR), A = 2 << (2 * PAIR);  // column, row
+    constexpr int OTHER = PAIR ? 1 : 4;                      // the groups' first entries: multiples of this below A | B left out
+#pragma unroll
+    for (int g0 = 0; g0 < (1 << RB) / 4; g0 += G) {
+        double2 x[G][4], y[G][4];
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int j = (g0 + g) * OTHER;
+            x[g][0] = v[j];
+            x[g][1] = v[j | B];
+            x[g][2] = v[j | A];
+            x[g][3] = v[j | A | B];
+#pragma unroll
+            for (int e = 0; e < 4; e++) y[g][e] = make_double2(0.0, 0.0);
+        }
+        for (int q = 0; q < nk; q++) {
+            const uint32_t type = m[3 * q].x;
+            const double2 r = *(const double2*)&m[3 * q + 1], c = *(const double2*)&m[3 * q + 2];
+            if (type <= 1) {
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    if (type == 0) {
+                        y[g][0] = d_kraus(y[g][0], r.x, c.x, x[g][0]);
+                        y[g][1] = d_kraus(y[g][1], r.x, c.y, x[g][1]);
+                        y[g][2] = d_kraus(y[g][2], r.y, c.x, x[g][2]);
+                        y[g][3] = d_kraus(y[g][3], r.y, c.y, x[g][3]);
+                    } else {
+                        y[g][0] = d_kraus(y[g][0], r.x, c.x, x[g][3]);
+                        y[g][1] = d_kraus(y[g][1], r.x, c.y, x[g][2]);
+                        y[g][2] = d_kraus(y[g][2], r.y, c.x, x[g][1]);
+                        y[g][3] = d_kraus(y[g][3], r.y, c.y, x[g][0]);
+                    }
+                }
+            } else if (type == 2) {
+#pragma unroll
+                for (int g = 0; g < G; g++) y[g][0] = d_kraus(y[g][0], r.x, c.x, x[g][3]);
+            } else {
+#pragma unroll
+                for (int g = 0; g < G; g++) y[g][3] = d_kraus(y[g][3], r.y, c.y, x[g][0]);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int j = (g0 + g) * OTHER;
+            v[j] = y[g][0];
+            v[j | B] = y[g][1];
+            v[j | A] = y[g][2];
+            v[j | A | B] = y[g][3];
+        }
+    }
+}
+
+// register index of (row i, column i ^ d) of the two qubits
+__device__ __host__ constexpr int d_orbit(int i, int d) {
+    return ((i ^ d) & 1) | ((i & 1) << 1) | ((((i ^ d) >> 1) & 1) << 2) | ((i >> 1) << 3);
+}
+
+// A 2-qubit channel whose operators all exchange a with a ^ x: the entries
+// (i, i ^ d) of one d stay among themselves, so a few accumulators at a time
+// serve; two values of d go through the operators together.
+__device__ __forceinline__ void r_chan2(double2 (&v)[16], const uint4* m, int nk) {
+#pragma unroll
+    for (int d0 = 0; d0 < 4; d0 += 2) {
+        double2 s[2][4], y[2][4];
+#pragma unroll
+        for (int g = 0; g < 2; g++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                s[g][i] = v[d_orbit(i, d0 + g)];
+                y[g][i] = make_double2(0.0, 0.0);
+            }
+        for (int q = 0; q < nk; q++) {
+            const uint4* w = m + 5 * q;
+            const double* r = (const double*)(w + 1);
+            const double* c = (const double*)(w + 3);
+            switch (w[0].x) {
+#define D_CHAN2(X)                                                                              \
+    case X:                                                                                     \
+        _Pragma("unroll") for (int g = 0; g < 2; g++) {                                         \
+            _Pragma("unroll") for (int i = 0; i < 4; i++)                                       \
+                y[g][i] = d_kraus(y[g][i], r[i], c[i ^ (d0 + g)], s[g][i ^ X]);                 \
+        }                                                                                       \
+        break;
+                D_CHAN2(0)
+                D_CHAN2(1)
+                D_CHAN2(2)
+            default:
+                D_CHAN2(3)
+#undef D_CHAN2
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < 2; g++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[d_orbit(i, d0 + g)] = y[g][i];
+    }
+}
+
+__device__ __forceinline__ void r_pauli2(double2 (&v)[16], const uint4* m) {
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        double2 s[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] = v[d_orbit(i, d)];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const double2 p = *(const double2*)&m[8 * d + 2 * i], q = *(const double2*)&m[8 * d + 2 * i + 1];
+            v[d_orbit(i, d)] = make_double2(fma(p.x, s[0].x, fma(p.y, s[1].x, fma(q.x, s[2].x, q.y * s[3].x))),
+                                            fma(p.x, s[0].y, fma(p.y, s[1].y, fma(q.x, s[2].y, q.y * s[3].y))));
+        }
+    }
+}
+
+// y_r = f_r sum_c R[r][c] x_c, or y_r = sum_c R[r][c] (f_c x_c): what the
+// rotations, dampings and depolarizations of one qubit between two gates
+// multiply to.  The 16 reals stay in registers for the four groups.
+template <int RB, int PAIR>
+__device__ __forceinline__ void r_real2(double2 (&v)[1 << RB], const uint4* m, bool cols) {
+    constexpr int B0 = 1 << (2 * PAIR), B1 = 2 << (2 * PAIR);
+    double2 R[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) R[i] = *(const double2*)&m[i];
+    const double2* f = (const double2*)&m[8];
+#pragma unroll
+    for (int j = 0; j < (1 << RB); j++) {
+        if (j & (B0 | B1)) continue;
+        double2 x[4] = {v[j], v[j | B0], v[j | B1], v[j | B0 | B1]}, y[4];
+        if (cols)
+#pragma unroll
+            for (int c = 0; c < 4; c++) x[c] = A128<false>::mul(A128<false>::Coef{f[c]}, x[c]);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const double2 p = R[2 * r], q = R[2 * r + 1];
+            y[r] = make_double2(fma(p.x, x[0].x, fma(p.y, x[1].x, fma(q.x, x[2].x, q.y * x[3].x))),
+                                fma(p.x, x[0].y, fma(p.y, x[1].y, fma(q.x, x[2].y, q.y * x[3].y))));
+        }
+        if (!cols)
+#pragma unroll
+            for (int r = 0; r < 4; r++) y[r] = A128<false>::mul(A128<false>::Coef{f[r]}, y[r]);
+        v[j] = y[0];
+        v[j | B0] = y[1];
+        v[j | B1] = y[2];
+        v[j | B0 | B1] = y[3];
+    }
+}
+
 // The ops of one segment on one thread's amplitudes.  t: the tile's number;
 // lb: the thread's tile position (register positions at 0).
-template <typename A, bool EXACT, int RB>
+// DMX: density-matrix steps among the ops (a kernel of its own: their
+// registers would spill the others' amplitudes).
+template <typename A, bool EXACT, int RB, bool DMX>
 __device__ __forceinline__ void r_ops(typename A::Amp (&v)[1 << RB], const uint4* ops, const uint4* coef, int begin,
                                       int end, uint32_t t, uint32_t lb) {
     for (int oi = begin; oi < end; oi++) {
@@ -405,6 +572,24 @@ __device__ __forceinline__ void r_ops(typename A::Amp (&v)[1 << RB], const uint4
         case RC_SWAP + 1:
             if constexpr (RB > 3) r_swap<A, RB, 1>(v, jm);
             break;
+        case RC_CHAN1 + 0:
+            if constexpr (DMX && EXACT) r_chan1<RB, 0, (RB > 3 ? 2 : 1)>(v, m, (int)w1.y);
+            break;
+        case RC_CHAN1 + 1:
+            if constexpr (DMX && EXACT && RB > 3) r_chan1<RB, 1, 2>(v, m, (int)w1.y);
+            break;
+        case RC_CHAN2:
+            if constexpr (DMX && EXACT && RB > 3) r_chan2(v, m, (int)w1.y);
+            break;
+        case RC_PAULI2:
+            if constexpr (DMX && !EXACT && RB > 3) r_pauli2(v, m);
+            break;
+        case RC_REAL2 + 0:
+            if constexpr (DMX && !EXACT) r_real2<RB, 0>(v, m, w1.y != 0);
+            break;
+        case RC_REAL2 + 1:
+            if constexpr (DMX && !EXACT && RB > 3) r_real2<RB, 1>(v, m, w1.y != 0);
+            break;
         case RC_NEG:
 #pragma unroll
             for (int j = 0; j < (1 << RB); j++)
@@ -484,7 +669,7 @@ constexpr int reg_ctas() {
 // the last segment has read it: thread 0 then issues the load of the tile
 // nbuf tiles on, which arrives while this one computes.  Every wait is
 // bounded: one that gives up sets *err and the pass's result is void.
-template <typename A, bool EXACT, int RB>
+template <typename A, bool EXACT, int RB, bool DMX>
 __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
     k_reg_tiles(typename A::Amp* __restrict__ st, const RHdr phdr, const uint4* __restrict__ gblob,
                 int* __restrict__ err, const __grid_constant__ CUtensorMap tmap) {
@@ -566,7 +751,7 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
                 if (threadIdx.x == 0 && (uint64_t)t + (uint64_t)nbuf * grid < hdr.ntiles) load(t + nbuf * grid, b);
             }
             if (!mine) continue;
-            r_ops<A, EXACT, RB>(v, ops, coef, (int)sg.x, (int)sg.y, t, lb);
+            r_ops<A, EXACT, RB, DMX>(v, ops, coef, (int)sg.x, (int)sg.y, t, lb);
             // the place again from the segment's words: kept through the ops
             // it would take registers from the amplitudes
             asm volatile("" ::: "memory");
@@ -626,6 +811,8 @@ static bool is_perm(const LGate& g) { return g.cls == GC_X || g.cls == GC_SWAP; 
 
 static bool reg_width(uint32_t nbits) { return nbits >= 4 && nbits <= 33; }
 static bool reg_gate(const LGate& g) { return !((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1)); }
+// steps on two qubits of a density matrix: all four register positions
+static bool four_bits(const LGate& g) { return g.cls == GC_CHAN2 || g.cls == GC_PAULI2; }
 
 bool reg_supported(const std::vector<LGate>& prog, uint32_t nbits) {
     if (!reg_width(nbits)) return false;
@@ -849,9 +1036,11 @@ struct Sign {
 struct PassBuilder {
     int rb;
     bool exact;
+    bool dm_form;         // a density matrix's FUSED program
     int8_t local[64];     // global bit -> tile position, -1 outside
     int8_t outside[64];   // global bit -> bit of the tile's number
     RegPass* p;
+    std::vector<std::pair<uint32_t, size_t>> shared;  // coefficients of density-matrix steps
 
     bool fits(const SegPlan& s, const LGate& g) const {
         if (!need_mask(g, exact)) return true;
@@ -859,14 +1048,18 @@ struct PassBuilder {
         for (int i = 0; i < g.k; i++)
             if (std::find(s.bits.begin(), s.bits.end(), (int)local[g.tb[i]]) == s.bits.end()) fresh++;
         if ((int)s.bits.size() + fresh > rb) return false;
-        if (g.k == 1) return true;
-        const int a = local[g.tb[0]], b = local[g.tb[1]];
-        for (const auto& q : s.pairs) {
-            if (q.first == a && q.second == b) return true;
-            if (g.cls == GC_SWAP && q.first == b && q.second == a) return true;
-            if (q.first == a || q.second == a || q.first == b || q.second == b) return false;
+        size_t more = 0;  // pairs that it would add
+        for (int i = 0; i + 1 < g.k; i += 2) {
+            const int a = local[g.tb[i]], b = local[g.tb[i + 1]];
+            bool have = false;
+            for (const auto& q : s.pairs) {
+                have |= q.first == a && q.second == b;
+                have |= g.cls == GC_SWAP && q.first == b && q.second == a;
+                if (!have && (q.first == a || q.second == a || q.first == b || q.second == b)) return false;
+            }
+            more += !have;
         }
-        return (int)s.pairs.size() < rb / 2;
+        return s.pairs.size() + more <= (size_t)rb / 2;
     }
     void add(SegPlan& s, const LGate& g) const {
         s.gates.push_back(&g);
@@ -874,11 +1067,11 @@ struct PassBuilder {
         for (int i = 0; i < g.k; i++)
             if (std::find(s.bits.begin(), s.bits.end(), (int)local[g.tb[i]]) == s.bits.end())
                 s.bits.push_back(local[g.tb[i]]);
-        if (g.k == 2) {
-            const int a = local[g.tb[0]], b = local[g.tb[1]];
-            for (const auto& q : s.pairs)
-                if (q.first == a || q.first == b) return;
-            s.pairs.push_back({a, b});
+        for (int i = 0; i + 1 < g.k; i += 2) {
+            const int a = local[g.tb[i]], b = local[g.tb[i + 1]];
+            bool have = false;
+            for (const auto& q : s.pairs) have |= q.first == a || q.first == b;
+            if (!have) s.pairs.push_back({a, b});
         }
     }
     void emit(const SegPlan& s) {
@@ -1045,6 +1238,28 @@ struct PassBuilder {
                     flush_sign(z);
                 }
             }
+            if (dm_form && g->cls == GC_DENSE && g->k == 2 && g->nc == 0) {
+                std::vector<Cx> m;
+                bool cols = false;
+                if (real_up_to_phases(g->m, m, &cols)) {
+                    op.coef = (uint32_t)p->coef.size();
+                    op.sel0 = cols;
+                    p->coef.insert(p->coef.end(), m.begin(), m.end());
+                    push(RC_REAL2 + p0 / 2, 0xffffu, op);
+                    continue;
+                }
+            }
+            if (g->cls >= GC_CHAN1) {
+                op.coef = coefs_of(dm_coefs(*g, p0 != 0));
+                if (g->cls == GC_PAULI2) {
+                    push(RC_PAULI2, 0xffffu, op);
+                } else {
+                    const uint32_t per = g->cls == GC_CHAN1 ? 3 : 5;
+                    op.sel0 = (uint32_t)g->m.size() / per;
+                    push(g->cls == GC_CHAN1 ? RC_CHAN1 + p0 / 2 : (uint32_t)RC_CHAN2, 0xffffu, op);
+                }
+                continue;
+            }
             op.coef = (uint32_t)p->coef.size();
             uint32_t code;
             auto is_real = [&](int i) { return g->m[i].im == 0.0; };
@@ -1076,6 +1291,73 @@ struct PassBuilder {
         flush();
         sg.op_end = (int32_t)p->ops.size();
         if (sg.op_end > sg.op_begin) p->segs.push_back(sg);
+    }
+
+    // A 4 x 4 matrix as a real one with a phase for every row, or for every
+    // column: the reals (8), then the phases (4).
+    static bool real_up_to_phases(const std::vector<Cx>& m, std::vector<Cx>& out, bool* cols) {
+        for (int side = 0; side < 2; side++) {
+            double R[16];
+            Cx f[4];
+            bool ok = true;
+            for (int r = 0; r < 4 && ok; r++) {
+                auto at = [&](int c) { return side ? m[4 * c + r] : m[4 * r + c]; };
+                int big = 0;
+                for (int c = 1; c < 4; c++)
+                    if (std::hypot(at(c).re, at(c).im) > std::hypot(at(big).re, at(big).im)) big = c;
+                const double norm = std::hypot(at(big).re, at(big).im);
+                f[r] = norm > 0.0 ? unit(at(big)) : Cx{1.0, 0.0};
+                for (int c = 0; c < 4; c++) {
+                    const Cx x = cmul(at(c), conj(f[r]));
+                    ok &= std::fabs(x.im) <= 1e-15 * norm;  // rounding of the products
+                    R[side ? 4 * c + r : 4 * r + c] = x.re;
+                }
+            }
+            if (!ok) continue;
+            out.clear();
+            for (int i = 0; i < 16; i += 2) out.push_back(Cx{R[i], R[i + 1]});
+            out.insert(out.end(), f, f + 4);
+            *cols = side == 1;
+            return true;
+        }
+        return false;
+    }
+
+    // The coefficients of a density-matrix step; swapped: its first qubit sits
+    // at the second pair of positions.
+    static std::vector<Cx> dm_coefs(const LGate& g, bool swapped) {
+        if (!four_bits(g) || !swapped) return g.m;
+        auto sw = [](int i) { return ((i & 1) << 1) | (i >> 1); };
+        std::vector<Cx> out(g.m);
+        const double* in = &g.m[0].re;
+        double* o = &out[0].re;
+        if (g.cls == GC_PAULI2) {
+            for (int d = 0; d < 4; d++)
+                for (int i = 0; i < 4; i++)
+                    for (int k = 0; k < 4; k++) o[16 * d + 4 * i + k] = in[16 * sw(d) + 4 * sw(i) + sw(k)];
+            return out;
+        }
+        for (size_t q = 0; q < g.m.size() / 5; q++) {
+            uint32_t x;
+            memcpy(&x, &in[10 * q], 4);
+            x = (uint32_t)sw((int)x);
+            memcpy(&o[10 * q], &x, 4);
+            for (int i = 0; i < 4; i++) {
+                o[10 * q + 2 + i] = in[10 * q + 2 + sw(i)];
+                o[10 * q + 6 + i] = in[10 * q + 6 + sw(i)];
+            }
+        }
+        return out;
+    }
+    // Where the pass holds these coefficients (a circuit's channels are often
+    // the same on every qubit).
+    uint32_t coefs_of(const std::vector<Cx>& m) {
+        for (const auto& q : shared)
+            if (q.second == m.size() && memcmp(&p->coef[q.first], m.data(), m.size() * sizeof(Cx)) == 0) return q.first;
+        const uint32_t at = (uint32_t)p->coef.size();
+        p->coef.insert(p->coef.end(), m.begin(), m.end());
+        shared.push_back({at, m.size()});
+        return at;
     }
 
     // A CZ (one control or two targets, one entry -1, the others 1).
@@ -1213,7 +1495,7 @@ size_t pass_bytes(const RegPass& p, size_t coef_bytes) {
 
 // The plan of prog[0 .. ngates).
 static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int32_t precision, int tbits_max,
-                           bool exact, RegPlan& out) {
+                           bool exact, RegPlan& out, bool dm = false) {
     out.passes.clear();
     out.blob.clear();
     const size_t amp = precision == YAO_C128 ? 16 : 8, coef_bytes = precision == YAO_C128 ? 16 : 32;
@@ -1226,7 +1508,10 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     // (8 in a 2^12 tile: at most 512 threads), which shortens an op's chain
     // where the time of one CTA is the time of the pass.
     const uint64_t ntiles = 1ull << (nbits - tbits);
-    const int rb = ntiles >= 296 ? 4 : (tbits > 11 ? 3 : 2);
+    int rb = ntiles >= 296 ? 4 : (tbits > 11 ? 3 : 2);
+    bool four = false;
+    for (size_t i = 0; i < ngates; i++) four |= four_bits(prog[i]);
+    if (four) rb = 4;
     std::vector<char> used(ngates, 0);
     size_t i0 = 0, left = ngates;
     while (left) {
@@ -1258,6 +1543,7 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
         PassBuilder pb;
         pb.rb = rb;
         pb.exact = exact;
+        pb.dm_form = !exact && dm;
         int nt = 0, no = 0;
         for (uint32_t b = 0; b < 64; b++) {
             pb.local[b] = pb.outside[b] = -1;
@@ -1287,8 +1573,9 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
                     continue;
                 }
                 // a diagonal may become one op per combination of its register targets
+                // (channels: once a pass, mostly)
                 const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) +
-                                  g.m.size() * coef_bytes;
+                                  (g.cls >= GC_CHAN1 ? std::min<size_t>(g.m.size(), 4) : g.m.size()) * coef_bytes;
                 if (bytes + nb > kRegBlobCap && !(p.ops.empty() && s.gates.empty())) {
                     full = true;
                     break;
@@ -1360,9 +1647,9 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
 
 // ================================================================== launch
 
-template <typename A, bool EXACT, int RB>
+template <typename A, bool EXACT, int RB, bool DMX>
 static int launch_k(Ctx* ctx, void* st, RHdr& hdr, const uint4* blob, size_t blob_bytes, const CUtensorMap& tmap) {
-    auto kern = k_reg_tiles<A, EXACT, RB>;
+    auto kern = k_reg_tiles<A, EXACT, RB, DMX>;
     static int optin = 0, sm_total = 0, fixed = 0;
     if (!optin) {
         int dev = 0, v = 0;
@@ -1396,11 +1683,11 @@ static int launch_k(Ctx* ctx, void* st, RHdr& hdr, const uint4* blob, size_t blo
     return YAO_OK;
 }
 
-template <typename A, bool EXACT>
+template <typename A, bool EXACT, bool DMX>
 static int launch_rb(Ctx* ctx, void* st, int rb, RHdr& hdr, const uint4* blob, size_t bytes, const CUtensorMap& tmap) {
-    if (rb == 4) return launch_k<A, EXACT, 4>(ctx, st, hdr, blob, bytes, tmap);
-    if (rb == 3) return launch_k<A, EXACT, 3>(ctx, st, hdr, blob, bytes, tmap);
-    return launch_k<A, EXACT, 2>(ctx, st, hdr, blob, bytes, tmap);
+    if (rb == 4) return launch_k<A, EXACT, 4, DMX>(ctx, st, hdr, blob, bytes, tmap);
+    if (rb == 3) return launch_k<A, EXACT, 3, DMX>(ctx, st, hdr, blob, bytes, tmap);
+    return launch_k<A, EXACT, 2, DMX>(ctx, st, hdr, blob, bytes, tmap);
 }
 
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
@@ -1431,14 +1718,18 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
         // (one tile: nothing to overlap, and no wait that could give up)
         h.use_tma = p.ntiles > 1 && tma_enabled() && tma_make_plan(p.tb, p.tbits, nbits, amp, st, h.tma, &tmap) ? 1 : 0;
         const uint4* blob = (const uint4*)(dblob + p.blob_off);
+        bool dmx = false;
+        for (const ROp& op : p.ops) dmx |= (op.head & 0xffu) >= RC_CHAN1;
         {
             ProfScope prof(ctx, exact ? "reg_pass_exact" : "reg_pass_fused",
                            (double)p.ntiles * (double)((uint64_t)1 << p.tbits) * 2.0 * (double)amp);
             if (precision == YAO_C128)
-                s = exact ? launch_rb<A128<true>, true>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap)
-                          : launch_rb<A128<false>, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap);
+                s = exact ? (dmx ? launch_rb<A128<true>, true, true>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap)
+                                 : launch_rb<A128<true>, true, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap))
+                          : (dmx ? launch_rb<A128<false>, false, true>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap)
+                                 : launch_rb<A128<false>, false, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap));
             else
-                s = launch_rb<A64, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap);
+                s = launch_rb<A64, false, false>(ctx, st, p.rb, h, blob, p.blob_bytes, tmap);
         }
         ctx->launches++;
         if (!s && cudaPeekAtLastError() != cudaSuccess) s = cuda_fail(cudaGetLastError(), "register pass launch");
@@ -1503,6 +1794,243 @@ int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
         }
     }
     return waits ? read_device_err(ctx, "apply") : YAO_OK;
+}
+
+// ==================================================== density matrices
+
+// entry (r, c) of a lowered Kraus operator
+static Cx entry_of(const LGate& g, int r, int c) {
+    const int nl = 1 << g.k;
+    if (g.cls == GC_DIAG) return r == c ? g.m[r] : Cx{0.0, 0.0};
+    return g.m[(size_t)r * nl + c];
+}
+
+static LGate dm_gate_on(const DMStep& s, int cls, int k) {
+    LGate g;
+    g.cls = cls;
+    g.k = 2 * k;
+    for (int i = 0; i < k; i++) {
+        g.tb[2 * i] = s.cols[0].tb[i];
+        g.tb[2 * i + 1] = s.rows[0].tb[i];
+    }
+    return g;
+}
+
+// The Kraus sum of a channel as GC_CHAN1 / GC_CHAN2: every operator has one
+// non-zero entry at most in a row, the same ones in K and conj(K), all real or
+// all imaginary (two imaginary weights multiply like real ones of opposite
+// sign).  False for other channels.
+static bool kraus_step(const std::vector<DMStep>& steps, size_t at, std::vector<LGate>& cache, LGate& g) {
+    const DMStep& s = steps[at];
+    if (s.like >= 0) {  // the same channel elsewhere: its coefficients, or none
+        if (cache[s.like].m.empty()) return false;
+        g = dm_gate_on(s, cache[s.like].cls, s.rows[0].k);
+        g.m = cache[s.like].m;
+        return true;
+    }
+    if (s.rows.empty()) return false;
+    const int k = s.rows[0].k, nl = 1 << k;
+    if (k > 2) return false;
+    g = dm_gate_on(s, k == 1 ? GC_CHAN1 : GC_CHAN2, k);
+    for (size_t q = 0; q < s.rows.size(); q++) {
+        int src[4];
+        double r[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
+        const bool diag = s.rows[q].cls == GC_DIAG;
+        bool real = true, imag = true;
+        for (int a = 0; a < nl; a++) {
+            src[a] = -1;
+            for (int b = 0; b < nl; b++) {
+                const Cx x = entry_of(s.rows[q], a, b), y = entry_of(s.cols[q], a, b);
+                if (is(x, 0.0) != is(y, 0.0)) return false;
+                // a diagonal's zeros multiply too (an infinity becomes NaN)
+                if (diag ? a != b : is(x, 0.0)) continue;
+                if (src[a] >= 0) return false;
+                src[a] = b;
+                real &= x.im == 0.0 && y.im == 0.0;
+                imag &= x.re == 0.0 && y.re == 0.0;
+            }
+        }
+        if (!real && (diag || !imag)) return false;
+        for (int a = 0; a < nl; a++) {
+            if (src[a] < 0) continue;
+            const Cx x = entry_of(s.rows[q], a, src[a]), y = entry_of(s.cols[q], a, src[a]);
+            r[a] = real ? x.re : -x.im;
+            c[a] = real ? y.re : y.im;
+        }
+        uint32_t type = 0;
+        if (k == 1) {
+            if (src[0] == 0 && src[1] == 1) type = 0;
+            else if (src[0] == 1 && src[1] == 0) type = 1;
+            else if (src[0] == 1 && src[1] < 0) type = 2;
+            else if (src[0] < 0 && src[1] == 0) type = 3;
+            else return false;
+        } else {
+            type = (uint32_t)src[0];
+            for (int a = 0; a < nl; a++)
+                if (src[a] < 0 || src[a] != (a ^ src[0])) return false;
+        }
+        Cx head{0.0, 0.0};
+        memcpy(&head.re, &type, 4);
+        g.m.push_back(head);
+        for (int a = 0; a < nl; a += 2) g.m.push_back(Cx{r[a], r[a + 1]});
+        for (int a = 0; a < nl; a += 2) g.m.push_back(Cx{c[a], c[a + 1]});
+    }
+    cache[at] = g;
+    return !g.m.empty();
+}
+
+// PLAIN steps on a density matrix.  Runs of gates and channels that the exact
+// register passes hold (the same products and sums in the same order as the
+// lone passes) share passes where the passes cost less; others run alone.
+int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps) {
+    const uint32_t nb = 2 * d->nbits;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    YAO_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    const bool passes = reg_width(nb) && cs == cudaStreamCaptureStatusNone;
+    const double bytes = (double)d->bytes(), entries = (double)(1ull << nb);
+    auto alone_step = [&](const DMStep& s) -> int {
+        if (s.channel && s.like >= 0) {
+            std::vector<LGate> rows = steps[s.like].rows, cols = steps[s.like].cols;
+            for (LGate& g : rows) std::copy(s.rows[0].tb, s.rows[0].tb + kMaxTargets, g.tb);
+            for (LGate& g : cols) std::copy(s.cols[0].tb, s.cols[0].tb + kMaxTargets, g.tb);
+            return launch_dm_channel(ctx, d, rows, cols, {}, {});
+        }
+        if (s.channel) return launch_dm_channel(ctx, d, s.rows, s.cols, {}, {});
+        for (size_t i = 0; i < s.rows.size(); i++) {
+            int st = launch_dm_gate(ctx, d, s.rows[i], s.cols[i]);
+            if (st) return st;
+        }
+        return YAO_OK;
+    };
+    bool waits = false;
+    std::vector<LGate> cache(steps.size());
+    for (size_t i = 0; i < steps.size();) {
+        // the steps from i on that a register pass can run
+        std::vector<LGate> prog;
+        size_t end = i;
+        double alone = 0.0, flops = 0.0;
+        for (; passes && end < steps.size(); end++) {
+            const DMStep& s = steps[end];
+            if (s.channel) {
+                LGate g;
+                if (!kraus_step(steps, end, cache, g)) break;
+                // measured: 1-qubit channels at 5.3 TB/s, 2-qubit ones at 1.8
+                alone += 3e-6 + 2.0 * bytes / (g.cls == GC_CHAN1 ? 5.3e12 : 1.8e12);
+                flops += 6.0 * (double)(s.like >= 0 ? steps[s.like] : s).rows.size();
+                prog.push_back(std::move(g));
+                continue;
+            }
+            bool ok = true;
+            for (const LGate& g : s.rows) ok &= reg_gate(g);
+            if (!ok) break;
+            for (size_t q = 0; q < s.rows.size(); q++) {
+                alone += 3e-6 + 2.0 * bytes / 6.2e12;
+                flops += 2.0 * gate_flops(s.rows[q]);
+                prog.push_back(s.rows[q]);
+                prog.push_back(s.cols[q]);
+            }
+        }
+        if (end - i >= 2) {
+            // the rule of plain_run
+            RegPlan plan;
+            reg_plan_range(prog.data(), prog.size(), nb, YAO_C128, 11, true, plan);
+            if ((double)plan.passes.size() * (8e-6 + 2.0 * bytes / 5.2e12) + flops * entries / 1e13 < alone) {
+                int s = reg_launch(ctx, d->d, nb, YAO_C128, true, plan, 0, 1);
+                if (s) return s;
+                waits |= nb > 11;
+                i = end;
+                continue;
+            }
+        }
+        for (end = std::max(i + 1, end); i < end; i++) {
+            int s = alone_step(steps[i]);
+            if (s) return s;
+        }
+    }
+    return waits ? read_device_err(ctx, "density-matrix apply") : YAO_OK;
+}
+
+// FUSED steps on a density matrix; *done = false where a step has no form here
+// (three or more targets, other 2-qubit channels): the block passes take it.
+// Measured on 12 qubits (256 MiB), eight layers of rotations, CZ (a channel
+// after each) and dampings: block passes 13.5 ms, these 5.3 (4.4 on the
+// device, bound by double-precision multiply-adds: a complex 4 x 4 step takes
+// 16 an entry, a real one with phases 12).
+int dm_fused_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps, bool* done) {
+    *done = false;
+    const uint32_t nb = 2 * d->nbits;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    YAO_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    if (!reg_width(nb) || cs != cudaStreamCaptureStatusNone) return YAO_OK;
+    // Everything on one qubit is a 4 x 4 superoperator on its column and row
+    // bit (they multiply together), a 2-qubit Pauli-type channel four real
+    // 4 x 4 matrices; other gates act on row and column bits apart.
+    std::vector<LGate> prog;
+    std::vector<std::vector<Cx>> cache(steps.size());
+    for (size_t si = 0; si < steps.size(); si++) {
+        const DMStep& s = steps[si];
+        const int k = s.rows[0].k, nl = 1 << k;
+        if (s.like >= 0) {
+            LGate g = dm_gate_on(s, k == 1 ? GC_DENSE : GC_PAULI2, k);
+            g.m = cache[s.like];
+            prog.push_back(std::move(g));
+            continue;
+        }
+        if (!s.channel && (k > 1 || s.rows[0].nc || s.rows.size() > 1)) {
+            for (size_t i = 0; i < s.rows.size(); i++) {
+                if (!reg_gate(s.rows[i])) return YAO_OK;
+                prog.push_back(s.rows[i]);
+                prog.push_back(s.cols[i]);
+            }
+            continue;
+        }
+        auto at = [&](const LGate& g, int r, int c) {
+            return g.cls == GC_X ? Cx{r != c ? 1.0 : 0.0, 0.0} : entry_of(g, r, c);
+        };
+        if (k > 2) return YAO_OK;
+        // S[(a, b), (c, e)] = sum_q K_q[a][c] conj(K_q)[b][e], (a, b) at b + nl a
+        std::vector<Cx> S((size_t)nl * nl * nl * nl, Cx{0.0, 0.0});
+        for (size_t q = 0; q < s.rows.size(); q++)
+            for (int a = 0; a < nl; a++)
+                for (int b = 0; b < nl; b++)
+                    for (int c = 0; c < nl; c++)
+                        for (int e = 0; e < nl; e++) {
+                            const Cx t = cmul(at(s.rows[q], a, c), at(s.cols[q], b, e));
+                            Cx& x = S[(size_t)(b + nl * a) * nl * nl + (e + nl * c)];
+                            x.re += t.re;
+                            x.im += t.im;
+                        }
+        if (k == 1) {
+            LGate g = dm_gate_on(s, GC_DENSE, 1);
+            cache[si] = S;
+            g.m = std::move(S);
+            prog.push_back(std::move(g));
+            continue;
+        }
+        LGate g = dm_gate_on(s, GC_PAULI2, 2);
+        g.m.assign(32, Cx{0.0, 0.0});
+        double* m = &g.m[0].re;
+        for (int a = 0; a < 4; a++)
+            for (int b = 0; b < 4; b++)
+                for (int c = 0; c < 4; c++)
+                    for (int e = 0; e < 4; e++) {
+                        const Cx x = S[(size_t)(b + 4 * a) * 16 + (e + 4 * c)];
+                        if (is(x, 0.0)) continue;
+                        if ((a ^ c) != (b ^ e) || x.im != 0.0) return YAO_OK;
+                        m[16 * (a ^ b) + 4 * a + c] = x.re;
+                    }
+        cache[si] = g.m;
+        prog.push_back(std::move(g));
+    }
+    std::vector<LGate> work;
+    fuse_two_qubit(prog, nb, work);
+    if (!reg_supported(work, nb)) return YAO_OK;
+    RegPlan plan;
+    reg_plan_range(work.data(), work.size(), nb, YAO_C128, 11, false, plan, true);
+    int s = reg_launch(ctx, d->d, nb, YAO_C128, false, plan, 0, 1);
+    if (s) return s;
+    *done = true;
+    return nb > 11 ? read_device_err(ctx, "density-matrix apply") : YAO_OK;
 }
 
 }  // namespace yao

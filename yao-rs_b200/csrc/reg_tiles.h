@@ -52,7 +52,11 @@ enum RCode : uint32_t {
     RC_SWAP = 30,    // + pair, masked
     RC_PHASE = 32,   // the masked amplitudes times one coefficient
     RC_DIAG = 33,    // the masked amplitudes, each times its own coefficient
-    RC_NEG = 34      // the masked amplitudes times -1
+    RC_NEG = 34,     // the masked amplitudes times -1
+    RC_CHAN1 = 35,   // + pair: a 1-qubit Kraus sum; sel0: operators, three coefficients each (exact passes)
+    RC_CHAN2 = 37,   // a 2-qubit Kraus sum; sel0: operators, five coefficients each (exact passes)
+    RC_PAULI2 = 38,  // four real 4 x 4 matrices (not in exact passes)
+    RC_REAL2 = 39    // + pair: a real 4 x 4 matrix with a phase a row (sel0 = 0) or a column (1)
 };
 
 struct RegPass {
@@ -86,6 +90,9 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
                size_t step);
 
+// Fusion into blocks of at most 2 qubits (sv_tiles.cu); density-matrix steps
+// on two qubits are kept.
+void fuse_two_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vector<LGate>& out);
 // A program with each gate's own arithmetic in program order (the PLAIN
 // form): runs of gates as exact register passes where that is faster, else
 // one launch a gate; the results are the same bits either way.  Wide gates,

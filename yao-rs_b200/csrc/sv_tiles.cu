@@ -1722,8 +1722,9 @@ static void fuse_blocks(const std::vector<LGate>& prog_in, uint32_t nbits, int k
         for (int c = 0; c < g.nc; c++) S.push_back(g.cb[c]);
         int B = -1;
         for (int b : S) B = std::max(B, last[b]);
-        if ((int)S.size() > kMaxTargets) {
-            // too wide to fuse (its block matrix would exceed 2^6 x 2^6)
+        if ((int)S.size() > kMaxTargets || g.cls >= GC_CHAN1) {
+            // too wide to fuse (its block matrix would exceed 2^6 x 2^6), or a
+            // density-matrix step of the register passes
             Block pb;
             pb.passthrough = true;
             pb.gate = g;
@@ -1771,6 +1772,10 @@ static void fuse_blocks(const std::vector<LGate>& prog_in, uint32_t nbits, int k
         }
         out.push_back(g);
     }
+}
+
+void fuse_two_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vector<LGate>& out) {
+    fuse_blocks(prog, nbits, 2, out);
 }
 
 // ------------------------------------------------------------ execution

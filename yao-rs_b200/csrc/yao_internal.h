@@ -43,7 +43,12 @@ enum GateClass : int32_t {
     GC_X = 0,     // amplitude-pair swap on one target bit (instruct_x[_controlled])
     GC_SWAP = 1,  // swap of the |01> / |10> amplitudes of two bits (instruct_swap)
     GC_DIAG = 2,  // elementwise product by d[local index] (instruct_*_diag*)
-    GC_DENSE = 3  // dense 2^k x 2^k product (instruct_1q / _2q / _nq [+controlled])
+    GC_DENSE = 3, // dense 2^k x 2^k product (instruct_1q / _2q / _nq [+controlled])
+    // Steps on a density matrix as a 2n-bit vector that only register passes
+    // run (reg_tiles.h); targets: column bit, row bit of each qubit.
+    GC_CHAN1 = 4,  // 1-qubit Kraus sum of real-weighted permutations, operator by operator
+    GC_CHAN2 = 5,  // the same for 2-qubit Pauli-type channels
+    GC_PAULI2 = 6  // a 2-qubit Pauli-type channel as one real 4 x 4 matrix per orbit
 };
 
 struct LGate {
@@ -285,6 +290,19 @@ int launch_remove_gather_fixed(Ctx* ctx, const Reg* src, Reg* dst, const uint32_
 int launch_dm_from_reg(Ctx* ctx, const Reg* r, DM* d);
 int launch_dm_mixed_accum(Ctx* ctx, const Reg* r, double w, DM* d);
 int launch_dm_gate(Ctx* ctx, DM* d, const LGate& row, const LGate& col);
+// Steps of a density-matrix circuit in order, each with its own arithmetic:
+// shared exact register passes where that is faster, else one launch a step
+// (reg_tiles.cu).
+struct DMStep {
+    bool channel = false;
+    std::vector<LGate> rows, cols;  // the gate on row and column bits; a channel's Kraus operators
+    int like = -1;                  // an earlier step with the same channel: rows and cols hold its first operator only
+};
+int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps);
+// The FUSED form of a circuit (gates on row and column bits, channels as
+// superoperators) as register passes; *done = false, and nothing launched,
+// when some step does not fit them.
+int dm_fused_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps, bool* done);
 int launch_dm_channel(Ctx* ctx, DM* d, const std::vector<LGate>& rows, const std::vector<LGate>& cols,
                       const std::vector<uint32_t>& row_bits, const std::vector<uint32_t>& col_bits);
 int reduce_dm_trace(Ctx* ctx, const DM* d, Cx* out);
