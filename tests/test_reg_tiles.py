@@ -115,3 +115,30 @@ def test_plain_copies_instead_of_tma(monkeypatch):
         Y.apply_inplace(c, r, Y.MODE_TILED)
         assert np.max(np.abs(r.state_vec() - O.apply_circuit(c, psi))) == 0.0
         assert math.isfinite(r.norm())
+
+
+@pytest.mark.parametrize("n", [20, 21])
+@pytest.mark.parametrize("gates", [("Ry",), ("Ry", "Rz"), ("Rx", "Ry", "Rz")])
+def test_layers_of_rotations(n, gates):
+    """Four rotations at a time with one diagonal for their phases and the
+    signs of CZs among them (16 amplitudes a thread: 2^20 complex128, 2^21
+    complex64), CZs and CNOTs on random pairs and some on three qubits in
+    between; without phases (Ry) the signs are an op of their own."""
+    rng = np.random.default_rng([n, len(gates)])
+    els = []
+    for _ in range(4):
+        els += [Y.put([q], getattr(Gate, g)(float(rng.uniform(-3, 3)))) for q in range(n) for g in gates]
+        for _ in range(n):
+            p = [int(x) for x in rng.permutation(n)]
+            if rng.random() < 0.1:
+                els.append(Y.control(p[:2], [p[2]], Gate.Z))
+            else:
+                els.append(Y.control([p[0]], [p[1]], Gate.Z if rng.random() < 0.7 else Gate.X))
+        els += [Y.put([q], Gate.Ry(float(rng.uniform(-3, 3)))) for q in range(0, n, 3)]
+    c, psi = Y.Circuit.qubits(n, els), random_state(rng, n)
+    ref = O.apply_circuit(c, psi)
+    # a few roundings (1.1e-16, 6e-8) a gate on a state of norm 1
+    for prec, eps in ((Y.C128, 5e-16), (Y.C64, 6e-8)):
+        r = Y.ArrayReg.from_vec(n, psi).to_precision(prec)
+        Y.apply_inplace(c, r, Y.MODE_FUSED, 1)
+        assert np.linalg.norm(r.state_vec() - ref) < eps * len(els), prec

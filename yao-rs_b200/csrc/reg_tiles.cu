@@ -6,16 +6,18 @@
 // tile positions and applies all ops of the segment in registers; between
 // segments the tile changes hands through shared memory (one barrier).
 //
-// What bounds it: an op's own latency (its description from shared memory,
-// the jump to its code, its coefficients: about 290 cycles) beside its FP64
-// or packed FP32 work (192 cycles a warp for a rotation of 16 amplitudes),
-// with three warps a scheduler to overlap them: the FP64 pipe is busy half of
-// the time.  So ops are few and large: a rotation carries the phase before
-// it and the CZ signs around it (561 ops for the 1950 gates of the layered
-// circuit, n = 28, 20 layers), and 16 amplitudes a thread share each op's
-// fixed cost.  Against the block passes of sv_tiles.cu on that circuit, kernel
-// time: complex128 FUSED 185 -> 109 ms, complex64 FUSED 222 -> 111 ms; TILED
-// at n = 25, 8 layers (no multiplication of gates, no FMA) 62.7 -> 23 ms.
+// What bounds it: issue.  A rotation of 16 amplitudes is 192 cycles a warp on
+// the FP64 pipe (complex64: packed FP32), with about as many instructions for
+// its description, coefficients, signs and the segment's addresses around it,
+// and three warps a scheduler to overlap their latencies: the FP64 pipe is
+// busy 55% of the time.  So ops are few and large: a rotation carries the
+// phase before it and the CZ signs around it (561 ops for the 1950 gates of
+// the layered circuit, n = 28, 20 layers), four of them share one diagonal
+// for phases and signs and one way through the op loop, and 16 amplitudes a
+// thread share each op's fixed cost.  Against the block passes of sv_tiles.cu
+// on that circuit, kernel time: complex128 FUSED 185 -> 94 ms (105 without the
+// layers of four and the kept places), complex64 FUSED 222 -> 91 ms (111);
+// TILED at n = 25, 8 layers (no multiplication of gates, no FMA) 62.7 -> 23 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -198,7 +200,13 @@ __device__ __forceinline__ void r_sign(typename A::Amp (&v)[1 << RB], uint32_t s
     if (sg) {
 #pragma unroll
         for (int j = 0; j < (1 << RB); j++)
-            if (!(j & (1 << P))) v[j | (1 << P)] = A::sign(v[j | (1 << P)], (sg << (31 - j)) & 0x80000000u);
+            if (!(j & (1 << P))) {
+                // (measured both ways: complex128 2% faster without the tests, complex64 6% with them)
+                if constexpr (sizeof(typename A::Amp) == 16)
+                    v[j | (1 << P)] = A::sign(v[j | (1 << P)], (sg << (31 - j)) & 0x80000000u);
+                else if ((sg >> j) & 1u)
+                    v[j | (1 << P)] = A::neg(v[j | (1 << P)]);
+            }
     }
 }
 
@@ -481,6 +489,16 @@ __device__ __forceinline__ void r_real2(double2 (&v)[1 << RB], const uint4* m, b
     }
 }
 
+// A REAL1 op without pair signs from its words, without the way over the switch.
+template <typename A, int RB, int P>
+__device__ __forceinline__ void r_next(typename A::Amp (&v)[1 << RB], const uint4*& op, const uint4* coef, uint32_t t,
+                                       uint32_t lb) {
+    const uint4 w0 = op[0], w1 = op[1];
+    op += 2;
+    const bool on = (t & w0.w) == w1.x && (lb & (w0.z & 0xffffu)) == (w0.z >> 16);
+    r_real1<A, RB, P>(v, coef + (size_t)w0.y * A::kCoef16, 0u, on && (w1.w >> 16) ? 0x80000000u : 0u);
+}
+
 // The ops of one segment on one thread's amplitudes.  t: the tile's number;
 // lb: the thread's tile position (register positions at 0).
 // DMX: density-matrix steps among the ops (a kernel of its own: their
@@ -590,6 +608,21 @@ __device__ __forceinline__ void r_ops(typename A::Amp (&v)[1 << RB], const uint4
         case RC_REAL2 + 1:
             if constexpr (DMX && !EXACT && RB > 3) r_real2<RB, 1>(v, m, w1.y != 0);
             break;
+        case RC_LAYER:
+            if constexpr (!EXACT && RB > 3 && !DMX) {
+                if (w1.y != ~0u) {
+                    const uint4* d = coef + (size_t)w1.y * A::kCoef16;
+#pragma unroll
+                    for (int j = 1; j < (1 << RB); j++) v[j] = A::mul(A::load(d + (j - 1) * A::kCoef16), v[j]);
+                }
+                const uint4* next = ops + 2 * oi;
+                r_next<A, RB, 0>(v, next, coef, t, lb);
+                r_next<A, RB, 1>(v, next, coef, t, lb);
+                r_next<A, RB, 2>(v, next, coef, t, lb);
+                r_next<A, RB, 3>(v, next, coef, t, lb);
+                oi += 3;
+            }
+            break;
         case RC_NEG:
 #pragma unroll
             for (int j = 0; j < (1 << RB); j++)
@@ -627,15 +660,19 @@ __device__ __forceinline__ uint64_t r_deposit(const RHdr& h, uint32_t l) {
 // 0) and the swizzled byte offsets of that and of each register position.
 template <int RB>
 struct RPlace {
-    uint32_t lb, sb, so[RB];
-    __device__ __forceinline__ RPlace(const uint4& sg, uint32_t amp) {
-        lb = threadIdx.x;
+    uint32_t sb, so[RB];
+    static __device__ __forceinline__ uint32_t position(const uint4& sg) {
+        uint32_t lb = threadIdx.x;
 #pragma unroll
         for (int i = 0; i < RB; i++) {
             const uint32_t p = (sg.z >> (8 * i)) & 0xffu;
             lb = ((lb >> p) << (p + 1)) | (lb & ((1u << p) - 1));
-            so[i] = tma::swizzle128(amp << ((sg.w >> (8 * i)) & 0xffu));
         }
+        return lb;
+    }
+    __device__ __forceinline__ RPlace(const uint4& sg, uint32_t lb, uint32_t amp) {
+#pragma unroll
+        for (int i = 0; i < RB; i++) so[i] = tma::swizzle128(amp << ((sg.w >> (8 * i)) & 0xffu));
         sb = tma::swizzle128(lb * amp);
     }
     __device__ __forceinline__ uint32_t at(int j) const {
@@ -650,12 +687,10 @@ struct RPlace {
 // Threads of a CTA and CTAs an SM that the registers are divided for.  At 16
 // amplitudes a thread, complex128 takes 168 registers (at 128 the compiler
 // spills, and the register passes of the layered circuit, n = 28, 20 layers,
-// took 118 ms against 109 ms) and 2^11 tiles; complex64 takes 128 and 2^12
-// tiles (one more moving bit a pass: 111 ms against 116 ms).
+// took 118 ms against 109 ms then) and 2^11 tiles; complex64 takes 128 and
+// 2^12 tiles (one more moving bit a pass: 111 ms against 116 ms then).
 template <typename A, int RB>
-constexpr int reg_threads() {
-    return RB < 4 ? 512 : sizeof(typename A::Amp) == 16 ? 128 : 256;
-}
+constexpr int kRegThreads = RB < 4 ? 512 : sizeof(typename A::Amp) == 16 ? 128 : 256;
 template <typename A, int RB>
 constexpr int reg_ctas() {
     return RB < 4 ? 1 : sizeof(typename A::Amp) == 16 ? 3 : 2;
@@ -670,7 +705,7 @@ constexpr int reg_ctas() {
 // nbuf tiles on, which arrives while this one computes.  Every wait is
 // bounded: one that gives up sets *err and the pass's result is void.
 template <typename A, bool EXACT, int RB, bool DMX>
-__global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
+__global__ void __launch_bounds__(kRegThreads<A, RB>, reg_ctas<A, RB>())
     k_reg_tiles(typename A::Amp* __restrict__ st, const RHdr phdr, const uint4* __restrict__ gblob,
                 int* __restrict__ err, const __grid_constant__ CUtensorMap tmap) {
     typedef typename A::Amp Amp;
@@ -679,6 +714,7 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
     __shared__ RHdr hdr;
     __shared__ uint64_t full_bar[4];
     __shared__ uint64_t tbase[4];  // base index of the tile in each buffer
+    __shared__ uint32_t place[kRegThreads<A, RB>];
     if (threadIdx.x == 0) hdr = phdr;
     __syncthreads();
     unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -710,6 +746,9 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
     const uint4* coef = blob + hdr.coef16;
     const bool mine = threadIdx.x < (1u << (hdr.tbits - RB));
     const int last = hdr.nsegs - 1;
+    // where the thread's amplitudes of the last segment go in a tile (its
+    // lowest three bits are those of the tile position; read by it alone)
+    place[threadIdx.x] = (uint32_t)(r_deposit(hdr, RPlace<RB>::position(blob[last])) >> 3);
     bool dead = false;
     uint32_t b = 0, par = 0;
     for (; t < hdr.ntiles; t += grid) {
@@ -735,11 +774,10 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
         for (int si = 0; si <= last; si++) {
             const uint4 sg = blob[si];
             if (si) __syncthreads();
-            uint32_t lb;
+            const uint32_t lb = RPlace<RB>::position(sg);
             Amp v[1 << RB];
             {
-                const RPlace<RB> pl(sg, AB);
-                lb = pl.lb;
+                const RPlace<RB> pl(sg, lb, AB);
                 if (mine) {
 #pragma unroll
                     for (int j = 0; j < (1 << RB); j++) v[j] = *(const Amp*)(s + pl.at(j));
@@ -756,12 +794,12 @@ __global__ void __launch_bounds__(reg_threads<A, RB>(), reg_ctas<A, RB>())
             // it would take registers from the amplitudes
             asm volatile("" ::: "memory");
             const uint4 sg2 = blob[si];
-            const RPlace<RB> pl(sg2, AB);
+            const RPlace<RB> pl(sg2, lb, AB);
             if (si < last) {
 #pragma unroll
                 for (int j = 0; j < (1 << RB); j++) *(Amp*)(s + pl.at(j)) = v[j];
             } else {
-                Amp* dst = st + (base | r_deposit(hdr, pl.lb));
+                Amp* dst = st + (base | ((uint64_t)place[threadIdx.x] << 3) | (lb & 7u));
                 uint64_t goff[RB];
 #pragma unroll
                 for (int i = 0; i < RB; i++) goff[i] = 1ull << hdr.tb[(sg2.w >> (8 * i)) & 0xffu];
@@ -1015,8 +1053,10 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
 
 // Description of a pass kept below this, so that three CTAs of 2^11
 // complex128 amplitudes (two buffers each) share an SM; a longer run of
-// gates becomes further passes.
-constexpr size_t kRegBlobCap = 8 * 1024;
+// gates becomes further passes.  Two CTAs of 2^12 complex64 amplitudes leave
+// more room, and its coefficients take twice the bytes (at 8 KB the layered
+// circuit took 27 passes instead of 21).
+constexpr size_t kRegBlobCap = 8 * 1024, kRegBlobCap64 = 16 * 1024;
 
 namespace {
 
@@ -1289,8 +1329,123 @@ struct PassBuilder {
         }
         for (const Sign& z : signs) flush_sign(z);
         flush();
+        if (!exact && !dm_form && rb == 4) group_layers((size_t)sg.op_begin);
         sg.op_end = (int32_t)p->ops.size();
         if (sg.op_end > sg.op_begin) p->segs.push_back(sg);
+    }
+
+    // Brings matrices on positions 0 to 3 that are real up to a phase of the
+    // second column together (RC_LAYER) where the ops in between commute with
+    // them: such matrices on other positions, unless one negates the pairs of
+    // the other's position.  The phases, and the signs between two of the four
+    // (a CZ before both), become one diagonal: 4 x 4 + 4 multiply-adds an
+    // amplitude instead of 4 x 6, and the four go through the op loop at once.
+    // Measured on the layered circuit, n = 28, 20 layers: complex128 105 -> 96
+    // ms, complex64 111 -> 99.  (Three of four positions with a test for each:
+    // 98 and 104, the code is no longer one straight line.)
+    void group_layers(size_t begin) {
+        auto code = [](const ROp& op) { return (op.head & 0xffu) & ~3u; };
+        auto pos = [](const ROp& op) { return (int)(op.head & 3u); };
+        // pairs of position a negated where position b is 1
+        auto cz = [](int a, int b) {
+            uint32_t m = 0;
+            for (uint32_t j = 0; j < 16; j++) m |= (uint32_t)(!((j >> a) & 1u) && ((j >> b) & 1u)) << j;
+            return m;
+        };
+        // the positions whose bits negate pairs of op's; false: not a product of CZs
+        auto reads = [&](const ROp& op, uint32_t& r) {
+            uint32_t left = op.sign & 0xffffu;
+            r = 0;
+            for (int q = 0; q < 4; q++)
+                if (q != pos(op) && (left >> (1u << q)) & 1u) {
+                    left ^= cz(pos(op), q);
+                    r |= 1u << q;
+                }
+            return left == 0;
+        };
+        // the second column's phase; false: it has none
+        auto phase = [&](const ROp& op, Cx& u, Cx (&m)[2]) {
+            const Cx* c = &p->coef[op.coef];
+            m[0] = c[0];
+            m[1] = c[1];
+            u = Cx{1.0, 0.0};
+            if (code(op) == RC_REAL1) return true;
+            const Cx b = c[1], d = c[2];
+            const double nb = std::hypot(b.re, b.im), nd = std::hypot(d.re, d.im), norm = std::max(nb, nd);
+            u = nb > nd ? unit(b) : unit(d);
+            const Cx x = cmul(b, conj(u)), y = cmul(d, conj(u));
+            m[0] = Cx{c[0].re, x.re};
+            m[1] = Cx{c[0].im, y.re};
+            return std::fabs(x.im) <= 1e-15 * norm && std::fabs(y.im) <= 1e-15 * norm;
+        };
+        std::vector<ROp> list(p->ops.begin() + (long)begin, p->ops.end()), out;
+        while (!list.empty()) {
+            int at[4] = {-1, -1, -1, -1};
+            uint32_t held = 0, read = 0, have = 0, r[4];  // positions of passed ops; those they read; the group's
+            Cx u[4], m[4][2];
+            for (size_t k = 0; k < list.size() && k < 16 && have != 15u; k++) {
+                const ROp& op = list[k];
+                if (code(op) != RC_RCOL1 && code(op) != RC_REAL1) break;
+                const int P = pos(op);
+                uint32_t rd;
+                if (!reads(op, rd)) break;
+                // (a sign that reads a member before it stays after that member)
+                if (!(((held | read | have) >> P) & 1u) && !(rd & (held | have)) && phase(op, u[P], m[P])) {
+                    at[P] = (int)k;
+                    r[P] = rd;
+                    have |= 1u << P;
+                } else {
+                    held |= 1u << P;
+                    read |= rd;
+                }
+            }
+            if (have != 15u) {
+                out.push_back(list[0]);
+                list.erase(list.begin());
+                continue;
+            }
+            Cx d[16];
+            uint32_t minus = 0;
+            bool phases = false;
+            for (uint32_t j = 0; j < 16; j++) {
+                d[j] = Cx{1.0, 0.0};
+                for (int P = 0; P < 4; P++) {
+                    if (!((j & have) >> P & 1u)) continue;
+                    d[j] = cmul(d[j], u[P]);
+                    if (__builtin_popcount(r[P] & j) & 1) minus ^= 1u << j;
+                }
+                if ((minus >> j) & 1u) d[j] = Cx{-d[j].re, -d[j].im};
+            }
+            for (int P = 0; P < 4; P++) phases |= ((have >> P) & 1u) && !is(u[P], 1.0);
+            if (!phases && minus) {
+                ROp neg;
+                memset(&neg, 0, sizeof(neg));
+                neg.head = RC_NEG | (minus << 16);
+                out.push_back(neg);
+            }
+            bool first = true;
+            for (int P = 0; P < 4; P++) {
+                if (!((have >> P) & 1u)) continue;
+                ROp op = list[(size_t)at[P]];
+                op.head = (op.head & ~0xffu) | (first ? (uint32_t)RC_LAYER : (uint32_t)RC_REAL1 + (uint32_t)P);
+                op.sign &= 0xffff0000u;
+                op.sel0 = ~0u;
+                op.sel1 = have;
+                // (in the place of the op's own coefficients)
+                p->coef[op.coef] = m[P][0];
+                p->coef[op.coef + 1] = m[P][1];
+                if (first && phases) {
+                    op.sel0 = (uint32_t)p->coef.size();
+                    p->coef.insert(p->coef.end(), d + 1, d + 16);
+                }
+                out.push_back(op);
+                first = false;
+            }
+            std::sort(at, at + 4);
+            for (int q = 3; q >= 0 && at[q] >= 0; q--) list.erase(list.begin() + at[q]);
+        }
+        p->ops.resize(begin);
+        p->ops.insert(p->ops.end(), out.begin(), out.end());
     }
 
     // A 4 x 4 matrix as a real one with a phase for every row, or for every
@@ -1574,9 +1729,11 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
                 }
                 // a diagonal may become one op per combination of its register targets
                 // (channels: once a pass, mostly)
-                const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) +
+                // (a layer of four matrices: their reals and a diagonal)
+                const size_t more = !exact && rb == 4 && g.cls == GC_DENSE && g.k == 1 ? 3 * coef_bytes : 0;
+                const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) + more +
                                   (g.cls >= GC_CHAN1 ? std::min<size_t>(g.m.size(), 4) : g.m.size()) * coef_bytes;
-                if (bytes + nb > kRegBlobCap && !(p.ops.empty() && s.gates.empty())) {
+                if (bytes + nb > (precision == YAO_C128 ? kRegBlobCap : kRegBlobCap64) && !(p.ops.empty() && s.gates.empty())) {
                     full = true;
                     break;
                 }
@@ -1668,7 +1825,7 @@ static int launch_k(Ctx* ctx, void* st, RHdr& hdr, const uint4* blob, size_t blo
     // as many CTAs as the registers allow, then as many tile buffers as fit
     auto ctas = [&](int nbuf) {
         const size_t per = (size_t)nbuf * tile + blob_bytes + 1024 + fixed + 1024;
-        const size_t limit = (size_t)reg_ctas<A, RB>() * reg_threads<A, RB>() / threads;
+        const size_t limit = (size_t)reg_ctas<A, RB>() * kRegThreads<A, RB> / threads;
         return std::min<size_t>((size_t)sm_total / per, std::max<size_t>(1, limit));
     };
     hdr.nbuf = 1;

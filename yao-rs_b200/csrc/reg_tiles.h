@@ -53,10 +53,13 @@ enum RCode : uint32_t {
     RC_PHASE = 32,   // the masked amplitudes times one coefficient
     RC_DIAG = 33,    // the masked amplitudes, each times its own coefficient
     RC_NEG = 34,     // the masked amplitudes times -1
-    RC_CHAN1 = 35,   // + pair: a 1-qubit Kraus sum; sel0: operators, three coefficients each (exact passes)
-    RC_CHAN2 = 37,   // a 2-qubit Kraus sum; sel0: operators, five coefficients each (exact passes)
-    RC_PAULI2 = 38,  // four real 4 x 4 matrices (not in exact passes)
-    RC_REAL2 = 39    // + pair: a real 4 x 4 matrix with a phase a row (sel0 = 0) or a column (1)
+    RC_LAYER = 35,   // amplitudes 1 to 15 times the coefficients from sel0 (~0: no such product), then
+                     // REAL1 ops without pair signs on the positions in sel1: this op and the next ones
+    // density-matrix steps
+    RC_CHAN1 = 36,   // + pair: a 1-qubit Kraus sum; sel0: operators, three coefficients each (exact passes)
+    RC_CHAN2 = 38,   // a 2-qubit Kraus sum; sel0: operators, five coefficients each (exact passes)
+    RC_PAULI2 = 39,  // four real 4 x 4 matrices (not in exact passes)
+    RC_REAL2 = 40    // + pair: a real 4 x 4 matrix with a phase a row (sel0 = 0) or a column (1)
 };
 
 struct RegPass {
