@@ -704,38 +704,33 @@ constexpr int reg_ctas() {
 // the last segment has read it: thread 0 then issues the load of the tile
 // nbuf tiles on, which arrives while this one computes.  Every wait is
 // bounded: one that gives up sets *err and the pass's result is void.
-template <typename A, bool EXACT, int RB, bool DMX>
-__global__ void __launch_bounds__(kRegThreads<A, RB>, reg_ctas<A, RB>())
-    k_reg_tiles(typename A::Amp* __restrict__ st, const RHdr phdr, const uint4* __restrict__ gblob,
-                int* __restrict__ err, const __grid_constant__ CUtensorMap tmap) {
+template <typename A, bool EXACT, int RB, bool DMX, bool TMA>
+__device__ __forceinline__ void r_pass(typename A::Amp* __restrict__ st, const RHdr& hdr, const uint4* __restrict__ gblob,
+                                       int* __restrict__ err, const CUtensorMap* tmap, uint32_t t, uint32_t grid) {
     typedef typename A::Amp Amp;
     constexpr uint32_t AB = sizeof(Amp);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ RHdr hdr;
     __shared__ uint64_t full_bar[4];
     __shared__ uint64_t tbase[4];  // base index of the tile in each buffer
     __shared__ uint32_t place[kRegThreads<A, RB>];
-    if (threadIdx.x == 0) hdr = phdr;
-    __syncthreads();
     unsigned char* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t tile_bytes = AB << hdr.tbits;
-    const uint32_t nbuf = (uint32_t)hdr.nbuf, grid = gridDim.x;
+    const uint32_t nbuf = (uint32_t)hdr.nbuf;
     uint4* blob = (uint4*)(smem + (size_t)nbuf * tile_bytes);
     for (int i = threadIdx.x; i < hdr.blob16; i += blockDim.x) blob[i] = gblob[i];
-    const bool use_tma = hdr.use_tma != 0;
-    uint32_t t = blockIdx.x;
+    const bool use_tma = TMA && hdr.use_tma != 0;
     uint32_t pending = 0;  // thread 0: buffers with a load in flight
     auto load = [&](uint32_t tt, uint32_t b) {
         const uint64_t base = r_base(hdr, tt);
         tbase[b] = base;
         if (!use_tma) return;
         tc::mbar_arrive_expect_tx(&full_bar[b], tile_bytes);
-        tma::load_boxes(&tmap, hdr.tma, base, tc::smem_u32(smem) + b * tile_bytes, tc::smem_u32(&full_bar[b]));
+        tma::load_boxes(tmap, hdr.tma, base, tc::smem_u32(smem) + b * tile_bytes, tc::smem_u32(&full_bar[b]));
         pending |= 1u << b;
     };
     if (threadIdx.x == 0) {
         if (use_tma) {
-            tma::prefetch_map(&tmap);
+            tma::prefetch_map(tmap);
             for (uint32_t q = 0; q < nbuf; q++) tc::mbar_init(&full_bar[q], 1);
         }
         for (uint32_t q = 0; q < nbuf; q++)
@@ -825,6 +820,36 @@ __global__ void __launch_bounds__(kRegThreads<A, RB>, reg_ctas<A, RB>())
                     while (!tc::mbar_try_wait(&full_bar[q], ph) && tma::now_ns() - t0 < tma::kWaitNs) {
                     }
     }
+}
+
+template <typename A, bool EXACT, int RB, bool DMX>
+__global__ void __launch_bounds__(kRegThreads<A, RB>, reg_ctas<A, RB>())
+    k_reg_tiles(typename A::Amp* __restrict__ st, const RHdr phdr, const uint4* __restrict__ gblob,
+                int* __restrict__ err, const __grid_constant__ CUtensorMap tmap) {
+    __shared__ RHdr hdr;
+    if (threadIdx.x == 0) hdr = phdr;
+    __syncthreads();
+    r_pass<A, EXACT, RB, DMX, true>(st, hdr, gblob, err, &tmap, blockIdx.x, gridDim.x);
+}
+
+// One pass of each of many registers: a CTA belongs to the pass owner[CTA].
+struct RBatchPass {
+    RHdr hdr;
+    uint64_t state, blob;   // addresses
+    uint32_t cta0, ctas;    // its CTAs
+};
+static_assert(sizeof(RBatchPass) % 8 == 0, "copied by words");
+
+template <typename A, bool EXACT, int RB>
+__global__ void __launch_bounds__(kRegThreads<A, RB>, reg_ctas<A, RB>())
+    k_reg_batch(const RBatchPass* __restrict__ passes, const uint32_t* __restrict__ owner) {
+    __shared__ RBatchPass pass;
+    const uint32_t* src = (const uint32_t*)(passes + owner[blockIdx.x]);
+    for (uint32_t i = threadIdx.x; i < sizeof(RBatchPass) / 4; i += blockDim.x) ((uint32_t*)&pass)[i] = src[i];
+    __syncthreads();
+    r_pass<A, EXACT, RB, false, false>((typename A::Amp*)(uintptr_t)pass.state, pass.hdr,
+                                       (const uint4*)(uintptr_t)pass.blob, nullptr, nullptr,
+                                       blockIdx.x - pass.cta0, pass.ctas);
 }
 
 // ================================================================= planner
@@ -1650,7 +1675,7 @@ size_t pass_bytes(const RegPass& p, size_t coef_bytes) {
 
 // The plan of prog[0 .. ngates).
 static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int32_t precision, int tbits_max,
-                           bool exact, RegPlan& out, bool dm = false) {
+                           bool exact, RegPlan& out, bool dm = false, uint64_t batch_tiles = 0) {
     out.passes.clear();
     out.blob.clear();
     const size_t amp = precision == YAO_C128 ? 16 : 8, coef_bytes = precision == YAO_C128 ? 16 : 32;
@@ -1663,7 +1688,8 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     // (8 in a 2^12 tile: at most 512 threads), which shortens an op's chain
     // where the time of one CTA is the time of the pass.
     const uint64_t ntiles = 1ull << (nbits - tbits);
-    int rb = ntiles >= 296 ? 4 : (tbits > 11 ? 3 : 2);
+    // (A batch counts the tiles of all its registers, in 2^tbits_max tiles.)
+    int rb = std::max(ntiles, batch_tiles) >= 296 ? 4 : ((batch_tiles ? tbits_max : tbits) > 11 ? 3 : 2);
     bool four = false;
     for (size_t i = 0; i < ngates; i++) four |= four_bits(prog[i]);
     if (four) rb = 4;
@@ -1798,8 +1824,9 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     }
 }
 
-void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out) {
-    reg_plan_range(prog.data(), prog.size(), nbits, precision, tbits, exact, out);
+void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out,
+              uint64_t batch_tiles) {
+    reg_plan_range(prog.data(), prog.size(), nbits, precision, tbits, exact, out, false, batch_tiles);
 }
 
 // ================================================================== launch
@@ -1847,6 +1874,18 @@ static int launch_rb(Ctx* ctx, void* st, int rb, RHdr& hdr, const uint4* blob, s
     return launch_k<A, EXACT, 2, DMX>(ctx, st, hdr, blob, bytes, tmap);
 }
 
+static void pass_header(const RegPass& p, RHdr& h) {
+    memset(&h, 0, sizeof(h));
+    h.tbits = p.tbits;
+    h.nsegs = (int32_t)p.segs.size();
+    h.blob16 = (int32_t)(p.blob_bytes / 16);
+    h.ops16 = (int32_t)(p.segs.size() * sizeof(RSeg) / 16);
+    h.coef16 = h.ops16 + (int32_t)(p.ops.size() * sizeof(ROp) / 16);
+    h.ntiles = (uint32_t)p.ntiles;
+    h.nbuf = 1;
+    memcpy(h.tb, p.tb, sizeof(h.tb));
+}
+
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
                size_t step) {
     if (plan.passes.empty()) return YAO_OK;
@@ -1862,14 +1901,7 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
     for (size_t i = first; i < plan.passes.size() && !s; i += step) {
         const RegPass& p = plan.passes[i];
         RHdr h;
-        memset(&h, 0, sizeof(h));
-        h.tbits = p.tbits;
-        h.nsegs = (int32_t)p.segs.size();
-        h.blob16 = (int32_t)(p.blob_bytes / 16);
-        h.ops16 = (int32_t)(p.segs.size() * sizeof(RSeg) / 16);
-        h.coef16 = h.ops16 + (int32_t)(p.ops.size() * sizeof(ROp) / 16);
-        h.ntiles = (uint32_t)p.ntiles;
-        memcpy(h.tb, p.tb, sizeof(h.tb));
+        pass_header(p, h);
         CUtensorMap tmap;
         memset(&tmap, 0, sizeof(tmap));
         // (one tile: nothing to overlap, and no wait that could give up)
@@ -1893,6 +1925,102 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
     }
     cudaFreeAsync(dblob, ctx->stream);
     return s;
+}
+
+template <typename A, bool EXACT, int RB>
+static int launch_batch_level(Ctx* ctx, const RBatchPass* passes, const uint32_t* owner, unsigned ctas, int tbits,
+                              size_t blob_bytes) {
+    auto kern = k_reg_batch<A, EXACT, RB>;
+    const size_t smem = (sizeof(typename A::Amp) << tbits) + blob_bytes + 1024;
+    YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<ctas, std::max(32u, 1u << (tbits - RB)), smem, ctx->stream>>>(passes, owner);
+    ctx->launches++;
+    YAO_CUDA(cudaGetLastError());
+    return YAO_OK;
+}
+
+// Level after level: one launch runs the next pass of every register that has
+// one left, a CTA a tile (plain loads: the registers sit in L2).  The launch
+// order is the only wait between a register's passes.  Measured on 60 layered
+// circuits, 10 to 18 qubits and 10 to 40 layers, FUSED: 19 launches, 1.6 ms
+// on the device against 2.9 of the block passes; planning, which the rest of
+// the call mostly is, 1.6 ms on 16 host threads.
+int reg_batch(Ctx* ctx, const std::vector<RegPlan>& plans, const std::vector<Reg*>& regs, bool exact) {
+    const int32_t precision = regs[0]->precision;
+    const size_t amp = precision == YAO_C128 ? 16 : 8;
+    constexpr uint32_t kMaxCtas = 2048;  // a register's CTAs in a launch
+    size_t levels = 0, npasses = 0, nowner = 0, nblob = 0;
+    std::vector<size_t> blob_at(plans.size());
+    for (size_t c = 0; c < plans.size(); c++) {
+        levels = std::max(levels, plans[c].passes.size());
+        npasses += plans[c].passes.size();
+        for (const RegPass& p : plans[c].passes) nowner += (size_t)std::min<uint64_t>(p.ntiles, kMaxCtas);
+        blob_at[c] = nblob;
+        nblob += (plans[c].blob.size() + 255) / 256 * 256;
+    }
+    if (npasses == 0) return YAO_OK;
+    const size_t b_pass = (npasses * sizeof(RBatchPass) + 255) / 256 * 256, b_owner = (nowner * 4 + 255) / 256 * 256;
+    const size_t total = nblob + b_pass + b_owner;
+    int st;
+    if ((st = grow_host(&ctx->batch_host, &ctx->batch_host_bytes, total))) return st;
+    if ((st = grow_dev(&ctx->batch_dev, &ctx->batch_dev_bytes, total, ctx->stream))) return st;
+    char* h = (char*)ctx->batch_host;
+    char* d = (char*)ctx->batch_dev;
+    for (size_t c = 0; c < plans.size(); c++) memcpy(h + blob_at[c], plans[c].blob.data(), plans[c].blob.size());
+    RBatchPass* hp = (RBatchPass*)(h + nblob);
+    uint32_t* ho = (uint32_t*)(h + nblob + b_pass);
+    struct Level {
+        size_t owner;
+        uint32_t ctas;
+        int tbits, rb;
+        size_t blob;
+        double bytes;
+    };
+    std::vector<Level> todo;
+    size_t at = 0, own = 0;
+    for (size_t l = 0; l < levels; l++) {
+        Level lv{own, 0, 0, 0, 0, 0.0};
+        for (size_t c = 0; c < plans.size(); c++) {
+            if (l >= plans[c].passes.size()) continue;
+            const RegPass& p = plans[c].passes[l];
+            RBatchPass& b = hp[at];
+            memset(&b, 0, sizeof(b));
+            pass_header(p, b.hdr);
+            b.state = (uint64_t)(uintptr_t)regs[c]->d;
+            b.blob = (uint64_t)(uintptr_t)(d + blob_at[c] + p.blob_off);
+            b.cta0 = lv.ctas;
+            b.ctas = (uint32_t)std::min<uint64_t>(p.ntiles, kMaxCtas);
+            for (uint32_t q = 0; q < b.ctas; q++) ho[own++] = (uint32_t)at;
+            lv.ctas += b.ctas;
+            lv.tbits = std::max(lv.tbits, p.tbits);
+            lv.rb = p.rb;
+            lv.blob = std::max(lv.blob, p.blob_bytes);
+            lv.bytes += (double)p.ntiles * (double)(1ull << p.tbits) * 2.0 * (double)amp;
+            at++;
+        }
+        todo.push_back(lv);
+    }
+    YAO_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, ctx->stream));
+    const RBatchPass* dp = (const RBatchPass*)(d + nblob);
+    const uint32_t* dow = (const uint32_t*)(d + nblob + b_pass);
+    for (const Level& lv : todo) {
+        ProfScope prof(ctx, exact ? "reg_batch_exact" : "reg_batch_fused", lv.bytes);
+        const uint32_t* o = dow + lv.owner;
+        if (precision != YAO_C128)
+            st = lv.rb == 4 ? launch_batch_level<A64, false, 4>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob)
+                            : launch_batch_level<A64, false, 2>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob);
+        else if (exact)
+            st = lv.rb == 4 ? launch_batch_level<A128<true>, true, 4>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob)
+                            : launch_batch_level<A128<true>, true, 2>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob);
+        else
+            st = lv.rb == 4 ? launch_batch_level<A128<false>, false, 4>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob)
+                            : launch_batch_level<A128<false>, false, 2>(ctx, dp, o, lv.ctas, lv.tbits, lv.blob);
+        if (st) break;
+    }
+    // (the tables are free for the next call)
+    const cudaError_t ce = cudaStreamSynchronize(ctx->stream);
+    if (!st && ce != cudaSuccess) return cuda_fail(ce, "batched register passes");
+    return st;
 }
 
 // ==================================================== gate-by-gate programs

@@ -88,10 +88,16 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
 // Passes over 2^tbits-amplitude tiles.  exact: program order, except that
 // permutations (X, SWAP, with controls) may move past gates on other qubits,
 // which changes no bit of the result; otherwise any gate may.
-void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out);
+// batch_tiles: the tiles of all registers that run together (0: this one).
+void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out,
+              uint64_t batch_tiles = 0);
 // Queues passes first, first + step, ... of the plan on the context's stream.
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
                size_t step);
+
+// Runs plan c on register c for all c, and waits.  Every plan has the same
+// number of amplitudes a thread (planned with the same batch_tiles).
+int reg_batch(Ctx* ctx, const std::vector<RegPlan>& plans, const std::vector<Reg*>& regs, bool exact);
 
 // Fusion into blocks of at most 2 qubits (sv_tiles.cu); density-matrix steps
 // on two qubits are kept.

@@ -211,6 +211,9 @@ int plan_info(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
               int32_t tbits, int32_t rb, int64_t info[7]);
 // Many circuits (one register each, same context and precision) in one
 // persistent, graph-captured launch (TILED or FUSED forms).
+// The batch tables of a context, grown to at least `bytes`.
+int grow_dev(void** p, size_t* have, size_t bytes, cudaStream_t s);
+int grow_host(void** p, size_t* have, size_t bytes);
 int launch_batch(Ctx* ctx, const std::vector<const std::vector<LGate>*>& progs, const std::vector<Reg*>& regs,
                  int32_t mode, int32_t k);
 
