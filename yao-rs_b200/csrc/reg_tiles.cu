@@ -1831,34 +1831,45 @@ void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
 
 // ================================================================== launch
 
+int kernel_fit(Ctx* ctx, const void* kernel, KernelFit* out, bool all) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, KernelFit> known;
+    std::lock_guard<std::mutex> g(mu);
+    KernelFit& f = known[{ctx->device, kernel}];
+    if (!f.limit) {
+        int v = 0;
+        cudaFuncAttributes fa;
+        YAO_CUDA(cudaDeviceGetAttribute(&f.total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+        YAO_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+        YAO_CUDA(cudaFuncGetAttributes(&fa, kernel));
+        f.fixed = (int)fa.sharedSizeBytes;
+        YAO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v - f.fixed));
+        if (all)
+            YAO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        f.limit = v - f.fixed;
+    }
+    *out = f;
+    return YAO_OK;
+}
+
 template <typename A, bool EXACT, int RB, bool DMX>
 static int launch_k(Ctx* ctx, void* st, RHdr& hdr, const uint4* blob, size_t blob_bytes, const CUtensorMap& tmap) {
     auto kern = k_reg_tiles<A, EXACT, RB, DMX>;
-    static int optin = 0, sm_total = 0, fixed = 0;
-    if (!optin) {
-        int dev = 0, v = 0;
-        YAO_CUDA(cudaGetDevice(&dev));
-        YAO_CUDA(cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-        cudaFuncAttributes fa;
-        YAO_CUDA(cudaFuncGetAttributes(&fa, kern));
-        fixed = (int)fa.sharedSizeBytes;
-        YAO_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, v - fixed));
-        YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-        optin = v;
-    }
+    KernelFit fit;
+    int sf = kernel_fit(ctx, (const void*)kern, &fit, true);
+    if (sf) return sf;
     const size_t tile = sizeof(typename A::Amp) << hdr.tbits;
     const unsigned threads = std::max(32u, 1u << (hdr.tbits - RB));
     // as many CTAs as the registers allow, then as many tile buffers as fit
     auto ctas = [&](int nbuf) {
-        const size_t per = (size_t)nbuf * tile + blob_bytes + 1024 + fixed + 1024;
+        const size_t per = (size_t)nbuf * tile + blob_bytes + 1024 + fit.fixed + 1024;
         const size_t limit = (size_t)reg_ctas<A, RB>() * kRegThreads<A, RB> / threads;
-        return std::min<size_t>((size_t)sm_total / per, std::max<size_t>(1, limit));
+        return std::min<size_t>((size_t)fit.total / per, std::max<size_t>(1, limit));
     };
     hdr.nbuf = 1;
     while (hdr.use_tma && hdr.nbuf < 4 && ctas(hdr.nbuf + 1) == ctas(hdr.nbuf)) hdr.nbuf++;
     const size_t smem = (size_t)hdr.nbuf * tile + blob_bytes + 1024;
-    if (smem + fixed > (size_t)optin) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
+    if (smem > (size_t)fit.limit) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
     int per_sm = 0;
     YAO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)threads, smem));
     if (per_sm < 1) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
@@ -1932,7 +1943,10 @@ static int launch_batch_level(Ctx* ctx, const RBatchPass* passes, const uint32_t
                               size_t blob_bytes) {
     auto kern = k_reg_batch<A, EXACT, RB>;
     const size_t smem = (sizeof(typename A::Amp) << tbits) + blob_bytes + 1024;
-    YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KernelFit fit;
+    int s = kernel_fit(ctx, (const void*)kern, &fit);
+    if (s) return s;
+    if (smem > (size_t)fit.limit) return fail(YAO_ERR_UNSUPPORTED, "register pass does not fit an SM");
     kern<<<ctas, std::max(32u, 1u << (tbits - RB)), smem, ctx->stream>>>(passes, owner);
     ctx->launches++;
     YAO_CUDA(cudaGetLastError());

@@ -376,16 +376,9 @@ static int expect_tiles(Ctx* ctx, const Reg* r, const std::vector<EPass>& passes
         ls.push_back(l);
     }
     const size_t tile = sizeof(V) << tbits;
-    static int optin = 0, fixed = 0;
-    if (!optin) {
-        cudaFuncAttributes fa;
-        YAO_CUDA(cudaFuncGetAttributes(&fa, kern));
-        fixed = (int)fa.sharedSizeBytes;
-        int v = 0;
-        YAO_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-        YAO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, v - fixed));
-        optin = v;
-    }
+    KernelFit fit;
+    int sf = kernel_fit(ctx, (const void*)kern, &fit);
+    if (sf) return sf;
     // two tile buffers a CTA (the next tile arrives while this one is summed)
     int nbuf = ntiles > 1 ? 2 : 1;
     size_t smem = (size_t)nbuf * tile + most * 16 + 1024;

@@ -866,12 +866,10 @@ struct SweepRun {
         YAO_CUDA(cudaMemcpyAsync(runs, p->runs.data(), p->runs.size() * sizeof(SRunDev), cudaMemcpyHostToDevice, s));
         YAO_CUDA(cudaMemcpyAsync(place, pl.data(), pl.size() * sizeof(SPlace), cudaMemcpyHostToDevice, s));
         YAO_CUDA(cudaMemcpyAsync(params, host_params, nsets * p->np * 8, cudaMemcpyHostToDevice, s));
-        static bool attr = false;
-        if (!attr) {
-            YAO_CUDA(cudaFuncSetAttribute(k_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            YAO_CUDA(cudaFuncSetAttribute(k_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            attr = true;
-        }
+        KernelFit fit;
+        int sf = kernel_fit(ctx, (const void*)k_sweep<true>, &fit);
+        if (!sf) sf = kernel_fit(ctx, (const void*)k_sweep<false>, &fit);
+        if (sf) return sf;
         return YAO_OK;
     }
 

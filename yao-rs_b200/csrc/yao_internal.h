@@ -211,6 +211,16 @@ int plan_info(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision,
               int32_t tbits, int32_t rb, int64_t info[7]);
 // Many circuits (one register each, same context and precision) in one
 // persistent, graph-captured launch (TILED or FUSED forms).
+// Shared memory of a device and of a kernel: `limit` dynamic bytes a CTA at
+// most (the kernel may use them from then on), `total` bytes an SM, `fixed`
+// static bytes.  Set once a device and kernel; safe from several threads.
+// all: the whole carveout for shared memory (the sweep and batch kernels,
+// which read global memory directly, lose L1 by it: a gradient at n = 22
+// took 5.3 ms instead of 4.9).
+struct KernelFit {
+    int limit = 0, total = 0, fixed = 0;
+};
+int kernel_fit(Ctx* ctx, const void* kernel, KernelFit* out, bool all = false);
 // The batch tables of a context, grown to at least `bytes`.
 int grow_dev(void** p, size_t* have, size_t bytes, cudaStream_t s);
 int grow_host(void** p, size_t* have, size_t bytes);
