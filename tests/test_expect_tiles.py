@@ -46,3 +46,23 @@ def test_expectation_over_tiles(n):
 def test_empty_operator():
     r = Y.ArrayReg.zero_state(5)
     assert Y.expect_arrayreg(r, Y.OperatorPolynomial.zero()) == 0
+
+
+# 20 and 22 qubits: one to four tiles a CTA and more, so that buffers are
+# loaded again and the barriers' phases turn; 23: the same for complex64
+@pytest.mark.gpu
+@pytest.mark.parametrize("tma", ["1", "0"])
+@pytest.mark.parametrize("n", [20, 22, 23])
+def test_several_tiles_a_cta(n, tma, monkeypatch):
+    monkeypatch.setenv("YAO_TMA", tma)
+    rng = np.random.default_rng(n)
+    psi = random_state(rng, n)
+    r = Y.ArrayReg.from_vec(n, psi)
+    single = r.to_precision(Y.C64)
+    op = strings(rng, n, PAULI, False)
+    op = Y.OperatorPolynomial(op.coeffs()[:8], op.opstrings()[:8])
+    # FP64 sums of at most 2^23 products whose magnitudes add up to 1 a string
+    tol = 1e-13 * sum(abs(c) for c in op.coeffs())
+    for reg in (r, single):
+        v = reg.state_vec().astype(np.complex128)
+        assert abs(Y.expect_arrayreg(reg, op) - O.expect_arrayreg(v, n, op)) < tol
