@@ -297,7 +297,7 @@ int yao_expect_dm(const yao_dm* d, const yao_term* terms, size_t nterms, double 
  * reverse sweep runs over shared-memory tiles of psi and lambda (circuits
  * with gates on more than 2 qubits, or YAO_ADJ_TILES=0: one step per gate). */
 /* Circuits whose parameters all sit in uncontrolled 1-qubit gates (and whose
- * other gates are 1-qubit gates, controlled X, SWAP or signs such as CZ) take
+ * other gates are unitary 1-qubit gates, controlled X, SWAP or signs such as CZ) take
  * the register sweep (sums over each run of 1-qubit gates); the others, and
  * runs with a YAO_ADJ_* switch set, the tiled or per-gate one. */
 /* The plan of expect_grad's tiled reverse sweep for c, computed on the host

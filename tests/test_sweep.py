@@ -95,3 +95,44 @@ def test_long_runs_of_ops_split_passes():
     value, grad = O.expect_grad(h, c, psi)
     v, g = Y.expect_grad(h, c, Y.ArrayReg.from_vec(n, psi))
     assert abs(v - value) < 1e-12 and np.max(np.abs(np.array(g) - np.array(grad))) < 1e-12
+
+
+def projected(n, m):
+    """A constant matrix that is not unitary at the end of a run, and before
+    and after other runs' ends; parameters on both sides of it."""
+    p = Gate.Custom(np.asarray(m, dtype=complex))
+    els = [Y.put([q], Gate.Ry(0.3 + 0.1 * q)) for q in range(n)] + [Y.put([1], Gate.Rx(0.4)), Y.put([0], p)]
+    els += [Y.control([0], [1], Gate.X), Y.put([1], Gate.Ry(0.5)), Y.put([1], p), Y.put([1], Gate.Rz(0.2))]
+    els += [Y.control([1], [2], Gate.X), Y.put([2], p), Y.put([2], Gate.Ry(-0.7)), Y.control([2], [0], Gate.Z)]
+    return Y.Circuit.qubits(n, els)
+
+
+# zero rows and columns
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 12])
+@pytest.mark.parametrize("m", [[[0, 0], [0, 1]], [[1, 0], [0, 0]], [[0, 1], [0, 0]], [[0, 0], [1, 0]], [[0, 0], [0, 0]]])
+def test_constants_that_are_not_unitary(n, m):
+    rng = np.random.default_rng(n)
+    c, h, psi = projected(n, m), hamiltonian(n), random_state(rng, n)
+    reg = Y.ArrayReg.from_vec(n, psi)
+    value, grad = O.expect_grad(h, c, psi)
+    v, g = Y.expect_grad(h, c, reg)
+    vs, gs = Y.expect_grad_batch(h, c, np.array([c.parameters()] * 2), reg)
+    # some tens of gates of 1.1e-16 each on terms of magnitude 1.7 n
+    for got_v, got_g in ((v, g), (vs[0], gs[0]), (vs[1], gs[1])):
+        assert abs(got_v - value) < 1e-12 and np.max(np.abs(np.array(got_g) - np.array(grad))) < 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [21, 22])
+def test_several_tiles_a_unit(n, monkeypatch):
+    """More tiles than units of work: against one step a gate."""
+    rng = np.random.default_rng(n)
+    c, h = ansatz(rng, n, 1, 1), hamiltonian(n)
+    reg = Y.ArrayReg.zero_state(n)
+    v, g = Y.expect_grad(h, c, reg)
+    vs, gs = Y.expect_grad_batch(h, c, np.array([c.parameters()] * 2), reg)
+    monkeypatch.setenv("YAO_ADJ_TILES", "0")
+    value, grad = Y.expect_grad(h, c, reg)
+    for got_v, got_g in ((v, g), (vs[0], gs[0]), (vs[1], gs[1])):
+        assert abs(got_v - value) < 1e-12 and np.max(np.abs(np.array(got_g) - np.array(grad))) < 1e-12

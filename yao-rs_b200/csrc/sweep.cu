@@ -480,6 +480,19 @@ static bool real_matrix(const SFactor& f) {
     return f.m[0].y == 0 && f.m[1].y == 0 && f.m[2].y == 0 && f.m[3].y == 0;
 }
 
+// U^dagger U = 1 to the rounding of the entries.  The steps of a sweep change
+// places on disjoint qubits: a dot of lambda and psi stays the same under a
+// matrix on another qubit when that matrix is unitary, else it does not.
+static bool unitary(const SFactor& f) {
+    const double2 *m = f.m;
+    auto sq = [](double2 z) { return z.x * z.x + z.y * z.y; };
+    const double re = m[0].x * m[1].x + m[0].y * m[1].y + m[2].x * m[3].x + m[2].y * m[3].y,
+                 im = m[0].x * m[1].y - m[0].y * m[1].x + m[2].x * m[3].y - m[2].y * m[3].x;
+    const double eps = 1e-14;
+    return std::fabs(sq(m[0]) + sq(m[2]) - 1.0) < eps && std::fabs(sq(m[1]) + sq(m[3]) - 1.0) < eps &&
+           std::fabs(re) < eps && std::fabs(im) < eps;
+}
+
 // The passes of `items` in the given order.  A step is taken past skipped
 // ones that share no qubit with it: the sums and states change by rounding
 // only.  back: an X joins the run on its target that follows it.
@@ -719,6 +732,7 @@ SweepPlan* sweep_plan_new(const Circuit* c, uint32_t n) {
                 } else {
                     for (int q = 0; q < 4; q++) f.m[q] = make_double2(l.m[q].re, l.m[q].im);
                 }
+                if (!unitary(f)) return nullptr;
                 pend[l.tb[0]].push_back(f);
                 continue;
             }

@@ -11,8 +11,8 @@ namespace yao {
 
 struct SweepPlan;
 // The plan of a circuit on n qubits, or null when it does not apply: every
-// parametric gate is an uncontrolled 1-qubit gate, and the others are 1-qubit
-// gates, (controlled) X, SWAP and sign gates such as CZ.
+// parametric gate is an uncontrolled 1-qubit gate, and the others are unitary
+// 1-qubit gates, (controlled) X, SWAP and sign gates such as CZ.
 SweepPlan* sweep_plan_new(const Circuit* c, uint32_t n);
 void sweep_plan_free(SweepPlan* p);
 
