@@ -295,7 +295,8 @@ int yao_expect_dm(const yao_dm* d, const yao_term* terms, size_t nterms, double 
  * Circuit::parameters() order; ngrad must equal num_params.  The forward
  * state is computed in FUSED form (within ~1e-15 of the PLAIN state) and the
  * reverse sweep runs over shared-memory tiles of psi and lambda (circuits
- * with gates on more than 2 qubits, or YAO_ADJ_TILES=0: one step per gate). */
+ * with gates on more than 2 qubits or gates that are not unitary, or
+ * YAO_ADJ_TILES=0: one step per gate). */
 /* Circuits whose parameters all sit in uncontrolled 1-qubit gates (and whose
  * other gates are unitary 1-qubit gates, controlled X, SWAP or signs such as CZ) take
  * the register sweep (sums over each run of 1-qubit gates); the others, and

@@ -107,10 +107,11 @@ def projected(n, m):
     return Y.Circuit.qubits(n, els)
 
 
-# zero rows and columns
+# zero rows and columns; a shear and a damping, which steps on other qubits must not pass
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [3, 12])
-@pytest.mark.parametrize("m", [[[0, 0], [0, 1]], [[1, 0], [0, 0]], [[0, 1], [0, 0]], [[0, 0], [1, 0]], [[0, 0], [0, 0]]])
+@pytest.mark.parametrize("m", [[[0, 0], [0, 1]], [[1, 0], [0, 0]], [[0, 1], [0, 0]], [[0, 0], [1, 0]], [[0, 0], [0, 0]],
+                               [[1, 0.25], [0, 1]], [[1, 0], [0, 0.5j]]])
 def test_constants_that_are_not_unitary(n, m):
     rng = np.random.default_rng(n)
     c, h, psi = projected(n, m), hamiltonian(n), random_state(rng, n)

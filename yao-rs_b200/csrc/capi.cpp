@@ -1340,8 +1340,11 @@ int yao_expect_grad(const yao_term* terms, size_t nterms, const yao_circuit* cc,
     const char* forms[] = {"YAO_ADJ_TILES", "YAO_ADJ_REORDER", "YAO_ADJ_SEGMENTS", "YAO_ADJ_UPAIR", "YAO_ADJ_XFOLD", "YAO_ADJ_FUSE"};
     bool form_set = false;
     for (const char* f : forms) form_set |= getenv(f) != nullptr;
-    if (np && !form_set) plan.s = sweep_plan_new(c, psi0->nbits);
-    if (np && !plan.s && !(at && at[0] == '0')) {
+    // (both reorder and fold steps, which leaves the dots alone only where the
+    // gates are unitary; else one step a gate, in the circuit's order)
+    const bool unitary = np && circuit_is_unitary(c);
+    if (unitary && !form_set) plan.s = sweep_plan_new(c, psi0->nbits);
+    if (unitary && !plan.s && !(at && at[0] == '0')) {
         int pst = YAO_OK;
         plan.p = adjoint_plan_new(c, psi0->nbits, YAO_C128, np, &pst);
         if (!plan.p && pst != YAO_ERR_UNSUPPORTED) return pst;
