@@ -1,0 +1,62 @@
+// The planner of the register passes on the host, linked against the library:
+//   plans norm N LAYERS    log of the factor by which the split program's
+//                          1-qubit matrices change the squared norm, minus
+//                          that of the gates it was made from (layers of Rx,
+//                          Ry, Rz on N qubits and a CNOT brickwork)
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+
+#include "reg_tiles.h"
+
+using namespace yao;
+
+static void gate(std::vector<LGate>& prog, uint32_t n, int32_t type, uint32_t target, double angle, int control = -1) {
+    GateElem g;
+    g.type = type;
+    g.targets = {target};
+    g.params[0] = angle;
+    if (control >= 0) {
+        g.ctrls = {(uint32_t)control};
+        g.cfgs = {1};
+    }
+    lower_gate(g, n, 0, false, prog);
+}
+
+static std::vector<LGate> layered(uint32_t n, int layers) {
+    std::mt19937_64 r(1);
+    std::uniform_real_distribution<double> angle(0.0, 6.283185307179586);
+    std::vector<LGate> prog;
+    for (int l = 0; l < layers; l++) {
+        for (uint32_t q = 0; q < n; q++)
+            for (int32_t type : {YAO_GATE_RX, YAO_GATE_RY, YAO_GATE_RZ}) gate(prog, n, type, q, angle(r));
+        for (uint32_t a = l % 2; a + 1 < n; a += 2) gate(prog, n, YAO_GATE_X, a + 1, 0.0, (int)a);
+    }
+    return prog;
+}
+
+// sum over the uncontrolled matrices of the log of their rows' mean squared length
+static long double log_norm(const std::vector<LGate>& prog) {
+    long double sum = 0.0L;
+    for (const LGate& g : prog) {
+        if (g.nc || g.m.empty()) continue;
+        long double t = 0.0L;
+        for (const Cx& c : g.m) t += (long double)c.re * c.re + (long double)c.im * c.im;
+        sum += std::log(t / (1 << g.k));
+    }
+    return sum;
+}
+
+int main(int argc, char** argv) {
+    if (argc == 4 && !strcmp(argv[1], "norm")) {
+        const uint32_t n = (uint32_t)atoi(argv[2]);
+        const std::vector<LGate> prog = layered(n, atoi(argv[3]));
+        std::vector<LGate> split;
+        split_single_qubit(prog, n, split);
+        printf("%zu %.6Le\n", split.size(), log_norm(split) - log_norm(prog));
+        return 0;
+    }
+    return 1;
+}

@@ -903,47 +903,91 @@ struct Scan {
 static Cx cmul(Cx a, Cx b) { return Cx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 static Cx conj(Cx a) { return Cx{a.re, -a.im}; }
 static bool is(Cx c, double re) { return c.re == re && c.im == 0.0; }
+
+// Extended precision (64 bits of mantissa) on the host: products of gates,
+// moduli and phases are taken from it with one rounding, and squares of any
+// double fit.
+struct CxL {
+    long double re, im;
+    CxL() : re(0.0L), im(0.0L) {}
+    CxL(long double r, long double i) : re(r), im(i) {}
+    CxL(Cx a) : re(a.re), im(a.im) {}
+    Cx round() const { return Cx{(double)re, (double)im}; }
+};
+static CxL operator+(CxL a, CxL b) { return CxL(a.re + b.re, a.im + b.im); }
+static CxL operator*(CxL a, CxL b) { return CxL(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re); }
+static CxL operator*(long double x, CxL a) { return CxL(x * a.re, x * a.im); }
+static CxL conj(CxL a) { return CxL(a.re, -a.im); }
+static bool is(CxL c, long double re) { return c.re == re && c.im == 0.0L; }
+static long double norm2(CxL a) { return a.re * a.re + a.im * a.im; }
 // a / |a|
-static Cx unit(Cx a) {
-    const double r = std::hypot(a.re, a.im);
-    return Cx{a.re / r, a.im / r};
-}
+static CxL unit(CxL a) { return 1.0L / std::sqrt(norm2(a)) * a; }
 
 namespace {
 
-// What waits to be applied on one qubit: nothing, a diagonal or a matrix.
+constexpr long double kRoot2 = 1.41421356237309504880168872420969808L;
+
+// What waits to be applied on one qubit: nothing, a diagonal or a matrix
+// (the product of `factors` matrices, a unitary one times the root of 2^twos
+// where the gates are unitary).
 struct Pend {
     bool on = false;
-    Cx m[4];
-    bool diag() const { return is(m[1], 0.0) && is(m[2], 0.0); }
+    int factors = 0, twos = 0;
+    CxL m[4];
+    bool diag() const { return is(m[1], 0.0L) && is(m[2], 0.0L); }
     void mul(const Cx* u) {  // m <- u m
         if (!on) {
             std::copy(u, u + 4, m);
             on = true;
+            factors = 1;
+            twos = 0;
             return;
         }
-        Cx r[4];
+        const CxL x[4] = {m[0], m[1], m[2], m[3]};
+        factors++;
+        if (is(u[1], 0.0) && is(u[2], 0.0)) {
+            for (int j = 0; j < 4; j++) m[j] = CxL(u[j & 2 ? 3 : 0]) * x[j];
+            return;
+        }
+        if (u[0].im == 0.0 && u[1].im == 0.0 && u[2].im == 0.0 && u[3].im == 0.0) {
+            for (int i = 0; i < 2; i++)
+                for (int j = 0; j < 2; j++) m[2 * i + j] = (long double)u[2 * i].re * x[j] + (long double)u[2 * i + 1].re * x[2 + j];
+            return;
+        }
         for (int i = 0; i < 2; i++)
-            for (int j = 0; j < 2; j++) {
-                const Cx x = cmul(u[2 * i], m[j]), y = cmul(u[2 * i + 1], m[2 + j]);
-                r[2 * i + j] = Cx{x.re + y.re, x.im + y.im};
-            }
-        std::copy(r, r + 4, m);
+            for (int j = 0; j < 2; j++) m[2 * i + j] = CxL(u[2 * i]) * x[j] + CxL(u[2 * i + 1]) * x[2 + j];
     }
+    // m <- by H m, where H is a Hadamard without its factor: with by = 1
+    // before a CZ and a half after it the two make 1 exactly (the root of a
+    // half rounded, squared and doubled is 1 + 2.2e-16)
+    void hadamard(long double by) {
+        if (!on) {
+            m[0] = m[3] = CxL(1.0L, 0.0L);
+            m[1] = m[2] = CxL(0.0L, 0.0L);
+            factors = twos = 0;
+            on = true;
+        }
+        for (int j = 0; j < 2; j++) {
+            const CxL x = m[j], y = m[2 + j];
+            m[j] = by * (x + y);
+            m[2 + j] = by * (x + -1.0L * y);
+        }
+        factors++;
+        twos += by == 1.0L ? 1 : -1;
+    }
+    // To the rounding of the factors (a number within 1e-13 of 1 may multiply it).
     bool unitary() const {
-        const double eps = 1e-13;
-        const double a = m[0].re * m[0].re + m[0].im * m[0].im, b = m[1].re * m[1].re + m[1].im * m[1].im,
-                     c = m[2].re * m[2].re + m[2].im * m[2].im, d = m[3].re * m[3].re + m[3].im * m[3].im;
-        const Cx x = cmul(conj(m[0]), m[1]), y = cmul(conj(m[2]), m[3]);
-        return std::fabs(a + c - 1.0) < eps && std::fabs(b + d - 1.0) < eps && std::fabs(x.re + y.re) < eps &&
-               std::fabs(x.im + y.im) < eps;
+        const long double two = std::ldexp(1.0L, twos), eps = 1e-15L * (factors + 1) * two;
+        const long double a = norm2(m[0]) + norm2(m[2]), b = norm2(m[1]) + norm2(m[3]);
+        const CxL x = conj(m[0]) * m[1] + conj(m[2]) * m[3];
+        return std::fabs(a - two) < 1e-13L * two && std::fabs(a - b) < eps && std::fabs(x.re) < eps && std::fabs(x.im) < eps;
     }
 };
 
 struct Splitter {
     std::vector<Pend> pend;
     std::vector<LGate>& out;
-    Cx phase{1.0, 0.0};  // of the whole state
+    CxL scale{1.0L, 0.0L};  // of the whole state
     Splitter(uint32_t n, std::vector<LGate>& o) : pend(n), out(o) {}
 
     void emit1(int b, int cls, std::vector<Cx> m) {
@@ -955,56 +999,71 @@ struct Splitter {
         out.push_back(std::move(g));
     }
     // Applies what waits on bit b, except a diagonal when `keep_diag`
-    // (what comes next commutes with it).
+    // (what comes next commutes with it).  Matrices are rounded once, here;
+    // the state's scale takes what the rounded ones are off in norm, so that
+    // a long circuit's norm strays by the roundings of its amplitudes alone.
     void flush(int b, bool keep_diag) {
         Pend& p = pend[b];
         if (!p.on) return;
-        const Cx *m = p.m, one{1.0, 0.0}, zero{0.0, 0.0};
+        const CxL *m = p.m, one(1.0L, 0.0L), zero(0.0L, 0.0L);
         if (!p.diag()) {
-            if (is(m[0], 0.0) && is(m[3], 0.0) && is(m[1], 1.0) && is(m[2], 1.0)) {
+            if (is(m[0], 0.0L) && is(m[3], 0.0L) && is(m[1], 1.0L) && is(m[2], 1.0L)) {
                 emit1(b, GC_X, {});
                 p.on = false;
                 return;
             }
             if (!p.unitary()) {
-                emit1(b, GC_DENSE, std::vector<Cx>(m, m + 4));
+                emit1(b, GC_DENSE, {m[0].round(), m[1].round(), m[2].round(), m[3].round()});
                 p.on = false;
                 return;
             }
-            // e^{i alpha} diag(1, f) [[c, -s], [s, c]] diag(1, l): the larger
-            // of a column's entries fixes its phase
-            const double c = std::hypot(m[0].re, m[0].im), s = std::hypot(m[2].re, m[2].im);
-            Cx al, f, l;
+            // r e^{i alpha} diag(1, f) [[c, -s], [s, c]] diag(1, l): the larger
+            // of a column's entries fixes its phase.  r and the columns' norms
+            // are the root of 2^twos to 1e-13, so series give their roots.
+            const long double root = p.twos == 0 ? 1.0L : p.twos > 0 ? kRoot2 : 0.5L * kRoot2, two = root * root;
+            const long double n0 = norm2(m[0]), n2 = norm2(m[2]), off = (n0 + n2) / two - 1.0L;
+            const long double i0 = n0 > 0.0L ? 1.0L / std::sqrt(n0) : 0.0L, i2 = n2 > 0.0L ? 1.0L / std::sqrt(n2) : 0.0L;
+            const long double col = (1.0L - 0.5L * off) / root, c = n0 * i0 * col, s = n2 * i2 * col;
+            CxL al = one, f = one, l = one;
             if (c >= s) {
-                al = unit(m[0]);
-                const Cx fl = cmul(unit(m[3]), conj(al));  // f l
-                f = s > 0.0 ? cmul(unit(m[2]), conj(al)) : fl;
-                l = cmul(fl, conj(f));
+                al = i0 * m[0];
+                const CxL fl = i0 * (m[3] * conj(al));  // f l
+                f = s > 0.0L ? i2 * (m[2] * conj(al)) : fl;
+                l = fl * conj(f);
             } else {
-                const Cx g = unit(m[2]);                               // alpha f
-                const Cx h = unit(Cx{-m[1].re, -m[1].im});             // alpha l
-                al = c > 0.0 ? unit(m[0]) : g;
-                f = cmul(g, conj(al));
-                l = cmul(h, conj(al));
+                const CxL g = i2 * m[2];       // alpha f
+                const CxL h = -i2 * m[1];      // alpha l
+                al = c > 0.0L ? i0 * m[0] : g;
+                f = g * conj(al);
+                l = h * conj(al);
             }
-            phase = cmul(phase, al);
             // what is left of the diagonal after it waits for the next
             // rotation of this bit, else it joins the matrix
-            const Cx g = keep_diag ? one : f;
-            emit1(b, GC_DENSE, {Cx{c, 0.0}, Cx{-s * l.re, -s * l.im}, Cx{s * g.re, s * g.im}, cmul(cmul(g, l), Cx{c, 0.0})});
+            const CxL g = keep_diag ? one : f;
+            const Cx e[4] = {CxL(c, 0.0L).round(), (-s * l).round(), (s * g).round(), (c * (g * l)).round()};
+            const CxL left = keep_diag ? CxL(f.round()) : one;
+            const long double have = (norm2(e[0]) + norm2(e[1]) + norm2(e[2]) + norm2(e[3])) * (1.0L + norm2(left));
+            const long double want = (n0 + n2 + norm2(m[1]) + norm2(m[3])) * 2.0L / two;
+            scale = scale * (root * (1.0L + 0.5L * (want / have - 1.0L)) * al);
+            emit1(b, GC_DENSE, std::vector<Cx>(e, e + 4));
             p.m[0] = one;
             p.m[1] = p.m[2] = zero;
-            p.m[3] = f;
-            p.on = keep_diag && !is(f, 1.0);
+            p.m[3] = left;
+            p.on = !is(left, 1.0L);
+            p.factors = 1;
+            p.twos = 0;
             return;
         }
         if (keep_diag || !p.on) return;
+        Cx d[2] = {m[0].round(), m[3].round()};
         if (p.unitary()) {
-            phase = cmul(phase, p.m[0]);
-            p.m[3] = cmul(p.m[3], conj(p.m[0]));
-            p.m[0] = one;
+            const CxL a = m[0];
+            d[0] = Cx{1.0, 0.0};
+            d[1] = ((1.0L / norm2(a)) * (conj(a) * m[3])).round();
+            const long double ratio = (norm2(a) + norm2(m[3])) / ((1.0L + norm2(d[1])) * norm2(a));
+            scale = scale * ((1.0L + 0.5L * (ratio - 1.0L)) * a);
         }
-        if (!(is(p.m[0], 1.0) && is(p.m[3], 1.0))) emit1(b, GC_DIAG, {p.m[0], p.m[3]});
+        if (!(is(d[0], 1.0) && is(d[1], 1.0))) emit1(b, GC_DIAG, {d[0], d[1]});
         p.on = false;
     }
 };
@@ -1028,8 +1087,6 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
         for (int q = 0; q < g.k; q++) next[g.tb[q]] = 0;
         for (int q = 0; q < g.nc; q++) next[g.cb[q]] = 0;
     }
-    const double h = std::sqrt(0.5);
-    const Cx had[4] = {{h, 0.0}, {h, 0.0}, {h, 0.0}, {-h, 0.0}};
     for (size_t i = 0; i < prog.size(); i++) {
         const LGate& g = prog[i];
         if (single(g)) {
@@ -1046,7 +1103,7 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
         }
         const int t = g.tb[0];
         if (g.cls == GC_X && g.nc == 1 && rot_next[i] && sp.pend[t].on && !sp.pend[t].diag() && sp.pend[t].unitary()) {
-            sp.pend[t].mul(had);
+            sp.pend[t].hadamard(1.0L);
             sp.flush(t, true);
             sp.flush(g.cb[0], true);
             LGate z;
@@ -1057,7 +1114,7 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
             z.m.assign(4, Cx{1.0, 0.0});
             z.m[g.cv[0] ? 3 : (t == z.tb[0] ? 1 : 2)] = Cx{-1.0, 0.0};
             out.push_back(std::move(z));
-            sp.pend[t].mul(had);
+            sp.pend[t].hadamard(0.5L);
             continue;
         }
         for (int q = 0; q < g.k; q++) sp.flush(g.tb[q], g.cls == GC_DIAG);
@@ -1065,15 +1122,16 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
         out.push_back(g);
     }
     for (uint32_t b = 0; b < nbits; b++) sp.flush((int)b, false);
-    // the state's phase joins the last phase gate, else the last matrix
-    if (is(sp.phase, 1.0)) return;
+    // the state's scale joins the last phase gate, else the last matrix
+    const Cx scale = sp.scale.round();
+    if (is(scale, 1.0)) return;
     for (int cls : {(int)GC_DIAG, (int)GC_DENSE})
         for (size_t i = out.size(); i-- > 0;)
             if (out[i].cls == cls && out[i].nc == 0) {
-                for (Cx& x : out[i].m) x = cmul(x, sp.phase);
+                for (Cx& x : out[i].m) x = cmul(x, scale);
                 return;
             }
-    sp.emit1(0, GC_DIAG, {sp.phase, sp.phase});
+    sp.emit1(0, GC_DIAG, {scale, scale});
 }
 
 // Description of a pass kept below this, so that three CTAs of 2^11
@@ -1388,26 +1446,28 @@ struct PassBuilder {
                 }
             return left == 0;
         };
-        // the second column's phase; false: it has none
-        auto phase = [&](const ROp& op, Cx& u, Cx (&m)[2]) {
+        // the second column's phase (its entries are rounded, and no further
+        // from the phase than that); false: it has none
+        auto phase = [&](const ROp& op, CxL& u, Cx (&m)[2]) {
             const Cx* c = &p->coef[op.coef];
             m[0] = c[0];
             m[1] = c[1];
-            u = Cx{1.0, 0.0};
+            u = CxL(1.0L, 0.0L);
             if (code(op) == RC_REAL1) return true;
-            const Cx b = c[1], d = c[2];
-            const double nb = std::hypot(b.re, b.im), nd = std::hypot(d.re, d.im), norm = std::max(nb, nd);
-            u = nb > nd ? unit(b) : unit(d);
-            const Cx x = cmul(b, conj(u)), y = cmul(d, conj(u));
-            m[0] = Cx{c[0].re, x.re};
-            m[1] = Cx{c[0].im, y.re};
-            return std::fabs(x.im) <= 1e-15 * norm && std::fabs(y.im) <= 1e-15 * norm;
+            const CxL b = c[1], d = c[2];
+            const long double nb = norm2(b), nd = norm2(d), eps = 4e-16L * std::sqrt(std::max(nb, nd));
+            u = unit(nb > nd ? b : d);
+            const CxL x = b * conj(u), y = d * conj(u);
+            m[0] = Cx{c[0].re, (double)x.re};
+            m[1] = Cx{c[0].im, (double)y.re};
+            return std::fabs(x.im) <= eps && std::fabs(y.im) <= eps;
         };
         std::vector<ROp> list(p->ops.begin() + (long)begin, p->ops.end()), out;
         while (!list.empty()) {
             int at[4] = {-1, -1, -1, -1};
             uint32_t held = 0, read = 0, have = 0, r[4];  // positions of passed ops; those they read; the group's
-            Cx u[4], m[4][2];
+            CxL u[4];
+            Cx m[4][2];
             for (size_t k = 0; k < list.size() && k < 16 && have != 15u; k++) {
                 const ROp& op = list[k];
                 if (code(op) != RC_RCOL1 && code(op) != RC_REAL1) break;
@@ -1431,43 +1491,38 @@ struct PassBuilder {
             }
             Cx d[16];
             uint32_t minus = 0;
-            bool phases = false;
             for (uint32_t j = 0; j < 16; j++) {
-                d[j] = Cx{1.0, 0.0};
+                CxL x(1.0L, 0.0L);
                 for (int P = 0; P < 4; P++) {
-                    if (!((j & have) >> P & 1u)) continue;
-                    d[j] = cmul(d[j], u[P]);
+                    if (!((j >> P) & 1u)) continue;
+                    x = x * u[P];
                     if (__builtin_popcount(r[P] & j) & 1) minus ^= 1u << j;
                 }
-                if ((minus >> j) & 1u) d[j] = Cx{-d[j].re, -d[j].im};
+                d[j] = ((minus >> j) & 1u ? -1.0L * x : x).round();
             }
-            for (int P = 0; P < 4; P++) phases |= ((have >> P) & 1u) && !is(u[P], 1.0);
+            const bool phases = !(is(u[0], 1.0L) && is(u[1], 1.0L) && is(u[2], 1.0L) && is(u[3], 1.0L));
             if (!phases && minus) {
                 ROp neg;
                 memset(&neg, 0, sizeof(neg));
                 neg.head = RC_NEG | (minus << 16);
                 out.push_back(neg);
             }
-            bool first = true;
             for (int P = 0; P < 4; P++) {
-                if (!((have >> P) & 1u)) continue;
                 ROp op = list[(size_t)at[P]];
-                op.head = (op.head & ~0xffu) | (first ? (uint32_t)RC_LAYER : (uint32_t)RC_REAL1 + (uint32_t)P);
+                op.head = (op.head & ~0xffu) | (P == 0 ? (uint32_t)RC_LAYER : (uint32_t)RC_REAL1 + (uint32_t)P);
                 op.sign &= 0xffff0000u;
                 op.sel0 = ~0u;
-                op.sel1 = have;
                 // (in the place of the op's own coefficients)
                 p->coef[op.coef] = m[P][0];
                 p->coef[op.coef + 1] = m[P][1];
-                if (first && phases) {
+                if (P == 0 && phases) {
                     op.sel0 = (uint32_t)p->coef.size();
                     p->coef.insert(p->coef.end(), d + 1, d + 16);
                 }
                 out.push_back(op);
-                first = false;
             }
             std::sort(at, at + 4);
-            for (int q = 3; q >= 0 && at[q] >= 0; q--) list.erase(list.begin() + at[q]);
+            for (int q = 3; q >= 0; q--) list.erase(list.begin() + at[q]);
         }
         p->ops.resize(begin);
         p->ops.insert(p->ops.end(), out.begin(), out.end());
@@ -1486,7 +1541,7 @@ struct PassBuilder {
                 for (int c = 1; c < 4; c++)
                     if (std::hypot(at(c).re, at(c).im) > std::hypot(at(big).re, at(big).im)) big = c;
                 const double norm = std::hypot(at(big).re, at(big).im);
-                f[r] = norm > 0.0 ? unit(at(big)) : Cx{1.0, 0.0};
+                f[r] = norm > 0.0 ? unit(at(big)).round() : Cx{1.0, 0.0};
                 for (int c = 0; c < 4; c++) {
                     const Cx x = cmul(at(c), conj(f[r]));
                     ok &= std::fabs(x.im) <= 1e-15 * norm;  // rounding of the products

@@ -54,7 +54,7 @@ enum RCode : uint32_t {
     RC_DIAG = 33,    // the masked amplitudes, each times its own coefficient
     RC_NEG = 34,     // the masked amplitudes times -1
     RC_LAYER = 35,   // amplitudes 1 to 15 times the coefficients from sel0 (~0: no such product), then
-                     // REAL1 ops without pair signs on the positions in sel1: this op and the next ones
+                     // REAL1 ops without pair signs on positions 0 to 3: this op and the next three
     // density-matrix steps
     RC_CHAN1 = 36,   // + pair: a 1-qubit Kraus sum; sel0: operators, three coefficients each (exact passes)
     RC_CHAN2 = 38,   // a 2-qubit Kraus sum; sel0: operators, five coefficients each (exact passes)
