@@ -33,3 +33,23 @@ def test_norm_of_a_batch():
     for r in regs:
         norm = float(np.sum(np.abs(r.state_vec().astype(np.clongdouble)) ** 2))
         assert abs(norm - 1.0) < 5.2e-14  # as above, on fewer qubits
+
+
+# complex64 with the norm restored (256 gates and more): amplitudes move by
+# one FP32 ulp (1.2e-7 at most) where the hash of their index says so, so what
+# is left is a sum of 2^23 independent moves: 2.4e-7 / sqrt(2^23) = 8e-11 at
+# most, five times that.  (Rounded to nearest, a factor within half an ulp of
+# 1 moves no amplitude at all.)
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [False, True])
+@pytest.mark.parametrize("seed", [1, 2])
+def test_norm_of_complex64(seed, batch):
+    n = 22
+    c = layered_circuit(n, 6, seed=seed)
+    r = Y.ArrayReg.zero_state(n, Y.C64)
+    if batch:
+        Y.batch_apply([c, c], [r, Y.ArrayReg.zero_state(n, Y.C64)], Y.MODE_FUSED)
+    else:
+        Y.apply_inplace(c, r, Y.MODE_FUSED)
+    norm = float(np.sum(np.abs(r.state_vec().astype(np.complex128)) ** 2))
+    assert abs(norm - 1.0) < 4e-10

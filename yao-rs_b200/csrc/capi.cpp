@@ -879,7 +879,7 @@ int yao_apply_inplace_mode(const yao_circuit* cc, yao_reg* r, int32_t mode, int3
     // shrinks it by up to about 1e-7 per block; a unitary circuit keeps the
     // input's norm, so the FP64 norm of the input is restored afterwards
     // when blocks ran on the tensor cores or the circuit has 256 gates or
-    // more (shorter CUDA-core runs drift by less than an FP32 ulp).
+    // more.
     // YAO_NORM_RESTORE=0 leaves the norm as the arithmetic produced it (for
     // measuring the drift)
     const char* nr_env = getenv("YAO_NORM_RESTORE");
@@ -893,7 +893,7 @@ int yao_apply_inplace_mode(const yao_circuit* cc, yao_reg* r, int32_t mode, int3
     if (renorm && n0 > 0.0 && (r->ctx->tc_used || prog.size() >= 256)) {
         double n1 = 0.0;
         if ((s = reduce_norm_sqr(r->ctx, r, &n1))) return s;
-        if (n1 > 0.0 && (s = launch_scale(r->ctx, r, std::sqrt(n1 / n0)))) return s;
+        if (n1 > 0.0 && (s = launch_norm_restore(r->ctx, r, std::sqrt(n1 / n0)))) return s;
     }
     YAO_CUDA(cudaGetLastError());
     return YAO_OK;

@@ -192,6 +192,45 @@ int launch_scale(Ctx* ctx, Reg* r, double norm) {
     return YAO_OK;
 }
 
+// x / d in FP32, up or down at random (a fixed hash of the amplitude's place)
+// with the odds that make the mean exact.  A divisor within half an FP32 ulp
+// of 1 rounds to nearest leave every amplitude as it is, so the norm that the
+// division restores would stay off by up to 1e-7.
+__device__ __forceinline__ float div_dithered(double x, double d, uint64_t place) {
+    const double q = __ddiv_rn(x, d);
+    const float lo = __double2float_rd(q), hi = __double2float_ru(q);
+    uint64_t h = place * 0x9e3779b97f4a7c15ull;  // splitmix64 (Steele, Lea, Flood 2014)
+    h = (h ^ (h >> 30)) * 0xbf58476d1ce4e5b9ull;
+    h = (h ^ (h >> 27)) * 0x94d049bb133111ebull;
+    h ^= h >> 31;
+    return (double)(h >> 11) * 0x1p-53 * ((double)hi - (double)lo) < q - (double)lo ? hi : lo;
+}
+// amplitude i of a register over d: dithered where d is within 8 FP32 ulps of
+// 1 (beyond them the roundings to nearest average out)
+__device__ __forceinline__ float2 restore_one(float2 v, double d, uint64_t i) {
+    if (fabs(d - 1.0) < 0x1p-20) return make_float2(div_dithered(v.x, d, 2 * i), div_dithered(v.y, d, 2 * i + 1));
+    return from_d2<float2>(make_double2(__ddiv_rn((double)v.x, d), __ddiv_rn((double)v.y, d)));
+}
+__device__ __forceinline__ double2 restore_one(double2 v, double d, uint64_t) {
+    return make_double2(__ddiv_rn(v.x, d), __ddiv_rn(v.y, d));
+}
+template <typename V>
+__global__ void k_restore(V* st, uint64_t n, double d) {
+    GRID_STRIDE(i, n) st[i] = restore_one(st[i], d, i);
+}
+
+int launch_norm_restore(Ctx* ctx, Reg* r, double d) {
+    const uint64_t n = (uint64_t)1 << r->nbits;
+    const unsigned g = grid_for(n, 256, ctx->num_sms);
+    if (r->precision == YAO_C128)
+        k_restore<double2><<<g, 256, 0, ctx->stream>>>((double2*)r->d, n, d);
+    else
+        k_restore<float2><<<g, 256, 0, ctx->stream>>>((float2*)r->d, n, d);
+    ctx->launches++;
+    YAO_CUDA(cudaGetLastError());
+    return YAO_OK;
+}
+
 // ------------------------------------------------------ norm / inner product
 
 template <typename V>
@@ -1254,10 +1293,8 @@ __global__ void __launch_bounds__(kRT) k_chunk_rescale(const NormChunk* __restri
     if (!(a > 0.0 && b > 0.0)) return;
     const double d = sqrt(b / a);
     V* st = (V*)(uintptr_t)c.p;
-    for (uint32_t i = threadIdx.x; i < c.len; i += blockDim.x) {
-        double2 v = to_d2(st[i]);
-        st[i] = from_d2<V>(make_double2(__ddiv_rn(v.x, d), __ddiv_rn(v.y, d)));
-    }
+    for (uint32_t i = threadIdx.x; i < c.len; i += blockDim.x)
+        st[i] = restore_one(st[i], d, (uint64_t)blockIdx.x * kNormChunk + i);
 }
 
 static void norm_chunks(const std::vector<Reg*>& regs, std::vector<NormChunk>& ch, std::vector<uint32_t>& first) {

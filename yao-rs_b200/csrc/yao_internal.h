@@ -233,6 +233,8 @@ int launch_deterministic_state(Ctx* ctx, Reg* r);
 int launch_convert(Ctx* ctx, const Reg* src, Reg* dst);
 int reduce_norm_sqr(Ctx* ctx, const Reg* r, double* out);
 int launch_scale(Ctx* ctx, Reg* r, double inv_norm);
+// amplitudes / d for a d near 1: exact in the mean also in FP32
+int launch_norm_restore(Ctx* ctx, Reg* r, double d);
 int adjoint_tiles(Ctx* ctx, Reg* psi, Reg* lam, const Circuit* c, double* grad, size_t np);
 // adjoint_tiles in two halves: the host plan (null with *status
 // YAO_ERR_UNSUPPORTED when the per-gate form must run) and its sweep
