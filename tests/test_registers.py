@@ -1,0 +1,88 @@
+"""Memory and streams of registers: what their device address may be used
+for, and where the memory of freed ones goes."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+import yao_rs as Y
+from helpers import random_state
+from yao_rs import _abi as A
+
+pytestmark = pytest.mark.gpu
+
+
+def device_ptr(reg):
+    p = C.c_void_p()
+    A.check(A.lib().yao_reg_device_ptr(reg.handle, C.byref(p)))
+    return p.value
+
+
+@pytest.mark.parametrize("n", [2, 10, 20, 24])
+def test_address_can_be_shared_with_other_processes(n):
+    """The address is plain device memory (cudaIpcGetMemHandle takes it), for
+    new registers and for ones that reuse memory."""
+    get = C.CDLL("libcuda.so.1").cuIpcGetMemHandle
+    get.argtypes = [C.c_void_p, C.c_uint64]
+    for _ in range(3):
+        reg = Y.ArrayReg.zero_state(n)
+        handle = (C.c_char * 64)()
+        assert get(handle, device_ptr(reg)) == 0
+        del reg
+
+
+def test_memory_of_freed_registers():
+    """Reused for registers of the same size in the order of the stream, from
+    several threads, and at most 1 GiB of it kept."""
+    torch = pytest.importorskip("torch")
+    regs = [Y.ArrayReg.zero_state(23) for _ in range(16)]  # 2 GiB
+    A.synchronize(0)
+    free = torch.cuda.mem_get_info(0)[0]
+    del regs
+    A.synchronize(0)
+    assert torch.cuda.mem_get_info(0)[0] - free >= (1 << 30)
+    rng = np.random.default_rng(0)
+    states = {n: random_state(rng, n) for n in (3, 12, 16, 20)}
+    failed = []
+
+    def work(seed):
+        order = np.random.default_rng(seed)
+        for _ in range(40):
+            n = int(order.choice(list(states)))
+            v = states[n] * np.exp(1j * seed)
+            a = Y.ArrayReg.from_vec(n, v)
+            b = Y.ArrayReg.zero_state(n)
+            del b
+            if not np.array_equal(a.state_vec(), v):
+                failed.append((seed, n))
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
+def test_address_on_another_stream():
+    """A register freed while another stream still reads its address: the free
+    waits for that stream, also where the memory is used again."""
+    torch = pytest.importorskip("torch")
+    n = 24
+    v = random_state(np.random.default_rng(1), n)
+    reg = Y.ArrayReg.from_vec(n, v)
+    side = torch.cuda.Stream()
+
+    class Amplitudes:
+        __cuda_array_interface__ = {"shape": (1 << n,), "typestr": "<c16", "data": (device_ptr(reg), False),
+                                    "version": 3, "strides": None}
+    src, big = torch.as_tensor(Amplitudes(), device="cuda"), torch.ones(1 << 27, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            big.mul_(1.0001)
+        got = src.clone()
+    del reg
+    other = Y.ArrayReg.zero_state(n)
+    torch.cuda.synchronize()
+    assert np.array_equal(got.cpu().numpy(), v) and other.norm() == 1.0

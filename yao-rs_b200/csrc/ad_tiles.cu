@@ -1322,7 +1322,7 @@ int adjoint_run(Ctx* ctx, Reg* psi, Reg* lam, const AdjPlan* plan, double* grad)
     const size_t b_ops = al(std::max<size_t>(1, nops) * sizeof(AdjTileOp)),
                  b_part = al((size_t)grid * kAdjMaxSlots * sizeof(double)), b_dots = al(std::max<size_t>(1, ndots) * 8);
     char* buf = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&buf, b_ops + b_part + b_dots, ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&buf, b_ops + b_part + b_dots));
     AdjTileOp* d_ops = (AdjTileOp*)buf;
     double* d_part = (double*)(buf + b_ops);
     double* d_dots = (double*)(buf + b_ops + b_part);

@@ -32,54 +32,101 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 // ----------------------------------------------------------------- context
-// cudaMalloc; when it fails, the freed memory that the device's default pool
-// keeps is released (after this context's queued frees) and it is tried once
-// more.
-static cudaError_t alloc_device(Ctx* ctx, void** p, size_t bytes) {
+// Memory of freed registers of up to 256 MiB is kept for the context's next
+// register of that size, at most 1 GiB a device: a cudaMalloc and a cudaFree
+// of a 16 MB register took 400 and 350 us where its whole circuit takes 280.
+// (Larger registers are milliseconds of work each.)  It is cudaMalloc's
+// memory, so that an address can go to cudaIpcGetMemHandle and to peers.  Work
+// queued on the context's stream precedes what the next register does; where
+// work may be elsewhere (free_state) the free waits for the device.
+constexpr size_t kKeptBlock = (size_t)256 << 20, kKeptDevice = (size_t)1 << 30, kKeptBlocks = 1024;
+
+struct Kept {
+    std::mutex mu;
+    std::multimap<std::pair<Ctx*, size_t>, void*> blocks;
+    std::map<int, size_t> held;  // bytes by device
+};
+static Kept& kept() {
+    static Kept* k = new Kept();  // (registers may be freed while statics are destroyed)
+    return *k;
+}
+
+// Gives the kept blocks of a device, or of one context, back to the driver
+// (cudaFree waits for work on them).
+static void release_kept(int device, Ctx* ctx = nullptr) {
+    Kept& k = kept();
+    std::lock_guard<std::mutex> g(k.mu);
+    for (auto it = k.blocks.begin(); it != k.blocks.end();) {
+        if (it->first.first->device != device || (ctx && it->first.first != ctx)) {
+            ++it;
+            continue;
+        }
+        cudaFree(it->second);
+        k.held[device] -= it->first.second;
+        it = k.blocks.erase(it);
+    }
+}
+
+cudaError_t alloc_device(Ctx* ctx, void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
     cudaMemPool_t pool;
+    release_kept(ctx->device);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
         cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
         return e;
     return cudaMalloc(p, bytes);
 }
 
-// Registers of up to 256 MiB come from the device's memory pool
-// (stream-ordered on the context's stream; it keeps at most 4 GiB): a
-// cudaMalloc and a cudaFree of a 16 MB register took 400 and 350 us where its
-// whole circuit takes 280.  Larger ones would soon take the pool beyond what
-// it keeps, and it then unmaps and maps again (1 GiB registers: passes of 13
-// ms took 95); they are milliseconds of work each and are given back to the
-// driver when freed.  An allocation made while the stream is captured must
-// outlive the graph.
-constexpr size_t kPooledBytes = (size_t)256 << 20;
+cudaError_t alloc_async(Ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    release_kept(ctx->device);
+    return cudaMallocAsync(p, bytes, ctx->stream);
+}
 
-static cudaError_t alloc_state(Ctx* ctx, void** p, size_t bytes, bool* pooled) {
-    *pooled = false;
+static bool capturing(Ctx* ctx) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (bytes <= kPooledBytes && cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess &&
-        cs == cudaStreamCaptureStatusNone) {
-        if (cudaMallocAsync(p, bytes, ctx->stream) == cudaSuccess) {
-            *pooled = true;
+    return cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+static cudaError_t alloc_state(Ctx* ctx, void** p, size_t bytes) {
+    // (memory taken while the stream is captured belongs to the graph's replays)
+    if (bytes <= kKeptBlock && !capturing(ctx)) {
+        Kept& k = kept();
+        std::lock_guard<std::mutex> g(k.mu);
+        const auto it = k.blocks.find({ctx, bytes});
+        if (it != k.blocks.end()) {
+            *p = it->second;
+            k.blocks.erase(it);
+            k.held[ctx->device] -= bytes;
             return cudaSuccess;
         }
-        cudaGetLastError();
     }
     return alloc_device(ctx, p, bytes);
 }
 
 // exported: the address was handed out, so work on any stream may still use
-// it (cudaFree waits for the device by itself)
-static void free_state(Ctx* ctx, void* p, bool pooled, bool exported) {
-    if (!pooled) {
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(p);
-        return;
+// it; so may replays of a graph captured from the context's stream, once that
+// was handed out.  (cudaFree waits for the device by itself.)
+static void free_state(Ctx* ctx, void* p, size_t bytes, bool exported) {
+    if (bytes <= kKeptBlock && !capturing(ctx)) {
+        const bool wait = exported || ctx->stream_out.load();
+        if (!wait || cudaDeviceSynchronize() == cudaSuccess) {
+            Kept& k = kept();
+            std::lock_guard<std::mutex> g(k.mu);
+            size_t& held = k.held[ctx->device];
+            if (held + bytes <= kKeptDevice && k.blocks.size() < kKeptBlocks) {
+                k.blocks.insert({{ctx, bytes}, p});
+                held += bytes;
+                return;
+            }
+        }
     }
-    if (exported) cudaDeviceSynchronize();
-    cudaFreeAsync(p, ctx->stream);
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(p);
 }
 
 int Ctx::ensure_scratch(size_t bytes) {
@@ -316,7 +363,7 @@ static int alloc_reg(Ctx* ctx, uint32_t nbits, int32_t prec, Reg** out) {
     r->ctx = ctx;
     r->nbits = nbits;
     r->precision = prec;
-    cudaError_t e = alloc_state(ctx, &r->d, r->bytes(), &r->pooled);
+    cudaError_t e = alloc_state(ctx, &r->d, r->bytes());
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate a " + std::to_string(nbits) + "-qubit register (" +
@@ -333,7 +380,7 @@ static int alloc_dm(Ctx* ctx, uint32_t nbits, DM** out) {
     std::unique_ptr<yao_dm> d(new yao_dm());
     d->ctx = ctx;
     d->nbits = nbits;
-    if (alloc_state(ctx, &d->d, d->bytes(), &d->pooled) != cudaSuccess) {
+    if (alloc_state(ctx, &d->d, d->bytes()) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the density matrix");
     }
@@ -403,6 +450,7 @@ int yao_ctx_destroy(yao_ctx* c) {
     if (!c) return YAO_OK;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
+    release_kept(c->device, c);
     if (c->scratch) cudaFree(c->scratch);
     if (c->d_err) cudaFree(c->d_err);
     if (c->host_pinned) cudaFreeHost(c->host_pinned);
@@ -429,6 +477,7 @@ int yao_ctx_launch_count(const yao_ctx* c, uint64_t* out) {
 int yao_ctx_stream(const yao_ctx* c, void** out) {
     CHECK_NULL(c);
     CHECK_NULL(out);
+    c->stream_out.store(true);
     *out = (void*)c->stream;
     return YAO_OK;
 }
@@ -634,7 +683,7 @@ int yao_reg_zero_state(yao_ctx* ctx, uint32_t nbits, int32_t precision, yao_reg*
     if (s) return s;
     s = launch_fill_zero_state(ctx, r, 0);
     if (s) {
-        free_state(ctx, r->d, r->pooled, false);
+        free_state(ctx, r->d, r->bytes(), false);
         delete r;
         return s;
     }
@@ -664,7 +713,7 @@ int yao_reg_from_host(yao_ctx* ctx, uint32_t nbits, const double* amps, yao_reg*
     cudaError_t e = cudaMemcpyAsync(r->d, amps, r->bytes(), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        free_state(ctx, r->d, r->pooled, false);
+        free_state(ctx, r->d, r->bytes(), false);
         delete r;
         return cuda_fail(e, "upload");
     }
@@ -716,7 +765,7 @@ int yao_reg_deterministic_state(yao_ctx* ctx, uint32_t nbits, yao_reg** out) {
 void yao_reg_free(yao_reg* r) {
     if (!r) return;
     cudaSetDevice(r->ctx->device);
-    free_state(r->ctx, r->d, r->pooled, r->exported);
+    free_state(r->ctx, r->d, r->bytes(), r->exported);
     delete r;
 }
 
@@ -777,9 +826,6 @@ int yao_reg_upload(yao_reg* r, const void* amps) {
 int yao_reg_device_ptr(const yao_reg* r, void** out) {
     CHECK_NULL(r);
     CHECK_NULL(out);
-    // stream-ordered memory may be used on other streams once its allocation
-    // has taken place
-    if (r->pooled && !r->exported) YAO_CUDA(cudaStreamSynchronize(r->ctx->stream));
     r->exported = true;
     *out = r->d;
     return YAO_OK;
@@ -1025,7 +1071,7 @@ int yao_dm_mixed(yao_ctx* ctx, const double* weights, const yao_reg* const* regs
 void yao_dm_free(yao_dm* d) {
     if (!d) return;
     cudaSetDevice(d->ctx->device);
-    free_state(d->ctx, d->d, d->pooled, false);
+    free_state(d->ctx, d->d, d->bytes(), false);
     delete d;
 }
 
@@ -1313,7 +1359,7 @@ int yao_expect_grad(const yao_term* terms, size_t nterms, const yao_circuit* cc,
         }
     } pool{ctx};
     const size_t bytes = psi_r.bytes();
-    if (cudaMallocAsync(&pool.a, bytes, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, &pool.a, bytes) != cudaSuccess) {
         cudaGetLastError();
         pool.a = nullptr;
         return fail(YAO_ERR_OUT_OF_MEMORY, "expect_grad: cannot allocate the forward state");
@@ -1364,7 +1410,7 @@ int yao_expect_grad(const yao_term* terms, size_t nterms, const yao_circuit* cc,
         *value = acc.re;
         return YAO_OK;
     }
-    if (cudaMallocAsync(&pool.b, bytes, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, &pool.b, bytes) != cudaSuccess) {
         cudaGetLastError();
         pool.b = nullptr;
         return fail(YAO_ERR_OUT_OF_MEMORY, "expect_grad: cannot allocate lambda");
@@ -1623,7 +1669,7 @@ int yao_batch_apply(const yao_circuit* const* circuits, yao_reg* const* regs, si
     double* d_norm = nullptr;
     int s;
     if (!nr.empty()) {
-        YAO_CUDA(cudaMallocAsync((void**)&d_norm, 2 * nr.size() * sizeof(double), ctx->stream));
+        YAO_CUDA(alloc_async(ctx, (void**)&d_norm, 2 * nr.size() * sizeof(double)));
         if ((s = launch_batch_norm_sqr(ctx, nr, d_norm))) {
             cudaFreeAsync(d_norm, ctx->stream);
             return s;

@@ -1960,7 +1960,7 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
         YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     }
     unsigned char* dblob = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&dblob, plan.blob.size(), ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&dblob, plan.blob.size()));
     YAO_CUDA(cudaMemcpyAsync(dblob, plan.blob.data(), plan.blob.size(), cudaMemcpyHostToDevice, ctx->stream));
     const size_t amp = precision == YAO_C128 ? 16 : 8;
     int s = YAO_OK;
@@ -2032,7 +2032,7 @@ int reg_batch(Ctx* ctx, const std::vector<RegPlan>& plans, const std::vector<Reg
     const size_t total = nblob + b_pass + b_owner;
     int st;
     if ((st = grow_host(&ctx->batch_host, &ctx->batch_host_bytes, total))) return st;
-    if ((st = grow_dev(&ctx->batch_dev, &ctx->batch_dev_bytes, total, ctx->stream))) return st;
+    if ((st = grow_dev(ctx, &ctx->batch_dev, &ctx->batch_dev_bytes, total))) return st;
     char* h = (char*)ctx->batch_host;
     char* d = (char*)ctx->batch_dev;
     for (size_t c = 0; c < plans.size(); c++) memcpy(h + blob_at[c], plans[c].blob.data(), plans[c].blob.size());

@@ -395,7 +395,7 @@ static int expect_tiles(Ctx* ctx, const Reg* r, const std::vector<EPass>& passes
     }
     double* part = (double*)ctx->scratch;
     uint4* dblob = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&dblob, blob.size() * sizeof(uint4), ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&dblob, blob.size() * sizeof(uint4)));
     YAO_CUDA(cudaMemcpyAsync(dblob, blob.data(), blob.size() * sizeof(uint4), cudaMemcpyHostToDevice, ctx->stream));
     for (size_t q = 0; q < ls.size(); q++) {
         EHdr& h = ls[q].hdr;

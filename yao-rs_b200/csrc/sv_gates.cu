@@ -203,7 +203,7 @@ static int launch_gate_n(Ctx* ctx, V* st, uint32_t nbits, const LGate& g, uint64
     memcpy(host.data() + nm * sizeof(V), locked, 64);
     memcpy(host.data() + nm * sizeof(V) + 64, g.tb, sizeof(int32_t) * kMaxTargets);
     void* dbuf = nullptr;
-    YAO_CUDA(cudaMallocAsync(&dbuf, bytes, ctx->stream));
+    YAO_CUDA(alloc_async(ctx, &dbuf, bytes));
     YAO_CUDA(cudaMemcpyAsync(dbuf, host.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
     // the pageable source is consumed before cudaMemcpyAsync returns
     const V* dm = (const V*)dbuf;

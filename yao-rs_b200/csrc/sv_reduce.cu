@@ -710,7 +710,7 @@ static int lambda_launch(Ctx* ctx, const void* psi_d, void* lam_d, uint32_t nbit
     }
     void* d = nullptr;
     size_t bytes = std::max<size_t>(1, h.size()) * sizeof(MonoFull);
-    YAO_CUDA(cudaMallocAsync(&d, bytes, ctx->stream));
+    YAO_CUDA(alloc_async(ctx, &d, bytes));
     if (!h.empty()) YAO_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(MonoFull), cudaMemcpyHostToDevice, ctx->stream));
     const unsigned grid = grid_for((n + kLamR - 1) / kLamR, kRT, ctx->num_sms);
     double* part = nullptr;
@@ -1317,7 +1317,7 @@ int launch_batch_norm_sqr(Ctx* ctx, const std::vector<Reg*>& regs, double* out) 
     const size_t b_ch = (ch.size() * sizeof(NormChunk) + 255) / 256 * 256,
                  b_first = (first.size() * sizeof(uint32_t) + 255) / 256 * 256;
     char* buf = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&buf, b_ch + b_first + ch.size() * sizeof(double), ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&buf, b_ch + b_first + ch.size() * sizeof(double)));
     NormChunk* d_ch = (NormChunk*)buf;
     uint32_t* d_first = (uint32_t*)(buf + b_ch);
     double* d_part = (double*)(buf + b_ch + b_first);
@@ -1343,7 +1343,7 @@ int launch_batch_rescale(Ctx* ctx, const std::vector<Reg*>& regs, const double* 
     std::vector<uint32_t> first;
     norm_chunks(regs, ch, first);
     NormChunk* d_ch = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&d_ch, ch.size() * sizeof(NormChunk), ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&d_ch, ch.size() * sizeof(NormChunk)));
     YAO_CUDA(cudaMemcpyAsync(d_ch, ch.data(), ch.size() * sizeof(NormChunk), cudaMemcpyHostToDevice, ctx->stream));
     if (regs[0]->precision == YAO_C128)
         k_chunk_rescale<double2><<<(unsigned)ch.size(), kRT, 0, ctx->stream>>>(d_ch, n0, n1);

@@ -1900,16 +1900,17 @@ static size_t padded_count(const std::vector<TOp>& ops, size_t ncoef, int rb, ui
 }
 
 // Grow a kept device / pinned host buffer to at least `bytes` (by 1.25x).
-int grow_dev(void** p, size_t* have, size_t bytes, cudaStream_t s) {
+int grow_dev(Ctx* ctx, void** p, size_t* have, size_t bytes) {
     if (bytes <= *have) return YAO_OK;
     const size_t nb = std::max(bytes, *have + *have / 4);
     if (*p) {
-        YAO_CUDA(cudaStreamSynchronize(s));
+        YAO_CUDA(cudaStreamSynchronize(ctx->stream));
         YAO_CUDA(cudaFree(*p));
         *p = nullptr;
         *have = 0;
     }
-    if (cudaMalloc(p, nb) != cudaSuccess) {
+    if (alloc_device(ctx, p, nb) != cudaSuccess) {
+        cudaGetLastError();
         *p = nullptr;
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the batch tables");
     }
@@ -2044,7 +2045,7 @@ static int run_pass(Ctx* ctx, V* st, uint32_t nbits, const PassPlan& pp) {
     size_t cb_off = sb_off + al(sb);
     size_t mb_off = cb_off + al(cb);
     void* dbuf = nullptr;
-    YAO_CUDA(cudaMallocAsync(&dbuf, mb_off + mb, ctx->stream));
+    YAO_CUDA(alloc_async(ctx, &dbuf, mb_off + mb));
     YAO_CUDA(cudaMemcpyAsync(dbuf, ops.data(), ob, cudaMemcpyHostToDevice, ctx->stream));
     YAO_CUDA(cudaMemcpyAsync((char*)dbuf + sb_off, pp.segs.data(), sb, cudaMemcpyHostToDevice, ctx->stream));
     YAO_CUDA(cudaMemcpyAsync((char*)dbuf + cb_off, hc.data(), cb, cudaMemcpyHostToDevice, ctx->stream));
@@ -2471,7 +2472,7 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
     }
     const size_t bytes = ((size_t)1 << n) * sizeof(V);
     V* scratch = nullptr;
-    if (cudaMallocAsync((void**)&scratch, bytes, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, (void**)&scratch, bytes) != cudaSuccess) {
         cudaGetLastError();
         return YAO_OK;
     }
@@ -2824,7 +2825,7 @@ static int batch_t(Ctx* ctx, const std::vector<const std::vector<LGate>*>& progs
     const size_t b_tab = b_ent + b_chk + b_ops + b_seg + b_coef;
     int st;
     if ((st = grow_host(&ctx->batch_host, &ctx->batch_host_bytes, b_tab))) return st;
-    if ((st = grow_dev(&ctx->batch_dev, &ctx->batch_dev_bytes, b_tab + b_ctr, ctx->stream))) return st;
+    if ((st = grow_dev(ctx, &ctx->batch_dev, &ctx->batch_dev_bytes, b_tab + b_ctr))) return st;
     char* hp = (char*)ctx->batch_host;
     BatchEntry* h_ent = (BatchEntry*)hp;
     BatchChunk* h_chk = (BatchChunk*)(hp + b_ent);
@@ -2992,7 +2993,7 @@ static int tune_batch(Ctx* ctx, const std::vector<const std::vector<LGate>*>& pr
         total += (regs[c]->bytes() + 255) / 256 * 256;
     }
     char* scratch = nullptr;
-    if (cudaMallocAsync((void**)&scratch, total, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, (void**)&scratch, total) != cudaSuccess) {
         cudaGetLastError();
         return YAO_OK;
     }

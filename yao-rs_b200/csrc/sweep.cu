@@ -853,7 +853,7 @@ struct SweepRun {
                      b_runs = al(p->runs.size() * sizeof(SRunDev)), b_place = al(pl.size() * sizeof(SPlace)),
                      b_par = al(nsets * p->np * 8), b_cf = al((size_t)group * p->runs.size() * 64),
                      b_part = al(np * 8), b_grad = al(nsets * p->np * 8);
-        if (cudaMallocAsync((void**)&buf, b_blob + b_fac + b_runs + b_place + b_par + 2 * b_cf + b_part + b_grad, ctx->stream) !=
+        if (alloc_async(ctx, (void**)&buf, b_blob + b_fac + b_runs + b_place + b_par + 2 * b_cf + b_part + b_grad) !=
             cudaSuccess) {
             cudaGetLastError();
             buf = nullptr;
@@ -955,7 +955,7 @@ int sweep_batch(Ctx* ctx, const SweepPlan* p, const std::vector<MonoTerm>& terms
     if (s) return s;
     char* st = nullptr;
     const size_t b_state = group * N * 16, b_val = (nsets * 8 + 255) / 256 * 256;
-    if (cudaMallocAsync((void**)&st, 2 * b_state + b_val, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, (void**)&st, 2 * b_state + b_val) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the batched gradient buffers");
     }

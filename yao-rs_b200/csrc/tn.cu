@@ -586,7 +586,7 @@ static int contract_pair(Ctx* ctx, const DevTensor& A, const DevTensor& B, const
     const size_t cbytes = (clen * sizeof(double2) + 255) / 256 * 256;
     const size_t tbytes = (tg.size() + tm.size() + tn.size() + tk.size()) * sizeof(int64_t);
     char* buf = nullptr;
-    YAO_CUDA(cudaMallocAsync((void**)&buf, cbytes + tbytes, ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&buf, cbytes + tbytes));
     double2* dc = (double2*)buf;
     int64_t* dtg = (int64_t*)(buf + cbytes);
     int64_t* dtm = dtg + tg.size();
@@ -664,7 +664,7 @@ int tn_contract(Ctx* ctx, const TNet& tn, double* out, const uint32_t* path, siz
         DevTensor d;
         d.legs = tn.ixs[t];
         d.len = tn.tensors[t].size();
-        if (cudaMallocAsync((void**)&d.d, std::max<size_t>(1, d.len) * sizeof(double2), ctx->stream) != cudaSuccess) {
+        if (alloc_async(ctx, (void**)&d.d, std::max<size_t>(1, d.len) * sizeof(double2)) != cudaSuccess) {
             release();
             return fail(YAO_ERR_OUT_OF_MEMORY, "tensor network: cannot allocate a tensor");
         }
@@ -785,7 +785,7 @@ int tn_contract(Ctx* ctx, const TNet& tn, double* out, const uint32_t* path, siz
     // the result: remaining summed labels traced out, legs in the order of iy
     DevTensor one;
     one.len = 1;
-    YAO_CUDA(cudaMallocAsync((void**)&one.d, sizeof(double2), ctx->stream));
+    YAO_CUDA(alloc_async(ctx, (void**)&one.d, sizeof(double2)));
     const double2 h1 = make_double2(1.0, 0.0);
     YAO_CUDA(cudaMemcpyAsync(one.d, &h1, sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
     DevTensor res;

@@ -370,7 +370,7 @@ int expect_grad_batch(Ctx* ctx, const std::vector<MonoTerm>& terms, const Circui
     const size_t gen_b = hg.size() * sizeof(double2), idx_b = std::max<size_t>(1, gidx.size()) * sizeof(int);
     char* buf = nullptr;
     const size_t total = 2 * sb + partial_b + 2 * coef_b + grad_b + vals_b + gen_b + idx_b + 4096;
-    if (cudaMallocAsync((void**)&buf, total, ctx->stream) != cudaSuccess) {
+    if (alloc_async(ctx, (void**)&buf, total) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the batched gradient buffers");
     }

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -130,6 +131,7 @@ struct Circuit {
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    mutable std::atomic<bool> stream_out{false};  // the stream was handed out (yao_ctx_stream)
     int num_sms = 148;
     // device scratch for reductions (grown on demand)
     void* scratch = nullptr;
@@ -177,12 +179,17 @@ struct ProfScope {
     }
 };
 
+// cudaMalloc, and cudaMallocAsync on the context's stream; when one fails, kept
+// memory of freed registers (and, for cudaMalloc, freed memory that the
+// device's default pool keeps) is given back and it is tried once more.
+cudaError_t alloc_device(Ctx* ctx, void** p, size_t bytes);
+cudaError_t alloc_async(Ctx* ctx, void** p, size_t bytes);
+
 struct Reg {
     Ctx* ctx = nullptr;
     uint32_t nbits = 0;
     int32_t precision = YAO_C128;
     void* d = nullptr;  // double2* (C128) or float2* (C64)
-    bool pooled = false;            // d is stream-ordered memory of ctx->stream
     mutable bool exported = false;  // the address was handed out (yao_reg_device_ptr)
     size_t bytes() const { return ((size_t)1 << nbits) * (precision == YAO_C128 ? 16 : 8); }
 };
@@ -191,7 +198,6 @@ struct DM {
     Ctx* ctx = nullptr;
     uint32_t nbits = 0;
     void* d = nullptr;  // double2*, 4^n
-    bool pooled = false;
     size_t bytes() const { return ((size_t)1 << (2 * nbits)) * 16; }
 };
 
@@ -222,7 +228,7 @@ struct KernelFit {
 };
 int kernel_fit(Ctx* ctx, const void* kernel, KernelFit* out, bool all = false);
 // The batch tables of a context, grown to at least `bytes`.
-int grow_dev(void** p, size_t* have, size_t bytes, cudaStream_t s);
+int grow_dev(Ctx* ctx, void** p, size_t* have, size_t bytes);
 int grow_host(void** p, size_t* have, size_t bytes);
 int launch_batch(Ctx* ctx, const std::vector<const std::vector<LGate>*>& progs, const std::vector<Reg*>& regs,
                  int32_t mode, int32_t k);
