@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
     uint32_t b = 0, par = 0;
     double acc[2] = {0.0, 0.0};
     for (; t < hdr.ntiles; t += grid) {
-        unsigned char* s = smem + (size_t)b * tile_bytes;
+        const unsigned char* s = smem + (size_t)b * tile_bytes;
         if (use_tma) {
             if (!dead) {
                 const uint64_t t0 = tma::now_ns();
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
             for (uint32_t l = threadIdx.x; l < (1u << hdr.tbits); l += blockDim.x) {
                 uint64_t o = base;
                 for (int j = 0; j < hdr.tbits; j++) o |= (uint64_t)((l >> j) & 1u) << hdr.tb[j];
-                *(V*)(s + tma::swizzle128(l * AB)) = st[o];
+                *(V*)(smem + tma::swizzle128(l * AB)) = st[o];  // the one buffer
             }
             __syncthreads();
         }
@@ -402,7 +402,7 @@ static int expect_tiles(Ctx* ctx, const Reg* r, const std::vector<EPass>& passes
         CUtensorMap tmap;
         memset(&tmap, 0, sizeof(tmap));
         h.use_tma = ntiles > 1 && tma_enabled() && tma_make_plan(h.tb, tbits, n, sizeof(V), r->d, h.tma, &tmap) ? 1 : 0;
-        h.nbuf = h.use_tma ? nbuf : 1;  // plain loads: nothing arrives ahead
+        h.nbuf = h.use_tma ? nbuf : 1;  // plain loads take turns in the first buffer: nothing arrives ahead
         ProfScope prof(ctx, "expect_tiles", (double)r->bytes());
         kern<<<grid, THREADS, smem, ctx->stream>>>((const V*)r->d, h, dblob + ls[q].off, part + 2 * (size_t)grid * q,
                                                    ctx->d_err, tmap);
