@@ -98,7 +98,11 @@ enum yao_precision { YAO_C128 = 0, YAO_C64 = 1 };
 /* Execution form of yao_apply_inplace_mode.
  *   PLAIN     every gate with yao-rs's own arithmetic, in order (bit-exact);
  *             on complex128 registers runs of gates share passes over the
- *             state where that is faster, else one kernel per gate;
+ *             state where that is faster, else one kernel per gate.  Returns
+ *             with the work queued on the context's stream; should a bounded
+ *             wait of that work give up, the next call that waits for
+ *             results (a download, a reduction, yao_ctx_synchronize) returns
+ *             YAO_ERR_TIMEOUT;
  *   TILED     runs of gates applied per tile of the state, same arithmetic
  *             and order as PLAIN (bit-exact), fewer HBM passes;
  *   FUSED     gates multiplied into dense k-qubit blocks on the host (FP64),

@@ -1,5 +1,5 @@
 """Memory and streams of registers: what their device address may be used
-for, and where the memory of freed ones goes."""
+for, where the memory of freed ones goes, calls that return with work queued."""
 import ctypes as C
 import threading
 
@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import yao_rs as Y
-from helpers import random_state
+from helpers import layered_circuit, random_state
 from yao_rs import _abi as A
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +86,22 @@ def test_address_on_another_stream():
     other = Y.ArrayReg.zero_state(n)
     torch.cuda.synchronize()
     assert np.array_equal(got.cpu().numpy(), v) and other.norm() == 1.0
+
+
+def test_plain_apply_returns_with_work_queued():
+    """PLAIN waits for nothing: one host thread keeps several contexts busy."""
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.ExternalStream(A.stream_ptr(0), device=torch.device("cuda", 0))
+    n = 27
+    c, reg = layered_circuit(n, 4, seed=3), Y.ArrayReg.zero_state(n)
+    Y.apply_inplace(c, reg)  # modules loaded, tables allocated
+    A.synchronize(0)
+    Y.apply_inplace(c, reg)
+    assert not stream.query()  # 50 ms and more of work
+    assert abs(reg.norm() - 1.0) < 1e-12
+    rho = Y.DensityMatrix.from_reg(Y.ArrayReg.zero_state(12))
+    layers = layered_circuit(12, 16, seed=4)
+    A.synchronize(0)
+    rho.apply(layers)
+    assert not stream.query()
+    assert abs(rho.trace() - 1.0) < 1e-12

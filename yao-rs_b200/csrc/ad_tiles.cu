@@ -1333,10 +1333,6 @@ int adjoint_run(Ctx* ctx, Reg* psi, Reg* lam, const AdjPlan* plan, double* grad)
         YAO_CUDA(cudaMemcpyAsync(d_ops, all.data(), all.size() * sizeof(AdjTileOp), cudaMemcpyHostToDevice,
                                  ctx->stream));
     }
-    if (!ctx->d_err) {
-        YAO_CUDA(cudaMalloc((void**)&ctx->d_err, sizeof(int)));
-        YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    }
     size_t ooff = 0, doff = 0;
     for (const AdjPass& p : passes) {
         AdjTileHdr hdr = p.hdr;
@@ -1375,6 +1371,7 @@ int adjoint_run(Ctx* ctx, Reg* psi, Reg* lam, const AdjPlan* plan, double* grad)
     YAO_CUDA(cudaFreeAsync(buf, ctx->stream));
     int herr = 0;
     YAO_CUDA(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    ctx->err_unread.store(false);
     YAO_CUDA(cudaStreamSynchronize(ctx->stream));
     if (herr) {
         YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));

@@ -439,6 +439,8 @@ int yao_ctx_create(int device, yao_ctx** out) {
     YAO_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
     uint64_t keep = (uint64_t)4 << 30;
     YAO_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    YAO_CUDA(cudaMalloc((void**)&c->d_err, sizeof(int)));
+    YAO_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     int sms = 0;
     YAO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     c->num_sms = sms;
@@ -463,8 +465,7 @@ int yao_ctx_destroy(yao_ctx* c) {
 
 int yao_ctx_synchronize(yao_ctx* c) {
     CHECK_NULL(c);
-    YAO_CUDA(cudaStreamSynchronize(c->stream));
-    return YAO_OK;
+    return wait_results(c, "synchronize");
 }
 
 int yao_ctx_launch_count(const yao_ctx* c, uint64_t* out) {
@@ -810,8 +811,7 @@ int yao_reg_to_host(const yao_reg* r, void* amps) {
     CHECK_NULL(amps);
     YAO_CUDA(cudaSetDevice(r->ctx->device));
     YAO_CUDA(cudaMemcpyAsync(amps, r->d, r->bytes(), cudaMemcpyDeviceToHost, r->ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(r->ctx->stream));
-    return YAO_OK;
+    return wait_results(r->ctx, "register download");
 }
 
 int yao_reg_upload(yao_reg* r, const void* amps) {
@@ -1098,8 +1098,7 @@ int yao_dm_to_host(const yao_dm* d, double* rho) {
     CHECK_NULL(rho);
     YAO_CUDA(cudaSetDevice(d->ctx->device));
     YAO_CUDA(cudaMemcpyAsync(rho, d->d, d->bytes(), cudaMemcpyDeviceToHost, d->ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(d->ctx->stream));
-    return YAO_OK;
+    return wait_results(d->ctx, "density-matrix download");
 }
 
 // FUSED density-matrix form: rho is a 2n-qubit vector (row bits above the
@@ -1520,8 +1519,7 @@ int yao_probs(const yao_reg* r, const uint32_t* locs, int32_t nlocs, double* out
         int s = launch_probs_full(ctx, r, (double*)ctx->scratch);
         if (s) return s;
         YAO_CUDA(cudaMemcpyAsync(out, ctx->scratch, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
-        YAO_CUDA(cudaStreamSynchronize(ctx->stream));
-        return YAO_OK;
+        return wait_results(ctx, "probs");
     }
     int s = check_measure_locs(r->nbits, locs, (uint32_t)nlocs);
     if (s) return s;

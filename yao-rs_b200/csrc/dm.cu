@@ -787,7 +787,8 @@ static int dm_finish(Ctx* ctx, double* part, int nb, int nv, double* host_out) {
     YAO_CUDA(cudaGetLastError());
     if (ctx->ensure_host_pinned(sizeof(double) * nv)) return YAO_ERR_OUT_OF_MEMORY;
     YAO_CUDA(cudaMemcpyAsync(ctx->host_pinned, dout, sizeof(double) * nv, cudaMemcpyDeviceToHost, ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int ws = wait_results(ctx, "density-matrix reduction");
+    if (ws) return ws;
     memcpy(host_out, ctx->host_pinned, sizeof(double) * nv);
     return YAO_OK;
 }
@@ -960,7 +961,8 @@ int reduce_dm_marginal(Ctx* ctx, const DM* d, const uint32_t* bits, int32_t nl, 
     YAO_CUDA(cudaGetLastError());
     std::vector<double> diag(dim);
     YAO_CUDA(cudaMemcpyAsync(diag.data(), dp, sizeof(double) * dim, cudaMemcpyDeviceToHost, ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int ws = wait_results(ctx, "density-matrix probs");
+    if (ws) return ws;
     if (nl < 0) {
         memcpy(host_out, diag.data(), sizeof(double) * dim);
         return YAO_OK;

@@ -1955,10 +1955,6 @@ static void pass_header(const RegPass& p, RHdr& h) {
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
                size_t step) {
     if (plan.passes.empty()) return YAO_OK;
-    if (!ctx->d_err) {
-        YAO_CUDA(cudaMalloc((void**)&ctx->d_err, sizeof(int)));
-        YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    }
     unsigned char* dblob = nullptr;
     YAO_CUDA(alloc_async(ctx, (void**)&dblob, plan.blob.size()));
     YAO_CUDA(cudaMemcpyAsync(dblob, plan.blob.data(), plan.blob.size(), cudaMemcpyHostToDevice, ctx->stream));
@@ -1972,6 +1968,7 @@ int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact
         memset(&tmap, 0, sizeof(tmap));
         // (one tile: nothing to overlap, and no wait that could give up)
         h.use_tma = p.ntiles > 1 && tma_enabled() && tma_make_plan(p.tb, p.tbits, nbits, amp, st, h.tma, &tmap) ? 1 : 0;
+        if (h.use_tma) ctx->err_unread.store(true);
         const uint4* blob = (const uint4*)(dblob + p.blob_off);
         bool dmx = false;
         for (const ROp& op : p.ops) dmx |= (op.head & 0xffu) >= RC_CHAN1;
@@ -2117,7 +2114,6 @@ int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
     YAO_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
     const bool passes = r->precision == YAO_C128 && reg_width(n) && cs == cudaStreamCaptureStatusNone;
     const double bytes = (double)r->bytes(), amps = (double)(1ull << n);
-    bool waits = false;
     for (size_t i = 0; i < prog.size();) {
         size_t end = i;  // the gates from i on that a register pass can run
         while (passes && end < prog.size() && reg_gate(prog[end])) end++;
@@ -2137,7 +2133,6 @@ int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
             if (joint < alone) {
                 int s = reg_launch(ctx, r->d, n, YAO_C128, true, plan, 0, 1);
                 if (s) return s;
-                waits |= n > 11;
                 i = end;
                 continue;
             }
@@ -2147,7 +2142,7 @@ int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
             if (s) return s;
         }
     }
-    return waits ? read_device_err(ctx, "apply") : YAO_OK;
+    return YAO_OK;
 }
 
 // ==================================================== density matrices
@@ -2256,7 +2251,6 @@ int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps) {
         }
         return YAO_OK;
     };
-    bool waits = false;
     std::vector<LGate> cache(steps.size());
     for (size_t i = 0; i < steps.size();) {
         // the steps from i on that a register pass can run
@@ -2291,7 +2285,6 @@ int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps) {
             if ((double)plan.passes.size() * (8e-6 + 2.0 * bytes / 5.2e12) + flops * entries / 1e13 < alone) {
                 int s = reg_launch(ctx, d->d, nb, YAO_C128, true, plan, 0, 1);
                 if (s) return s;
-                waits |= nb > 11;
                 i = end;
                 continue;
             }
@@ -2301,7 +2294,7 @@ int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps) {
             if (s) return s;
         }
     }
-    return waits ? read_device_err(ctx, "density-matrix apply") : YAO_OK;
+    return YAO_OK;
 }
 
 // FUSED steps on a density matrix; *done = false where a step has no form here
@@ -2384,7 +2377,7 @@ int dm_fused_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps, bool* done) 
     int s = reg_launch(ctx, d->d, nb, YAO_C128, false, plan, 0, 1);
     if (s) return s;
     *done = true;
-    return nb > 11 ? read_device_err(ctx, "density-matrix apply") : YAO_OK;
+    return ctx->err_unread.load() ? read_device_err(ctx, "density-matrix apply") : YAO_OK;
 }
 
 }  // namespace yao

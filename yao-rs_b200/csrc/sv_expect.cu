@@ -389,10 +389,6 @@ static int expect_tiles(Ctx* ctx, const Reg* r, const std::vector<EPass>& passes
     const size_t npart = 2 * (size_t)grid * ls.size();
     if (ctx->ensure_scratch(sizeof(double) * (npart + 2)) || ctx->ensure_host_pinned(3 * sizeof(double)))
         return YAO_ERR_OUT_OF_MEMORY;
-    if (!ctx->d_err) {
-        YAO_CUDA(cudaMalloc((void**)&ctx->d_err, sizeof(int)));
-        YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    }
     double* part = (double*)ctx->scratch;
     uint4* dblob = nullptr;
     YAO_CUDA(alloc_async(ctx, (void**)&dblob, blob.size() * sizeof(uint4)));
@@ -415,6 +411,7 @@ static int expect_tiles(Ctx* ctx, const Reg* r, const std::vector<EPass>& passes
     double* hp = (double*)ctx->host_pinned;
     YAO_CUDA(cudaMemcpyAsync(hp, part + npart, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     YAO_CUDA(cudaMemcpyAsync(hp + 2, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    ctx->err_unread.store(false);
     YAO_CUDA(cudaStreamSynchronize(ctx->stream));
     int herr;
     memcpy(&herr, hp + 2, sizeof(int));

@@ -70,7 +70,8 @@ static int finish_sum(Ctx* ctx, double* partial, int nblocks, int nv, double* ho
     YAO_CUDA(cudaGetLastError());
     if (ctx->ensure_host_pinned(sizeof(double) * nv)) return YAO_ERR_OUT_OF_MEMORY;
     YAO_CUDA(cudaMemcpyAsync(ctx->host_pinned, dout, sizeof(double) * nv, cudaMemcpyDeviceToHost, ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int ws = wait_results(ctx, "reduction");
+    if (ws) return ws;
     memcpy(host_out, ctx->host_pinned, sizeof(double) * nv);
     return YAO_OK;
 }
@@ -341,7 +342,8 @@ int reduce_max_abs_diff(Ctx* ctx, const Reg* a, const Reg* b, double* out) {
     YAO_CUDA(cudaGetLastError());
     if (ctx->ensure_host_pinned(sizeof(double))) return YAO_ERR_OUT_OF_MEMORY;
     YAO_CUDA(cudaMemcpyAsync(ctx->host_pinned, part + nb, sizeof(double), cudaMemcpyDeviceToHost, s));
-    YAO_CUDA(cudaStreamSynchronize(s));
+    const int ws = wait_results(ctx, "max_abs_diff");
+    if (ws) return ws;
     memcpy(out, ctx->host_pinned, sizeof(double));
     return YAO_OK;
 }
@@ -614,7 +616,8 @@ int expect_terms(Ctx* ctx, const Reg* r, const std::vector<MonoTerm>& terms, std
     ExpectPending pend;
     int s = expect_terms_launch(ctx, r, terms, pend);
     if (s) return s;
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+    s = wait_results(ctx, "expect");
+    if (s) return s;
     expect_terms_collect(ctx, pend, values);
     return YAO_OK;
 }
@@ -977,8 +980,7 @@ int reduce_marginal(Ctx* ctx, const Reg* r, const uint32_t* bits, uint32_t nl, d
     ctx->launches += 2;
     YAO_CUDA(cudaGetLastError());
     YAO_CUDA(cudaMemcpyAsync(host_out, dout, sizeof(double) * nout, cudaMemcpyDeviceToHost, ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
-    return YAO_OK;
+    return wait_results(ctx, "probs");
 }
 
 // collapse_qubits_to (src/measure.rs:158-185), first half: zero the
@@ -1233,7 +1235,8 @@ int expect_noalloc(Ctx* ctx, const Reg* r, const yao_term* terms, size_t nterms,
         YAO_CUDA(cudaGetLastError());
         double res[kNoAllocValues];
         YAO_CUDA(cudaMemcpyAsync(res, dres, sizeof(double) * nv, cudaMemcpyDeviceToHost, ctx->stream));
-        YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+        const int ws = wait_results(ctx, "expect");
+        if (ws) return ws;
         for (int q = 0; q < cnt; q++) values[idx[q]] = Cx{res[2 * q], res[2 * q + 1]};
     }
     // sum_t coeff_t * value_t in term order (src/expect.rs:7-11)

@@ -2114,15 +2114,12 @@ static int run_pass(Ctx* ctx, V* st, uint32_t nbits, const PassPlan& pp) {
     const TSeg* dsegs = (const TSeg*)((char*)dbuf + sb_off);
     const C* dcoef = (const C*)((char*)dbuf + cb_off);
     const float* dmmat = (const float*)((char*)dbuf + mb_off);
-    if (!ctx->d_err) {
-        YAO_CUDA(cudaMalloc((void**)&ctx->d_err, sizeof(int)));
-        YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    }
     {
         ProfScope prof(ctx, hdr.mma ? "tile_pass_tc" : (EXACT ? "tile_pass_exact" : "tile_pass_fused"),
                        (double)pp.hdr.ntiles * (double)((uint64_t)1 << pp.hdr.tbits) * 2.0 * sizeof(V));
         int s = launch_tile<V, EXACT>(pp.rb, ctx->num_sms, threads, smem, ctx->stream, st, hdr, dops, dsegs, dcoef,
                                       dmmat, ctx->d_err, tmap);
+        ctx->err_unread.store(true);
         if (s) return s;
     }
     ctx->launches++;
@@ -2295,16 +2292,8 @@ static int run_program_cfg(Ctx* ctx, V* st, uint32_t nbits, int32_t precision, c
     // operand copy or MMA completion) gave up: the run's result is void
     // (check_err false: the caller reads the error word at its own
     // synchronisation)
-    if (ctx->d_err && check_err) {
-        int herr = 0;
-        YAO_CUDA(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        YAO_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (herr) {
-            YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-            return fail(YAO_ERR_TIMEOUT, "tile pass: a bounded wait (tile copy, tensor-core operand or MMA) gave up");
-        }
-    }
-    return YAO_OK;
+    return check_err && ctx->err_unread.load() ? read_device_err(ctx, "tile pass (tile copy, tensor-core operand or MMA)")
+                                               : YAO_OK;
 }
 
 // ------------------------------------------------------------ autotuner
@@ -2668,13 +2657,19 @@ int launch_program(Ctx* ctx, Reg* r, const std::vector<LGate>& prog, int32_t mod
 }
 
 int read_device_err(Ctx* ctx, const char* what) {
-    if (!ctx->d_err) return YAO_OK;
     int herr = 0;
+    ctx->err_unread.store(false);
     YAO_CUDA(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     YAO_CUDA(cudaStreamSynchronize(ctx->stream));
     if (!herr) return YAO_OK;
     YAO_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     return fail(YAO_ERR_TIMEOUT, std::string(what) + ": a bounded wait of a kernel gave up");
+}
+
+int wait_results(Ctx* ctx, const char* what) {
+    if (ctx->err_unread.load()) return read_device_err(ctx, what);
+    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
+    return YAO_OK;
 }
 
 int plan_info(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int32_t mode, int32_t k,

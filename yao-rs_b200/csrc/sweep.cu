@@ -977,8 +977,8 @@ int sweep_batch(Ctx* ctx, const SweepPlan* p, const std::vector<MonoTerm>& terms
         cudaMemcpyAsync(grads, r.grads, nsets * p->np * 8, cudaMemcpyDeviceToHost, ctx->stream);
     }
     cudaFreeAsync(st, ctx->stream);
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
-    return s;
+    const int ws = wait_results(ctx, "expect_grad_batch");
+    return s ? s : ws;
 }
 
 }  // namespace yao

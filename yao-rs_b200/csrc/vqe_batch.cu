@@ -483,8 +483,9 @@ int expect_grad_batch(Ctx* ctx, const std::vector<MonoTerm>& terms, const Circui
     if (np) YAO_CUDA(cudaMemcpyAsync(grads, dgrad, nsets * np * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     if (!hv.empty())
         YAO_CUDA(cudaMemcpyAsync(hv.data(), dvals, hv.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->stream));
-    YAO_CUDA(cudaStreamSynchronize(ctx->stream));
     YAO_CUDA(cudaFreeAsync(buf, ctx->stream));
+    const int ws = wait_results(ctx, "expect_grad_batch");
+    if (ws) return ws;
     for (size_t set = 0; set < nsets; set++) {
         double re = 0.0;
         for (size_t t = 0; t < terms.size(); t++) {

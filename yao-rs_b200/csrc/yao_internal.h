@@ -142,6 +142,9 @@ struct Ctx {
     uint64_t launches = 0;
     // device word a kernel sets when one of its bounded waits gave up
     int* d_err = nullptr;
+    // work that may set it was queued and nobody has read it since: the next
+    // call that waits for results does (wait_results)
+    std::atomic<bool> err_unread{false};
     // the last TILED / FUSED run put some blocks on the tensor cores
     bool tc_used = false;
     // tables of the batched launch (device and pinned host copies), kept and
@@ -209,6 +212,8 @@ int launch_gate(Ctx* ctx, void* state, int32_t precision, uint32_t nbits, const 
 int launch_program(Ctx* ctx, Reg* r, const std::vector<LGate>& prog, int32_t mode, int32_t k, bool check_err = true);
 // Synchronises, and turns a set error word into YAO_ERR_TIMEOUT (clearing it)
 int read_device_err(Ctx* ctx, const char* what);
+// Synchronises, with read_device_err where queued work left the word unread.
+int wait_results(Ctx* ctx, const char* what);
 // Time TILED / FUSED candidates for this program and register (always
 // re-tunes); out = {k, tile bits, register bits}.
 int autotune_program(Ctx* ctx, Reg* r, const std::vector<LGate>& prog, int32_t mode, int32_t k, int32_t out[4]);
