@@ -105,3 +105,34 @@ def test_plain_apply_returns_with_work_queued():
     rho.apply(layers)
     assert not stream.query()
     assert abs(rho.trace() - 1.0) < 1e-12
+
+
+def test_registers_of_two_contexts():
+    """A mixture and a difference of registers of two contexts wait for the
+    work queued on both, and memory freed afterwards is used again only once
+    it has been read."""
+    lib, n = A.lib(), 11
+    ctx = C.c_void_p()
+    A.check(lib.yao_ctx_create(0, C.byref(ctx)))
+    c = layered_circuit(n, 400, seed=2)  # some milliseconds of work
+    ref = Y.ArrayReg.zero_state(n)
+    Y.apply_inplace(c, ref)
+    want = Y.DensityMatrix.from_reg(ref).state_data().ravel()
+    for _ in range(3):
+        other, zero, rho = C.c_void_p(), C.c_void_p(), C.c_void_p()
+        A.check(lib.yao_reg_zero_state(ctx, n, Y.C128, C.byref(other)))
+        A.check(lib.yao_apply_inplace(c.handle, other))
+        weights, regs = (C.c_double * 1)(1.0), (C.c_void_p * 1)(other)
+        A.check(lib.yao_dm_mixed(A.context(0), weights, regs, 1, C.byref(rho)))
+        lib.yao_reg_free(other)
+        A.check(lib.yao_reg_zero_state(ctx, n, Y.C128, C.byref(zero)))  # the freed memory
+        got = np.zeros(1 << (2 * n), dtype=np.complex128)
+        A.check(lib.yao_dm_to_host(rho, got.ctypes.data_as(A.dptr)))
+        assert np.max(np.abs(got - want)) < 1e-15
+        A.check(lib.yao_apply_inplace(c.handle, zero))
+        diff = C.c_double()
+        A.check(lib.yao_reg_max_abs_diff(ref.handle, zero, C.byref(diff)))
+        assert diff.value == 0.0
+        lib.yao_reg_free(zero)
+        lib.yao_dm_free(rho)
+    A.check(lib.yao_ctx_destroy(ctx))

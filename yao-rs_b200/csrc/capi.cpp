@@ -400,6 +400,18 @@ static int check_measure_locs(uint32_t nbits, const uint32_t* locs, uint32_t n) 
     return YAO_OK;
 }
 
+// Work that `after` queues from now on runs after what `before` has queued.
+static int order_contexts(const Ctx* before, const Ctx* after) {
+    if (before == after) return YAO_OK;
+    YAO_CUDA(cudaSetDevice(before->device));
+    cudaEvent_t e;
+    YAO_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaError_t r = cudaEventRecord(e, before->stream);
+    if (r == cudaSuccess) r = cudaStreamWaitEvent(after->stream, e, 0);
+    cudaEventDestroy(e);  // (freed once the wait is over)
+    return r == cudaSuccess ? YAO_OK : cuda_fail(r, "order of two contexts");
+}
+
 static Cx cxmul(Cx a, Cx b) { return Cx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 
 }  // namespace yao
@@ -869,6 +881,8 @@ int yao_reg_max_abs_diff(const yao_reg* a, const yao_reg* b, double* out) {
     CHECK_NULL(b);
     CHECK_NULL(out);
     if (a->nbits != b->nbits) return fail(YAO_ERR_NBITS_MISMATCH, "registers with different qubit counts");
+    const int s = order_contexts(b->ctx, a->ctx);
+    if (s) return s;
     YAO_CUDA(cudaSetDevice(a->ctx->device));
     return reduce_max_abs_diff(a->ctx, a, b, out);
 }
@@ -1063,7 +1077,13 @@ int yao_dm_mixed(yao_ctx* ctx, const double* weights, const yao_reg* const* regs
     int s = alloc_dm(ctx, nb, &d);
     if (s) return s;
     YAO_CUDA(cudaMemsetAsync(d->d, 0, d->bytes(), ctx->stream));
+    // registers of other contexts: read after what their streams hold, and
+    // used again (or their memory, once freed) after the reads
+    for (size_t i = 0; i < n && !s; i++) s = order_contexts(regs[i]->ctx, ctx);
+    YAO_CUDA(cudaSetDevice(ctx->device));
     for (size_t i = 0; i < n && !s; i++) s = launch_dm_mixed_accum(ctx, regs[i], weights[i], d);
+    for (size_t i = 0; i < n && !s; i++) s = order_contexts(ctx, regs[i]->ctx);
+    YAO_CUDA(cudaSetDevice(ctx->device));
     *out = static_cast<yao_dm*>(d);
     return s;
 }
