@@ -3,6 +3,9 @@
 //                          1-qubit matrices change the squared norm, minus
 //                          that of the gates it was made from (layers of Rx,
 //                          Ry, Rz on N qubits and a CNOT brickwork)
+//   plans supported        whether a pass takes a rotation, a matrix without
+//                          targets, a swap of a qubit with itself, a control
+//                          given twice
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -56,6 +59,28 @@ int main(int argc, char** argv) {
         std::vector<LGate> split;
         split_single_qubit(prog, n, split);
         printf("%zu %.6Le\n", split.size(), log_norm(split) - log_norm(prog));
+        return 0;
+    }
+    if (argc == 2 && !strcmp(argv[1], "supported")) {
+        GateElem one, swap, twice;
+        one.type = YAO_GATE_CUSTOM;
+        one.custom_dim = 1;
+        one.custom = {Cx{0.0, 1.0}};
+        swap.type = YAO_GATE_SWAP;
+        swap.targets = {2, 2};
+        twice.type = YAO_GATE_X;
+        twice.targets = {0};
+        twice.ctrls = {1, 1};
+        twice.cfgs = {1, 1};
+        std::vector<LGate> prog;
+        gate(prog, 6, YAO_GATE_RY, 3, 0.4);
+        printf("%d", reg_supported(prog, 6));
+        for (const GateElem* g : {&one, &swap, &twice}) {
+            std::vector<LGate> with(prog);
+            lower_gate(*g, 6, 0, false, with);
+            printf(" %d", reg_supported(with, 6));
+        }
+        puts("");
         return 0;
     }
     return 1;

@@ -8,7 +8,7 @@ import pytest
 import oracle as O
 import yao_rs as Y
 from helpers import random_state
-from yao_rs import Gate, NoiseChannel as N
+from yao_rs import Gate, NoiseChannel as N, _abi as A
 
 ONE = [N.AmplitudeDamping(0.1, 0.0), N.AmplitudeDamping(0.1, 0.3), N.PhaseDamping(0.2), N.BitFlip(0.1),
        N.PauliChannel(0.1, 0.05, 0.02), N.Reset(0.1, 0.05), N.PhaseAmplitudeDamping(0.1, 0.1, 0.2),
@@ -72,3 +72,15 @@ def test_sixteen_amplitudes_a_thread():
     fused.apply(c, Y.MODE_FUSED)
     assert np.array_equal(run.state_data(), steps.state_data())
     assert np.abs(fused.state_data() - run.state_data()).max() < 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ops", [[np.eye(2) * 0.25] * 17, [np.array([[0.5]])]])
+def test_channels_that_are_refused(ops):
+    """More than 16 Kraus operators, and none of the qubits: refused by PLAIN
+    wherever they stand."""
+    locs = [1] if ops[0].shape[0] == 2 else []
+    c = Y.Circuit.qubits(4, [Y.put([0], Gate.H), Y.channel(locs, N.Custom(ops))] * 2)
+    with pytest.raises(Y.YaoError) as e:
+        Y.DensityMatrix.from_reg(Y.ArrayReg.zero_state(4)).apply(c)
+    assert e.value.status == A.YAO_ERR_UNSUPPORTED

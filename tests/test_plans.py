@@ -37,3 +37,8 @@ def test_split_program_keeps_the_norm(plans, n, layers):
     count, off = plans("norm", n, layers).split()
     assert int(count) > n * layers
     assert abs(float(off)) < 1e-15
+
+
+def test_gates_without_targets_or_with_a_qubit_twice_are_not_planned(plans):
+    """They are left to the passes of one gate."""
+    assert plans("supported").split() == ["1", "0", "0", "0"]

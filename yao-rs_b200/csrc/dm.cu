@@ -209,7 +209,6 @@ int launch_dm_gate(Ctx* ctx, DM* d, const LGate& row, const LGate& col) {
 
 // ---------------------------------------------------------- channel pass
 
-constexpr int kMaxKraus = 16;
 constexpr int kDCT = 128;  // channel kernel block size
 // A channel pass's description travels in the kernel parameters (about
 // 8.7 KB: no allocation and no copy per launch).  `mono[q]`: Kraus operator q

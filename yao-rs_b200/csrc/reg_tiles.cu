@@ -873,7 +873,12 @@ static uint64_t need_mask(const LGate& g, bool exact) {
 static bool is_perm(const LGate& g) { return g.cls == GC_X || g.cls == GC_SWAP; }
 
 static bool reg_width(uint32_t nbits) { return nbits >= 4 && nbits <= 33; }
-static bool reg_gate(const LGate& g) { return !((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1)); }
+// (Gates without a target, or with a qubit twice, are left to the passes of
+// one gate, which refuse them or give them a meaning.)
+static bool reg_gate(const LGate& g) {
+    if (g.k < 1 || __builtin_popcountll(qubit_mask(g)) != g.k + g.nc) return false;
+    return !((g.cls == GC_DENSE && g.k > 2) || (g.cls == GC_X && g.k != 1));
+}
 // steps on two qubits of a density matrix: all four register positions
 static bool four_bits(const LGate& g) { return g.cls == GC_CHAN2 || g.cls == GC_PAULI2; }
 
@@ -2179,7 +2184,7 @@ static bool kraus_step(const std::vector<DMStep>& steps, size_t at, std::vector<
     }
     if (s.rows.empty()) return false;
     const int k = s.rows[0].k, nl = 1 << k;
-    if (k > 2) return false;
+    if (k < 1 || k > 2 || s.rows.size() > (size_t)kMaxKraus) return false;
     g = dm_gate_on(s, k == 1 ? GC_CHAN1 : GC_CHAN2, k);
     for (size_t q = 0; q < s.rows.size(); q++) {
         int src[4];
@@ -2334,7 +2339,7 @@ int dm_fused_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps, bool* done) 
         auto at = [&](const LGate& g, int r, int c) {
             return g.cls == GC_X ? Cx{r != c ? 1.0 : 0.0, 0.0} : entry_of(g, r, c);
         };
-        if (k > 2) return YAO_OK;
+        if (k < 1 || k > 2) return YAO_OK;
         // S[(a, b), (c, e)] = sum_q K_q[a][c] conj(K_q)[b][e], (a, b) at b + nl a
         std::vector<Cx> S((size_t)nl * nl * nl * nl, Cx{0.0, 0.0});
         for (size_t q = 0; q < s.rows.size(); q++)

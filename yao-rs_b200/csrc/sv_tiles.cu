@@ -2432,7 +2432,7 @@ static int tune_program(Ctx* ctx, const Reg* r, const std::vector<LGate>& prog, 
     } else if (kreq <= 2) {
         std::vector<LGate> w2;
         fuse_blocks(prog, n, 2, w2);
-        reg = reg_supported(w2, n);
+        reg = reg_supported(w2, n) && reg_supported(prog, n);  // fused, and kept apart
     }
     std::vector<TileConfig> forms;
     if (reg) {

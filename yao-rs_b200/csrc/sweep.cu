@@ -480,6 +480,12 @@ static bool real_matrix(const SFactor& f) {
     return f.m[0].y == 0 && f.m[1].y == 0 && f.m[2].y == 0 && f.m[3].y == 0;
 }
 
+static uint64_t target_bits(const LGate& l) {
+    uint64_t m = 0;
+    for (int q = 0; q < l.k; q++) m |= 1ull << l.tb[q];
+    return m;
+}
+
 // U^dagger U = 1 to the rounding of the entries.  The steps of a sweep change
 // places on disjoint qubits: a dot of lambda and psi stays the same under a
 // matrix on another qubit when that matrix is unitary, else it does not.
@@ -736,6 +742,7 @@ SweepPlan* sweep_plan_new(const Circuit* c, uint32_t n) {
                 pend[l.tb[0]].push_back(f);
                 continue;
             }
+            if (__builtin_popcountll(l.cmask() | target_bits(l)) != l.k + l.nc) return nullptr;  // a qubit twice
             Item it;
             it.k = l.k;
             for (int q = 0; q < l.k && q < 2; q++) it.tb[q] = l.tb[q];

@@ -36,6 +36,8 @@ int cuda_fail(cudaError_t e, const char* what);
 constexpr int kMaxQubits = 34;
 // Largest number of targets of one lowered gate (2^6 x 2^6 matrix).
 constexpr int kMaxTargets = 6;
+// Largest number of Kraus operators of a channel summed operator by operator.
+constexpr int kMaxKraus = 16;
 
 // ------------------------------------------------------------------ gates
 // A gate after dispatch_arrayreg_gate's decision (yao-rs src/apply.rs:7-120),
