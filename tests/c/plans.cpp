@@ -3,9 +3,14 @@
 //                          1-qubit matrices change the squared norm, minus
 //                          that of the gates it was made from (layers of Rx,
 //                          Ry, Rz on N qubits and a CNOT brickwork)
+//   plans time N BITS WHAT GATES
+//                          seconds to plan GATES gates on the first N of BITS
+//                          qubits (and, with "last", one on the next qubit at
+//                          the end): WHAT = exact, fused, last, sweep
 //   plans supported        whether a pass takes a rotation, a matrix without
 //                          targets, a swap of a qubit with itself, a control
 //                          given twice
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -13,6 +18,7 @@
 #include <random>
 
 #include "reg_tiles.h"
+#include "sweep.h"
 
 using namespace yao;
 
@@ -52,7 +58,46 @@ static long double log_norm(const std::vector<LGate>& prog) {
     return sum;
 }
 
+static double seconds(uint32_t n, uint32_t nbits, const char* what, size_t gates) {
+    std::mt19937_64 r(1);
+    std::uniform_real_distribution<double> angle(0.0, 6.283185307179586);
+    std::vector<LGate> prog;
+    Circuit c;
+    for (size_t i = 0; i < gates; i++) {
+        const uint32_t t = (uint32_t)(r() % n), k = (t + 1 + (uint32_t)(r() % (n - 1))) % n;
+        GateElem g;
+        g.type = i % 4 == 3 ? YAO_GATE_X : YAO_GATE_RY;
+        g.targets = {t};
+        g.params[0] = angle(r);
+        if (i % 4 == 3) {
+            g.ctrls = {k};
+            g.cfgs = {1};
+        }
+        Element e;
+        e.g = g;
+        c.elems.push_back(e);
+        lower_gate(g, nbits, 0, false, prog);
+    }
+    if (!strcmp(what, "last")) gate(prog, nbits, YAO_GATE_RY, n, 0.5);
+    double best = 1e9;
+    for (int i = 0; i < 3; i++) {
+        const auto t0 = std::chrono::steady_clock::now();
+        if (!strcmp(what, "sweep")) {
+            sweep_plan_free(sweep_plan_new(&c, nbits));
+        } else {
+            RegPlan plan;
+            reg_plan(prog, nbits, YAO_C128, 11, strcmp(what, "fused") != 0, plan);
+        }
+        best = std::min(best, std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
+    }
+    return best;
+}
+
 int main(int argc, char** argv) {
+    if (argc == 6 && !strcmp(argv[1], "time")) {
+        printf("%.6f\n", seconds((uint32_t)atoi(argv[2]), (uint32_t)atoi(argv[3]), argv[4], (size_t)atoll(argv[5])));
+        return 0;
+    }
     if (argc == 4 && !strcmp(argv[1], "norm")) {
         const uint32_t n = (uint32_t)atoi(argv[2]);
         const std::vector<LGate> prog = layered(n, atoi(argv[3]));

@@ -42,3 +42,12 @@ def test_split_program_keeps_the_norm(plans, n, layers):
 def test_gates_without_targets_or_with_a_qubit_twice_are_not_planned(plans):
     """They are left to the passes of one gate."""
     assert plans("supported").split() == ["1", "0", "0", "0"]
+
+
+# four times the gates: four times the time, twice that allowed (16 times and
+# more where every scan runs to the program's end)
+@pytest.mark.parametrize("n,nbits,what", [(13, 13, "exact"), (13, 14, "exact"), (13, 14, "last"), (13, 14, "fused"),
+                                          (8, 9, "exact"), (24, 30, "fused"), (13, 14, "sweep"), (8, 9, "sweep")])
+def test_planning_time_is_linear(plans, n, nbits, what):
+    few, many = (float(plans("time", n, nbits, what, gates)) for gates in (20000, 80000))
+    assert many < 8.0 * few, (few, many)

@@ -889,20 +889,34 @@ bool reg_supported(const std::vector<LGate>& prog, uint32_t nbits) {
     return true;
 }
 
+// What the scans below ask of a gate: its qubits, the bits it needs in the
+// tile, whether it only moves amplitudes.
+struct GateBits {
+    uint64_t qubits, need;
+    bool perm;
+};
+
 // Which gates of a list may be taken next, scanning it in order: a gate
 // passes skipped ones only when it shares no qubit with them (and, for an
-// exact result, it or all of them are permutations).
+// exact result, it or all of them are permutations).  A scan ends where no
+// gate can pass any more, or after kScanSkipped skipped ones: a qubit that no
+// gate touches for long would keep every scan going to the end of the program
+// (80000 gates on 14 qubits, one of them idle: planned in 1.5 s).
+constexpr size_t kScanSkipped = 1024;
+
 struct Scan {
     bool exact;
     uint64_t blocked = 0;
+    size_t skipped = 0;
     bool arith = false;  // some skipped gate computes
     explicit Scan(bool e) : exact(e) {}
-    bool free(const LGate& g) const { return !(qubit_mask(g) & blocked) && (!exact || !arith || is_perm(g)); }
-    void skip(const LGate& g) {
-        blocked |= qubit_mask(g);
-        arith |= !is_perm(g);
+    bool free(const GateBits& g) const { return !(g.qubits & blocked) && (!exact || !arith || g.perm); }
+    void skip(const GateBits& g) {
+        blocked |= g.qubits;
+        arith |= !g.perm;
+        skipped++;
     }
-    bool closed(uint64_t all) const { return (blocked & all) == all; }
+    bool closed(uint64_t all) const { return (blocked & all) == all || skipped >= kScanSkipped; }
 };
 
 static Cx cmul(Cx a, Cx b) { return Cx{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
@@ -1742,8 +1756,15 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     const int low = precision == YAO_C128 ? 3 : 4;  // 128-byte runs: the tile's lowest bits
     const int tbits = std::min((int)nbits, tbits_max);
     const bool whole = (int)nbits <= tbits;
-    const uint64_t lowmask = whole ? 0 : ((1ull << low) - 1), all = (1ull << nbits) - 1;
+    const uint64_t lowmask = whole ? 0 : ((1ull << low) - 1);
     const int cap = whole ? (int)nbits : tbits - low;
+    const size_t blob_cap = precision == YAO_C128 ? kRegBlobCap : kRegBlobCap64;
+    std::vector<GateBits> bits(ngates);
+    uint64_t all = 0;  // the bits that gates touch
+    for (size_t i = 0; i < ngates; i++) {
+        bits[i] = GateBits{qubit_mask(prog[i]), need_mask(prog[i], exact), is_perm(prog[i])};
+        all |= bits[i].qubits;
+    }
     // Amplitudes a thread: 16 once the tiles fill the GPU twice over, else 4
     // (8 in a 2^12 tile: at most 512 threads), which shortens an op's chain
     // where the time of one CTA is the time of the pass.
@@ -1756,23 +1777,20 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     std::vector<char> used(ngates, 0);
     size_t i0 = 0, left = ngates;
     while (left) {
-        // the gates of this pass
-        std::vector<const LGate*> run;
-        std::vector<size_t> at;
+        // the gates of this pass (at most twice what its description holds)
+        std::vector<size_t> run;
         uint64_t hi = 0;
         {
             Scan sc(exact);
-            for (size_t j = i0; j < ngates && !sc.closed(all); j++) {
+            for (size_t j = i0; j < ngates && !sc.closed(all) && run.size() < 2 * blob_cap / sizeof(ROp); j++) {
                 if (used[j]) continue;
-                const LGate& g = prog[j];
-                const uint64_t nh = hi | (need_mask(g, exact) & ~lowmask);
-                if (!sc.free(g) || __builtin_popcountll(nh) > cap) {
-                    sc.skip(g);
+                const uint64_t nh = hi | (bits[j].need & ~lowmask);
+                if (!sc.free(bits[j]) || __builtin_popcountll(nh) > cap) {
+                    sc.skip(bits[j]);
                     continue;
                 }
                 hi = nh;
-                run.push_back(&g);
-                at.push_back(j);
+                run.push_back(j);
             }
         }
         uint64_t tile = hi | lowmask;
@@ -1808,9 +1826,9 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
             bool full = false;
             for (size_t j = first; j < run.size() && !full && !sc.closed(all); j++) {
                 if (done[j]) continue;
-                const LGate& g = *run[j];
-                if (!sc.free(g) || !pb.fits(s, g)) {
-                    sc.skip(g);
+                const LGate& g = prog[run[j]];
+                if (!sc.free(bits[run[j]]) || !pb.fits(s, g)) {
+                    sc.skip(bits[run[j]]);
                     continue;
                 }
                 // a diagonal may become one op per combination of its register targets
@@ -1819,7 +1837,7 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
                 const size_t more = !exact && rb == 4 && g.cls == GC_DENSE && g.k == 1 ? 3 * coef_bytes : 0;
                 const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) + more +
                                   (g.cls >= GC_CHAN1 ? std::min<size_t>(g.m.size(), 4) : g.m.size()) * coef_bytes;
-                if (bytes + nb > (precision == YAO_C128 ? kRegBlobCap : kRegBlobCap64) && !(p.ops.empty() && s.gates.empty())) {
+                if (bytes + nb > blob_cap && !(p.ops.empty() && s.gates.empty())) {
                     full = true;
                     break;
                 }
@@ -1836,7 +1854,7 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
         }
         for (size_t j = 0; j < run.size(); j++)
             if (done[j]) {
-                used[at[j]] = 1;
+                used[run[j]] = 1;
                 left--;
             }
         while (i0 < ngates && used[i0]) i0++;

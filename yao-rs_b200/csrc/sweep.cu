@@ -42,6 +42,7 @@ constexpr int kSThreads = 1 << (kSTile - kSB);
 constexpr int kSLow = 3;               // 128-byte runs
 constexpr int kSMaxRuns = 40;          // runs of a pass (their sums and matrices in shared memory)
 constexpr int kSMaxOps = 160;          // ops of a pass
+constexpr int kSMaxSkipped = 1024;     // steps a pass's scan skips: an idle qubit does not take it to the circuit's end
 
 enum SCode : uint32_t {
     SC_RUN = 0,    // + position: the run's matrix (and sums); pairs in the mask swap first where the controls match
@@ -505,21 +506,24 @@ static bool unitary(const SFactor& f) {
 static void plan_items(const std::vector<const Item*>& items, uint32_t n, bool back, std::vector<SPass>& out) {
     const int tbits = std::min<int>((int)n, kSTile);
     const bool whole = (int)n <= tbits;
-    const uint64_t lowmask = whole ? 0 : (1ull << kSLow) - 1, all = (1ull << n) - 1;
+    const uint64_t lowmask = whole ? 0 : (1ull << kSLow) - 1;
+    uint64_t all = 0;  // the bits that steps touch
+    for (const Item* it : items) all |= it->qubits;
     const int cap = whole ? (int)n : tbits - kSLow;
     std::vector<char> used(items.size(), 0);
     size_t first = 0, left = items.size();
     while (left) {
         uint64_t hi = 0, blocked = 0;
         std::vector<size_t> take;
-        int nruns = 0;
-        for (size_t j = first; j < items.size() && (blocked & all) != all; j++) {
+        int nruns = 0, skipped = 0;
+        for (size_t j = first; j < items.size() && (blocked & all) != all && (int)take.size() < kSMaxOps && skipped < kSMaxSkipped;
+             j++) {
             if (used[j]) continue;
             const Item& it = *items[j];
             const uint64_t nh = hi | (it.need & ~lowmask);
-            if ((it.qubits & blocked) || __builtin_popcountll(nh) > cap || (int)take.size() >= kSMaxOps ||
-                (it.kind == IT_RUN && nruns >= kSMaxRuns)) {
+            if ((it.qubits & blocked) || __builtin_popcountll(nh) > cap || (it.kind == IT_RUN && nruns >= kSMaxRuns)) {
                 blocked |= it.qubits;
+                skipped++;
                 continue;
             }
             hi = nh;
