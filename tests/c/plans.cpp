@@ -7,6 +7,9 @@
 //                          seconds to plan GATES gates on the first N of BITS
 //                          qubits (and, with "last", one on the next qubit at
 //                          the end): WHAT = exact, fused, last, sweep
+//   plans sizes            the largest description of a pass in bytes: 300
+//                          different 2-qubit channels on 8 bits, phases between
+//                          register bits and bits outside the tile on 24
 //   plans supported        whether a pass takes a rotation, a matrix without
 //                          targets, a swap of a qubit with itself, a control
 //                          given twice
@@ -104,6 +107,50 @@ int main(int argc, char** argv) {
         std::vector<LGate> split;
         split_single_qubit(prog, n, split);
         printf("%zu %.6Le\n", split.size(), log_norm(split) - log_norm(prog));
+        return 0;
+    }
+    if (argc == 2 && !strcmp(argv[1], "sizes")) {
+        std::mt19937_64 r(1);
+        std::uniform_real_distribution<double> x(0.0, 1.0);
+        std::vector<LGate> channels, phases;
+        for (int i = 0; i < 300; i++) {
+            LGate g;
+            g.cls = GC_CHAN2;
+            g.k = 4;
+            for (int q = 0; q < 2; q++) {
+                g.tb[2 * q] = i < 150 ? q : q + 1;
+                g.tb[2 * q + 1] = 4 + g.tb[2 * q];
+            }
+            for (int op = 0; op < 16; op++) {
+                const uint32_t type = (uint32_t)(op & 3);
+                Cx head{0.0, 0.0};
+                memcpy(&head.re, &type, 4);
+                g.m.push_back(head);
+                for (int j = 0; j < 4; j++) g.m.push_back(Cx{x(r), x(r)});
+            }
+            channels.push_back(g);
+        }
+        for (uint32_t q = 0; q < 24; q++) gate(phases, 24, YAO_GATE_RY, q, x(r));
+        for (int i = 0; i < 300; i++) {
+            LGate g;
+            g.cls = GC_DIAG;
+            g.k = 1;
+            g.tb[0] = (int)(r() % 7);
+            g.nc = 1;
+            g.cb[0] = 11 + i % 13;
+            g.cv[0] = 1;
+            const double t = x(r);
+            g.m = {Cx{1.0, 0.0}, Cx{std::cos(t), std::sin(t)}};
+            phases.push_back(g);
+        }
+        RegPlan plan;
+        for (auto* prog : {&channels, &phases}) {
+            reg_plan(*prog, prog == &channels ? 8 : 24, YAO_C128, 11, prog == &channels, plan);
+            size_t most = 0;
+            for (const RegPass& p : plan.passes) most = std::max(most, p.blob_bytes);
+            printf("%zu ", most);
+        }
+        puts("");
         return 0;
     }
     if (argc == 2 && !strcmp(argv[1], "supported")) {

@@ -84,3 +84,23 @@ def test_channels_that_are_refused(ops):
     with pytest.raises(Y.YaoError) as e:
         Y.DensityMatrix.from_reg(Y.ArrayReg.zero_state(4)).apply(c)
     assert e.value.status == A.YAO_ERR_UNSUPPORTED
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 6])
+def test_channels_that_all_differ(n):
+    """As in a calibrated noise model: their coefficients fill several passes."""
+    rng = np.random.default_rng(n)
+    els = []
+    for i in range(60):
+        p = [int(x) for x in rng.permutation(n)]
+        els += [Y.channel(p[:2] if i % 3 else [0, 1], N.Depolarizing(2, float(rng.uniform(0, 0.1)))),
+                Y.channel([p[0]], N.PauliChannel(*rng.uniform(0, 0.1, 3))), Y.put([p[1]], Gate.Ry(rng.uniform(-3, 3)))]
+    c, psi = Y.Circuit.qubits(n, els), random_state(rng, n)
+    ref = O.dm_apply_circuit(c, O.dm_from_reg(psi, n)).ravel()
+    plain, fused = (Y.DensityMatrix.from_reg(Y.ArrayReg.from_vec(n, psi)) for _ in range(2))
+    plain.apply(c)
+    fused.apply(c, Y.MODE_FUSED)
+    assert np.array_equal(plain.state_data(), ref)
+    # 180 steps of 1e-16 each on entries of magnitude 1 at most
+    assert np.abs(fused.state_data() - ref).max() < 1e-13

@@ -51,3 +51,9 @@ def test_gates_without_targets_or_with_a_qubit_twice_are_not_planned(plans):
 def test_planning_time_is_linear(plans, n, nbits, what):
     few, many = (float(plans("time", n, nbits, what, gates)) for gates in (20000, 80000))
     assert many < 8.0 * few, (few, many)
+
+
+def test_descriptions_fit(plans):
+    """8 KiB a pass (three CTAs an SM), with 16 bytes for one more segment."""
+    sizes = [int(x) for x in plans("sizes").split()]
+    assert len(sizes) == 2 and max(sizes) <= 8192 + 16

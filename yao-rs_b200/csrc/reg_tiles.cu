@@ -1831,8 +1831,8 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
                     sc.skip(bits[run[j]]);
                     continue;
                 }
-                // a diagonal may become one op per combination of its register targets
-                // (channels: once a pass, mostly)
+                // a diagonal may become one op per combination of its register targets;
+                // a channel's coefficients are there already, mostly
                 // (a layer of four matrices: their reals and a diagonal)
                 const size_t more = !exact && rb == 4 && g.cls == GC_DENSE && g.k == 1 ? 3 * coef_bytes : 0;
                 const size_t nb = (g.cls == GC_DIAG ? std::min<size_t>(1u << g.k, 16) : 1) * sizeof(ROp) + more +
@@ -1846,7 +1846,23 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
                 took.push_back(j);
             }
             if (took.empty()) break;  // the description is full
+            // The count above is a guess: a diagonal may bring a table, a
+            // channel more coefficients.  Without its last gates the segment
+            // fits (a gate alone always does).
+            const size_t segs0 = p.segs.size(), ops0 = p.ops.size(), coef0 = p.coef.size(), shared0 = pb.shared.size();
             pb.emit(s);
+            while (pass_bytes(p, coef_bytes) > blob_cap && (took.size() > 1 || ops0 > 0)) {
+                p.segs.resize(segs0);
+                p.ops.resize(ops0);
+                p.coef.resize(coef0);
+                pb.shared.resize(shared0);
+                full = true;
+                took.resize(took.size() * 3 / 4);
+                if (took.empty()) break;
+                s = SegPlan();
+                for (size_t j : took) pb.add(s, prog[run[j]]);
+                pb.emit(s);
+            }
             for (size_t j : took) done[j] = 1;
             ndone += took.size();
             while (first < run.size() && done[first]) first++;
