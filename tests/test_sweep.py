@@ -1,6 +1,11 @@
 """Gradients by the register sweep (csrc/sweep.cu), of one and of several
 parameter vectors, against the oracle at register counts around its tile
 and thread edges."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -137,3 +142,34 @@ def test_several_tiles_a_unit(n, monkeypatch):
     value, grad = Y.expect_grad(h, c, reg)
     for got_v, got_g in ((v, g), (vs[0], gs[0]), (vs[1], gs[1])):
         assert abs(got_v - value) < 1e-12 and np.max(np.abs(np.array(got_g) - np.array(grad))) < 1e-12
+
+
+MEMORY = """
+import numpy as np, torch
+import yao_rs as Y
+from helpers import tfim, vqe_ansatz
+n, depth, nsets = 4, 100, 20000
+c, h, reg = vqe_ansatz(n, depth, np.zeros(2 * n * depth)), tfim(n), Y.ArrayReg.zero_state(n)
+sets = np.random.default_rng(0).uniform(-3, 3, size=(nsets, c.num_params()))
+Y.expect_grad_batch(h, c, sets[:4], reg)
+before = torch.cuda.mem_get_info(0)[0]
+vs, gs = Y.expect_grad_batch(h, c, sets, reg)
+print(before - torch.cuda.mem_get_info(0)[0])
+for s in (0, 4095, 19999):
+    c.dispatch(list(sets[s]))
+    v, g = Y.expect_grad(h, c, reg)
+    assert abs(v - vs[s]) < 1e-11 and np.max(np.abs(np.array(g) - gs[s])) < 1e-11
+"""
+
+
+@pytest.mark.gpu
+def test_memory_of_many_sets_and_runs():
+    """800 parameters in 400 runs, 20000 sets: parameters and gradients are
+    128 MB each, and what the sweep needs stays below 64 + 256 MB (matrices
+    and sums of all sets at once would be 1.3 GB)."""
+    pytest.importorskip("torch")
+    root = Path(__file__).resolve().parent.parent
+    env = dict(os.environ, PYTHONPATH=f"{root / 'yao-rs_b200'}:{root / 'tests'}")
+    r = subprocess.run([sys.executable, "-c", MEMORY], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert int(r.stdout.split()[0]) < 700e6
