@@ -4,6 +4,7 @@ and thread edges."""
 import os
 import subprocess
 import sys
+import time
 from pathlib import Path
 
 import numpy as np
@@ -173,3 +174,21 @@ def test_memory_of_many_sets_and_runs():
     r = subprocess.run([sys.executable, "-c", MEMORY], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert int(r.stdout.split()[0]) < 700e6
+
+
+@pytest.mark.gpu
+def test_two_large_sets_cost_what_two_calls_cost():
+    """24 qubits: no part of a batch runs on one SM (the energy alone took
+    eight times the gradient)."""
+    n = 24
+    c, h = ansatz(np.random.default_rng(0), n, 1, 0), hamiltonian(n)
+    reg, sets = Y.ArrayReg.zero_state(n), np.array([c.parameters()] * 2)
+
+    def best(f):
+        times = []
+        for _ in range(4):
+            t = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t)
+        return min(times)
+    assert best(lambda: Y.expect_grad_batch(h, c, sets, reg)) < 4.0 * best(lambda: Y.expect_grad(h, c, reg))

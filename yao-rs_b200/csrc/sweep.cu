@@ -422,14 +422,26 @@ __global__ void k_sweep_grads(const SFactor* __restrict__ fac, const SRunDev* __
     }
 }
 
-// values[set] = Re <psi_s|lambda_s>
+// Re <psi_s|lambda_s>, `per` blocks a set: the sum of block b is set b / per's
 __global__ void __launch_bounds__(256) k_sweep_energy(const double2* __restrict__ psi, const double2* __restrict__ lam,
-                                                      uint64_t n, double* __restrict__ values) {
+                                                      uint64_t n, uint32_t per, double* __restrict__ sums) {
     __shared__ double sm[8];
-    const double2 *p = psi + blockIdx.x * n, *l = lam + blockIdx.x * n;
+    const uint64_t set = blockIdx.x / per, part = blockIdx.x % per;
+    const double2 *p = psi + set * n, *l = lam + set * n;
     double e = 0.0;
-    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) e = fma(p[i].x, l[i].x, fma(p[i].y, l[i].y, e));
-    block_sum_write(&e, 1, sm, values + blockIdx.x);
+    for (uint64_t i = part * blockDim.x + threadIdx.x; i < n; i += (uint64_t)per * blockDim.x)
+        e = fma(p[i].x, l[i].x, fma(p[i].y, l[i].y, e));
+    block_sum_write(&e, 1, sm, sums + blockIdx.x);
+}
+// values[set] from its blocks' sums, a warp a set
+__global__ void __launch_bounds__(128) k_sweep_energy_final(const double* __restrict__ sums, uint32_t per, uint32_t nsets,
+                                                            double* __restrict__ values) {
+    const uint32_t set = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (set >= nsets) return;
+    double e = 0.0;
+    for (uint32_t i = threadIdx.x & 31; i < per; i += 32) e += sums[(size_t)set * per + i];
+    e = warp_sum(e);
+    if ((threadIdx.x & 31) == 0) values[set] = e;
 }
 
 __global__ void k_sweep_broadcast(const double2* __restrict__ src, double2* __restrict__ dst, uint64_t mask, uint64_t total) {
@@ -968,13 +980,18 @@ int sweep_batch(Ctx* ctx, const SweepPlan* p, const std::vector<MonoTerm>& terms
     int s = r.init(params, nsets);
     if (s) return s;
     char* st = nullptr;
-    const size_t b_state = group * N * 16, b_val = (nsets * 8 + 255) / 256 * 256;
-    if (alloc_async(ctx, (void**)&st, 2 * b_state + b_val) != cudaSuccess) {
+    // few sets of large states: several blocks for the energy of one, 16
+    // amplitudes a thread at least (one block read both states of a set by
+    // itself: at 22 qubits 7.8 ms a set, now 0.03)
+    const uint32_t per = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>(N / 4096, (4ull * (uint64_t)ctx->num_sms + group - 1) / group));
+    const size_t b_state = group * N * 16, b_val = (nsets * 8 + 255) / 256 * 256, b_sum = group * per * 8;
+    if (alloc_async(ctx, (void**)&st, 2 * b_state + b_val + b_sum) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the batched gradient buffers");
     }
     double2 *psi = (double2*)st, *lam = (double2*)(st + b_state);
-    double* vals = (double*)(st + 2 * b_state);
+    double *vals = (double*)(st + 2 * b_state), *sums = (double*)(st + 2 * b_state + b_val);
     for (size_t f = 0; f < nsets && !s; f += group) {
         const uint32_t m = (uint32_t)std::min(group, nsets - f);
         k_sweep_broadcast<<<grid_for(m * N, 256, ctx->num_sms), 256, 0, ctx->stream>>>((const double2*)psi0->d, psi, N - 1, m * N);
@@ -982,16 +999,23 @@ int sweep_batch(Ctx* ctx, const SweepPlan* p, const std::vector<MonoTerm>& terms
         if ((s = r.coefs(f, m, true)) || (s = r.passes(false, psi, nullptr, m)) ||
             (s = build_lambda_sets(ctx, psi, lam, p->n, m, terms)))
             break;
-        k_sweep_energy<<<m, 256, 0, ctx->stream>>>(psi, lam, N, vals + f);
+        {
+            ProfScope prof(ctx, "sweep_energy", (double)m * (double)N * 32.0);
+            k_sweep_energy<<<m * per, 256, 0, ctx->stream>>>(psi, lam, N, per, per > 1 ? sums : vals + f);
+        }
         ctx->launches++;
+        if (per > 1) {
+            k_sweep_energy_final<<<(m + 3) / 4, 128, 0, ctx->stream>>>(sums, per, m, vals + f);
+            ctx->launches++;
+        }
         if (!(s = r.passes(true, psi, lam, m))) s = r.gradients(f, m);
     }
-    if (!s) {
-        cudaMemcpyAsync(values, vals, nsets * 8, cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(grads, r.grads, nsets * p->np * 8, cudaMemcpyDeviceToHost, ctx->stream);
-    }
+    cudaError_t ce = cudaGetLastError();
+    if (!s && ce == cudaSuccess) ce = cudaMemcpyAsync(values, vals, nsets * 8, cudaMemcpyDeviceToHost, ctx->stream);
+    if (!s && ce == cudaSuccess) ce = cudaMemcpyAsync(grads, r.grads, nsets * p->np * 8, cudaMemcpyDeviceToHost, ctx->stream);
     cudaFreeAsync(st, ctx->stream);
     const int ws = wait_results(ctx, "expect_grad_batch");
+    if (!s && ce != cudaSuccess) return cuda_fail(ce, "expect_grad_batch");
     return s ? s : ws;
 }
 
