@@ -418,7 +418,7 @@ def main():
     f0.record(stream)
     A.check(A.lib().yao_reg_upload(reg.handle, A.C.c_void_p(hp)))
     for i in range(args.steps):
-        Y.apply_inplace(circuits[i % LAYERS], reg)
+        apply_gates(Y, gates[i % LAYERS], reg)
     A.check(A.lib().yao_reg_to_host(reg.handle, A.C.c_void_p(hp)))
     f1.record(stream)
     f1.synchronize()
@@ -426,8 +426,21 @@ def main():
     state_bytes = 16 * (1 << n)
     e2e = {"value": job_gbps(nbytes, world, e2e_ms), "unit": "GB/s",
            "h2d_bytes_per_step": state_bytes / args.steps, "d2h_bytes_per_step": state_bytes / args.steps,
-           "note": "one state upload + one download per K steps; a layer is one apply call, which runs several gates "
-                   "a pass (bit-identical; bytes counted per gate as in value)"}
+           "note": "one state upload + one download per K steps, the gates applied one by one as in value"}
+    # the same layers with one apply call each, which runs several gates a
+    # pass (bit-identical): the passes' own bytes
+    barrier()
+    A.profile(True, dev)
+    f0.record(stream)
+    for i in range(args.steps):
+        Y.apply_inplace(circuits[i % LAYERS], reg)
+    f1.record(stream)
+    f1.synchronize()
+    shared = A.profile_report(dev)
+    A.profile(False, dev)
+    shared_ms = max_over_ranks(torch, f0.elapsed_time(f1), world, f"cuda:{dev}")
+    e2e["layer_calls"] = {"ms_per_step": shared_ms / args.steps, "passes_per_step": sum(p["launches"] for p in shared) / args.steps,
+                          "pass_GBps": job_gbps(sum(p["bytes"] for p in shared), world, shared_ms)}
     del host
 
     extras = {}

@@ -5,11 +5,14 @@ detail line, it stays short enough to survive a 3000-byte tail of stdout even
 with every float at full precision, and both arms describe the same workload."""
 import json
 import random
+import subprocess
 import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parents[1]
 sys.path.insert(0, str(ROOT))
+
+import pytest  # noqa: E402
 
 import bench  # noqa: E402
 
@@ -65,3 +68,20 @@ def test_last_line_fits_a_3000_byte_tail():
     # the driver keeps about 3000 bytes of stdout, including its own header
     # and the stderr marker
     assert len(text) < 2900, len(text)
+
+
+@pytest.mark.gpu
+def test_rates_are_rates_the_memory_has():
+    """value and e2e time the same gates, applied one by one, and neither
+    counts bytes that no pass moves: at most the measured copy rate, a tenth
+    above it for what the copy itself leaves."""
+    cmd = [sys.executable, str(ROOT / "bench.py"), "--qubits", "27", "--steps", "8", "--warmup", "3", "--no-extras",
+           "--cpu-budget", "1"]
+    r = subprocess.run(cmd, capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stderr[-2000:]
+    text = r.stdout.strip().splitlines()[-1]
+    last = json.loads(text)
+    peak = last["roofline"]["peak"]
+    assert last["value"] < 1.1 * peak and last["e2e"]["value"] < 1.1 * peak
+    assert last["e2e"]["value"] < last["value"]  # the copies of the state come on top
+    assert len(text) < 2900
