@@ -1,7 +1,11 @@
 """Memory and streams of registers: what their device address may be used
 for, where the memory of freed ones goes, calls that return with work queued."""
 import ctypes as C
+import os
+import subprocess
+import sys
 import threading
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -136,3 +140,55 @@ def test_registers_of_two_contexts():
         lib.yao_reg_free(zero)
         lib.yao_dm_free(rho)
     A.check(lib.yao_ctx_destroy(ctx))
+
+
+FULL = """
+import ctypes as C
+import numpy as np
+import yao_rs as Y
+from yao_rs import _abi as A
+from helpers import layered_circuit, tfim
+n, m = 25, 13  # registers of their own allocations
+c, op = layered_circuit(n, 1, seed=1), tfim(n)
+noisy = Y.Circuit.qubits(m, [Y.channel([q], Y.NoiseChannel.Depolarizing(1, 0.1)) for q in range(4)] * 2)
+regs = [Y.ArrayReg.zero_state(n) for _ in range(3)]
+rhos = [Y.DensityMatrix.zero_state(m) for _ in range(2)]
+for e in c.elements:  # launches of their own, and shared passes: kernels loaded
+    Y.apply_inplace(Y.Circuit.qubits(n, [e]), regs[0])
+for e in noisy.elements:
+    rhos[0].apply(Y.Circuit.qubits(m, [e]))
+Y.apply_inplace(c, regs[1])
+for x in (Y.OperatorPolynomial([1.0], [Y.OperatorString([(0, Y.Op.P0)])]), op):
+    want = Y.expect_arrayreg(regs[1], x)
+A.synchronize(0)
+cu = C.CDLL("libcuda.so.1")
+pool, held = C.c_void_p(), []
+assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0 and cu.cuMemPoolTrimTo(pool, C.c_size_t(0)) == 0
+size = 64 << 30
+while size >= 1 << 10:
+    p = C.c_uint64()
+    if cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(size)) == 0:
+        held.append(p)
+    else:
+        size //= 2
+q = C.c_void_p()
+status = A.lib().yao_reg_zero_state(A.context(0), 24, Y.C128, C.byref(q))
+Y.apply_inplace(c, regs[2])
+rhos[1].apply(noisy)
+got = Y.expect_arrayreg(regs[1], op)
+for p in held:
+    cu.cuMemFree_v2(p)
+assert regs[2].max_abs_diff(regs[1]) == 0.0 and abs(got - want) < 1e-12
+assert np.array_equal(Y.probs(rhos[1]), Y.probs(rhos[0]))
+print(status)
+"""
+
+
+def test_calls_that_need_no_memory_without_memory():
+    """PLAIN on states and density matrices and expectation values on a GPU
+    whose memory is taken: one launch a gate, a channel, a mask."""
+    root = Path(__file__).resolve().parent.parent
+    env = dict(os.environ, PYTHONPATH=f"{root / 'yao-rs_b200'}:{root / 'tests'}")
+    r = subprocess.run([sys.executable, "-c", FULL], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert int(r.stdout.split()[0]) == A.YAO_ERR_OUT_OF_MEMORY

@@ -84,7 +84,9 @@ cudaError_t alloc_async(Ctx* ctx, void** p, size_t bytes) {
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
     release_kept(ctx->device);
-    return cudaMallocAsync(p, bytes, ctx->stream);
+    e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e != cudaSuccess) cudaGetLastError();  // the caller's to report
+    return e;
 }
 
 static bool capturing(Ctx* ctx) {

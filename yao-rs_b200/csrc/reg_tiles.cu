@@ -1992,11 +1992,13 @@ static void pass_header(const RegPass& p, RHdr& h) {
 }
 
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
-               size_t step) {
+               size_t step, bool* queued) {
+    if (queued) *queued = false;
     if (plan.passes.empty()) return YAO_OK;
     unsigned char* dblob = nullptr;
     YAO_CUDA(alloc_async(ctx, (void**)&dblob, plan.blob.size()));
     YAO_CUDA(cudaMemcpyAsync(dblob, plan.blob.data(), plan.blob.size(), cudaMemcpyHostToDevice, ctx->stream));
+    if (queued) *queued = true;
     const size_t amp = precision == YAO_C128 ? 16 : 8;
     int s = YAO_OK;
     for (size_t i = first; i < plan.passes.size() && !s; i += step) {
@@ -2170,10 +2172,14 @@ int plain_run(Ctx* ctx, Reg* r, const std::vector<LGate>& prog) {
                 joint += gate_flops(prog[q]) * amps / 1e13;
             }
             if (joint < alone) {
-                int s = reg_launch(ctx, r->d, n, YAO_C128, true, plan, 0, 1);
-                if (s) return s;
-                i = end;
-                continue;
+                bool queued;
+                int s = reg_launch(ctx, r->d, n, YAO_C128, true, plan, 0, 1, &queued);
+                if (s && (queued || s != YAO_ERR_OUT_OF_MEMORY)) return s;
+                if (!s) {
+                    i = end;
+                    continue;
+                }
+                clear_error();  // no memory for the description: the launches need none
             }
         }
         for (end = std::max(i + 1, end); i < end; i++) {
@@ -2322,10 +2328,14 @@ int dm_plain_run(Ctx* ctx, DM* d, const std::vector<DMStep>& steps) {
             RegPlan plan;
             reg_plan_range(prog.data(), prog.size(), nb, YAO_C128, 11, true, plan);
             if ((double)plan.passes.size() * (8e-6 + 2.0 * bytes / 5.2e12) + flops * entries / 1e13 < alone) {
-                int s = reg_launch(ctx, d->d, nb, YAO_C128, true, plan, 0, 1);
-                if (s) return s;
-                i = end;
-                continue;
+                bool queued;
+                int s = reg_launch(ctx, d->d, nb, YAO_C128, true, plan, 0, 1, &queued);
+                if (s && (queued || s != YAO_ERR_OUT_OF_MEMORY)) return s;
+                if (!s) {
+                    i = end;
+                    continue;
+                }
+                clear_error();  // as in plain_run
             }
         }
         for (end = std::max(i + 1, end); i < end; i++) {

@@ -92,8 +92,9 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
 void reg_plan(const std::vector<LGate>& prog, uint32_t nbits, int32_t precision, int tbits, bool exact, RegPlan& out,
               uint64_t batch_tiles = 0);
 // Queues passes first, first + step, ... of the plan on the context's stream.
+// *queued: whether an error left some of them queued.
 int reg_launch(Ctx* ctx, void* st, uint32_t nbits, int32_t precision, bool exact, const RegPlan& plan, size_t first,
-               size_t step);
+               size_t step, bool* queued = nullptr);
 
 // Runs plan c on register c for all c, and waits.  Every plan has the same
 // number of amplitudes a thread (planned with the same batch_tiles).

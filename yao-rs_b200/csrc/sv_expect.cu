@@ -464,7 +464,11 @@ int expect_sum(Ctx* ctx, const Reg* r, const std::vector<MonoTerm>& terms, Cx* o
     }
     if (!passes.empty()) {
         int s = c64 ? expect_tiles<float2, 12>(ctx, r, passes, out) : expect_tiles<double2, 11>(ctx, r, passes, out);
-        if (s) return s;
+        if (s && s != YAO_ERR_OUT_OF_MEMORY) return s;
+        if (s) {  // no memory for the descriptions: one mask a launch
+            clear_error();
+            rest = terms;
+        }
     }
     if (rest.empty()) return YAO_OK;
     std::vector<Cx> vals;
