@@ -1770,7 +1770,7 @@ static void reg_plan_range(const LGate* prog, size_t ngates, uint32_t nbits, int
     // where the time of one CTA is the time of the pass.
     const uint64_t ntiles = 1ull << (nbits - tbits);
     // (A batch counts the tiles of all its registers, in 2^tbits_max tiles.)
-    int rb = std::max(ntiles, batch_tiles) >= 296 ? 4 : ((batch_tiles ? tbits_max : tbits) > 11 ? 3 : 2);
+    int rb = std::max(ntiles, batch_tiles) >= kManyTiles ? 4 : ((batch_tiles ? tbits_max : tbits) > 11 ? 3 : 2);
     bool four = false;
     for (size_t i = 0; i < ngates; i++) four |= four_bits(prog[i]);
     if (four) rb = 4;

@@ -85,6 +85,9 @@ bool reg_supported(const std::vector<LGate>& prog, uint32_t nbits);
 // becomes a CZ (its Hadamards join the rotations), and phases move past
 // controls and diagonals to the next rotation.  Other gates are kept.
 void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vector<LGate>& out);
+// Tiles that fill the GPU twice over (148 SMs; a constant, so that a program
+// has one plan wherever it is made).
+constexpr uint64_t kManyTiles = 2 * 148;
 // Passes over 2^tbits-amplitude tiles.  exact: program order, except that
 // permutations (X, SWAP, with controls) may move past gates on other qubits,
 // which changes no bit of the result; otherwise any gate may.

@@ -3115,7 +3115,7 @@ static int batch_reg(Ctx* ctx, const std::vector<const std::vector<LGate>*>& pro
     }
     TileConfig cfg;
     cfg.k = std::max(1, k);
-    cfg.tbits = sizeof(V) == 8 && tiles12 >= 296 ? 12 : 11;
+    cfg.tbits = sizeof(V) == 8 && tiles12 >= kManyTiles ? 12 : 11;
     std::vector<RegPlan> plans(progs.size());
     // the long programs first: the threads end together
     std::vector<size_t> order(progs.size());
