@@ -1010,12 +1010,12 @@ struct Splitter {
     Splitter(uint32_t n, std::vector<LGate>& o) : pend(n), out(o) {}
 
     void emit1(int b, int cls, std::vector<Cx> m) {
-        LGate g;
+        out.emplace_back();
+        LGate& g = out.back();
         g.cls = cls;
         g.k = 1;
         g.tb[0] = b;
         g.m = std::move(m);
-        out.push_back(std::move(g));
     }
     // Applies what waits on bit b, except a diagonal when `keep_diag`
     // (what comes next commutes with it).  Matrices are rounded once, here;
@@ -1091,6 +1091,7 @@ struct Splitter {
 
 void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vector<LGate>& out) {
     out.clear();
+    out.reserve(prog.size() + nbits);  // (grown step by step, the gates' 576 bytes each move twice)
     Splitter sp(nbits, out);
     auto single = [](const LGate& g) { return g.k == 1 && g.nc == 0; };
     // per gate: whether the next gate on its target that is no 1-qubit
@@ -1125,14 +1126,14 @@ void split_single_qubit(const std::vector<LGate>& prog, uint32_t nbits, std::vec
             sp.pend[t].hadamard(1.0L);
             sp.flush(t, true);
             sp.flush(g.cb[0], true);
-            LGate z;
+            out.emplace_back();
+            LGate& z = out.back();
             z.cls = GC_DIAG;
             z.k = 2;
             z.tb[0] = std::min(t, (int)g.cb[0]);
             z.tb[1] = std::max(t, (int)g.cb[0]);
             z.m.assign(4, Cx{1.0, 0.0});
             z.m[g.cv[0] ? 3 : (t == z.tb[0] ? 1 : 2)] = Cx{-1.0, 0.0};
-            out.push_back(std::move(z));
             sp.pend[t].hadamard(0.5L);
             continue;
         }
