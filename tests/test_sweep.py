@@ -77,6 +77,25 @@ def test_gradients(n, kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,nsets,extra", [(5, 3, 0), (5, 3, 1), (8, 1, 1), (8, 4, 1), (2, 1, 1)])
+def test_sets_of_circuits_that_leave_the_sweep(n, nsets, extra):
+    """Odd and even numbers of gradients in all (the complex numbers that lie
+    behind them in memory need 16-byte boundaries): a controlled rotation is
+    not the register sweep's."""
+    rng = np.random.default_rng([n, nsets])
+    els = [Y.put([q], Gate.Ry(0.3)) for q in range(n)] + [Y.control([0], [1], Gate.Rx(0.7)), Y.put([1], Gate.Rz(0.2))]
+    els += [Y.put([0], Gate.Rx(0.1)) for _ in range(extra + n % 2)]
+    c, h, psi = Y.Circuit.qubits(n, els), hamiltonian(n), random_state(rng, n)
+    assert c.num_params() % 2 == (1 if extra else 0)
+    sets = rng.uniform(-3, 3, size=(nsets, c.num_params()))
+    vs, gs = Y.expect_grad_batch(h, c, sets, Y.ArrayReg.from_vec(n, psi))
+    for s in range(nsets):
+        c.dispatch(list(sets[s]))
+        value, grad = O.expect_grad(h, c, psi)
+        assert abs(vs[s] - value) < 1e-12 and np.max(np.abs(gs[s] - np.array(grad))) < 1e-12
+
+
+@pytest.mark.gpu
 def test_more_sets_than_a_group():
     """Groups of states that fit the cache, the last one smaller: every set as
     by itself."""

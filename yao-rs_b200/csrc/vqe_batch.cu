@@ -330,13 +330,15 @@ int expect_grad_batch(Ctx* ctx, const std::vector<MonoTerm>& terms, const Circui
             lowered_coefs(dg, neg, n, &hd[(s.coef_off * nsets + set) * 16]);
         }
     }
-    // device memory
-    const size_t sb = nsets * N * sizeof(double2);
+    // device memory: every part at a multiple of 256 bytes (an odd number of
+    // gradients left the complex parts after them misaligned)
+    auto al = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t sb = al(nsets * N * sizeof(double2));
     const int nbx = (int)std::max<uint64_t>(1, std::min<uint64_t>((N / 2 + kBT - 1) / kBT, 64));
-    const size_t partial_b = nsets * (size_t)nbx * 16 * sizeof(double);
-    const size_t coef_b = std::max<size_t>(1, hf.size()) * sizeof(double2);
-    const size_t grad_b = std::max<size_t>(1, nsets * np) * sizeof(double);
-    const size_t vals_b = std::max<size_t>(1, nsets * terms.size()) * sizeof(double2);
+    const size_t partial_b = al(nsets * (size_t)nbx * 16 * sizeof(double));
+    const size_t coef_b = al(std::max<size_t>(1, hf.size()) * sizeof(double2));
+    const size_t grad_b = al(std::max<size_t>(1, nsets * np) * sizeof(double));
+    const size_t vals_b = al(std::max<size_t>(1, nsets * terms.size()) * sizeof(double2));
     // term groups (x-mask, <= 8 terms) of the energy reduction
     std::vector<BGroup> groups;
     std::vector<int> gidx;
@@ -367,9 +369,9 @@ int expect_grad_batch(Ctx* ctx, const std::vector<MonoTerm>& terms, const Circui
             groups.push_back(grp);
         }
     }
-    const size_t gen_b = hg.size() * sizeof(double2), idx_b = std::max<size_t>(1, gidx.size()) * sizeof(int);
+    const size_t gen_b = al(hg.size() * sizeof(double2)), idx_b = std::max<size_t>(1, gidx.size()) * sizeof(int);
     char* buf = nullptr;
-    const size_t total = 2 * sb + partial_b + 2 * coef_b + grad_b + vals_b + gen_b + idx_b + 4096;
+    const size_t total = 2 * sb + partial_b + 2 * coef_b + grad_b + vals_b + gen_b + idx_b;
     if (alloc_async(ctx, (void**)&buf, total) != cudaSuccess) {
         cudaGetLastError();
         return fail(YAO_ERR_OUT_OF_MEMORY, "cannot allocate the batched gradient buffers");
@@ -385,7 +387,7 @@ int expect_grad_batch(Ctx* ctx, const std::vector<MonoTerm>& terms, const Circui
     int* didx = (int*)((char*)dgen + gen_b);
     YAO_CUDA(cudaMemcpyAsync(dfwd, hf.data(), hf.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
     YAO_CUDA(cudaMemcpyAsync(ddag, hd.data(), hd.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
-    YAO_CUDA(cudaMemcpyAsync(dgen, hg.data(), gen_b, cudaMemcpyHostToDevice, ctx->stream));
+    YAO_CUDA(cudaMemcpyAsync(dgen, hg.data(), hg.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
     if (!gidx.empty())
         YAO_CUDA(cudaMemcpyAsync(didx, gidx.data(), gidx.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     const uint64_t tot = nsets * N;
